@@ -211,6 +211,66 @@ void launch_tma(FusedArgs<S, C> a, const TmaMaps &maps, bool energy, cudaStream_
 constexpr int TMA_QW = TMA_W + 8;    // columns of a 16-bit coefficient box: from 8 before the strip's core
                                      // (a 16-byte boundary) to 4 beyond the 128 loaded field columns
 
+// on-chip runs of the elastic step (resident.cuh): many steps in one cooperative launch, ntx x nty
+// tiles of the grid, one CTA each, FP32 / FP64 storage, free-surface x ends, periodic y
+constexpr int RES_THREADS = 512;
+constexpr int RES_PAD = 4;            // rows / columns around a tile in shared memory
+constexpr int RES_LANES_COLS = 64;    // columns a row's threads cover: 4 on the left, then up to RES_W
+constexpr int RES_W = 58;             // most columns of a tile (column My included)
+constexpr int RES_P = 68;             // values of a shared row (FP32 rows of 5 fields 1360 bytes apart: 13 or
+                                      // 14 vectors a row, two or three rows a warp, few bank conflicts)
+constexpr int RES_MIN = 8;            // least rows / columns of a tile: halos and closures meet one neighbour
+template <class C>
+struct ResArgs {
+    const C *in[5];           // state before the run
+    C *out[5];                // state after it
+    const C *rin[5];          // residuals (compensation codes)
+    C *rout[5];
+    const C *coef[5];
+    const C *coefx[2];        // 1/rho of MN and NM with 4 periodic columns on the left and 8 on the
+                              // right (tiles whose coefficients stay in L2), rows of xpitch elements
+    long xpitch;
+    long pitch;
+    int Mx, My;
+    Ops<C> op;
+    int ntx, nty;             // tiles along x and y
+    int rows_s;               // rows of a tile's shared memory
+    int n;                    // steps of this run
+    unsigned tag0;            // steps the handle has run this way before: tags of the exchange words
+    unsigned long long *xbuf; // exchange words: [2][NN, MM0, MM1][(Mx + 1) x xcols], FP64 two words a value
+    long xarr;                // words of one array
+    int xcols;
+    const double *src_inc;
+    int src_grid, src_ix, src_iy;
+    const int *step;          // read by every CTA; the last CTA to finish advances it by n
+    int *step_w;
+    int *done;
+    int *flags;
+    int max_steps;
+    const double *w[5];       // energy weights
+    double *energy;
+    const int *rcv_off;       // receivers by tile
+    const int *rcv;           // [n][4]: field slot, row, column, trace row
+    double *traces;
+};
+struct ResPlan {
+    int ntx = 0, nty = 0;     // 0: the grid does not fit
+    int rows_s = 0;
+    bool cs = true;           // coefficients in shared memory
+    size_t smem = 0;
+};
+// the tiling of a grid over n_sm SMs with smem_max bytes each
+ResPlan resident_plan(long Mx, long My, int esize, bool comp, int n_sm, size_t smem_max);
+// tile index of a point (host side receiver lists)
+int resident_tile(const ResPlan &p, long Mx, long My, int row, int col);
+template <class C>
+cudaError_t prepare_resident(int cpst, bool energy, const ResPlan &p);
+template <class C>
+cudaError_t launch_resident(const ResArgs<C> &a, int cpst, bool energy, const ResPlan &p, cudaStream_t st);
+// rows of `in` (cols periodic M- or N-type columns) with 4 more columns on the left and 8 on the right
+template <class C>
+void launch_pad_columns(const C *in, long pitch, C *out, long xpitch, int rows, int My, int n_type, cudaStream_t st);
+
 // free y ends on the fused step (ysat_fix.cu): the fused kernel steps every column with the
 // periodic y rule; these two launches then recompute, from the step's input buffers, the points
 // whose y stencils meet an end (velocities, then the stresses that read them), with the SBP

@@ -1,0 +1,884 @@
+// On-chip runs of the elastic step: many steps in one cooperative launch, each CTA keeping one
+// tile of the grid in shared memory, for grids that fit on the chip's SMs (FP32: up to about 1.1
+// million cells).
+//
+// Such a grid is bound by latency, not by bytes: one launch a step leaves the machine idle
+// between launches, and a launch's first loads and its boundary strips are a serial chain of some
+// 30 us whatever the grid's size. Here the state never leaves the SMs between steps. What limits
+// a step is the exchange of tile edges (about a microsecond: one store and one load through L2)
+// and the instructions of the largest tile. Us a step, one launch a step -> here (B200, FP32, energy
+// off): 48 x 40 29.1 -> 2.4, 200 x 150 27.2 -> 2.5, 509 x 317 28.9 -> 3.4, 700 x 700 30.7 -> 7.4, 1024 x 1024
+// 38.1 -> 15.7; with the energy 509 x 317 33.9 -> 4.8; FP64 509 x 317 30.9 -> 5.0, 700 x 700 32.7 -> 13.1;
+// '6C' 509 x 317 32.9 -> 3.9.
+//
+// A tile owns rows [x0, x1) and columns [y0, y1) (the last tiles also the N-type row Mx and column
+// My). It holds the stresses with a halo of 3 points on each side and the velocities with 2, which
+// it recomputes itself, so one exchange of stresses a step suffices:
+//   V: velocities of the tile and of its halo from the stresses (they read nothing the
+//      neighbour's own velocities need, so both compute the same values);
+//   S: stresses of the tile from the velocities; the points within 3 of an edge also go to the
+//      exchange buffer;
+//   X: the halo points of the neighbours' stresses are read from the exchange buffer.
+// An exchanged value travels as 64-bit words of 32 value bits and a 32-bit tag, the number of the
+// step in the handle's life: a reader polls the word itself until the tag is the one it waits
+// for, so there is no flag, fence or barrier between CTAs. Words alternate between two buffers by
+// the tag's parity: a CTA can be at most one step ahead of its neighbours, since it needs their
+// words of the step before. Every poll is bounded; a CTA that gives up raises FLAG_TIMEOUT and
+// leaves, and so in turn do the CTAs that wait for it.
+//
+// Thread layout: an item is one row of 16 bytes' worth of columns (4 FP32, 2 FP64), items are
+// dealt to the threads row by row. Per point the arithmetic and the order of the right-hand-side
+// terms are those of step_kernels.cu: results are bit-identical. FP32 sums and products go two at
+// a time (mul / add / sub .rn.f32x2: each half is rounded on its own, as the scalar instruction).
+#pragma once
+#include "kernels.h"
+#include "stepper.cuh"
+
+namespace tw {
+
+namespace {
+
+using u64 = unsigned long long;
+using tw::add;   // (the scalar overloads beside the vector ones below)
+using tw::mul;
+
+// ---- vectors of 16 bytes
+template <class C> struct Vec;
+template <> struct Vec<float> {
+    static constexpr int N = 4;
+    using W = u64;   // a weight, in both halves
+    u64 a, b;
+};
+template <> struct Vec<double> {
+    static constexpr int N = 2;
+    using W = double;
+    double a, b;
+};
+using VF = Vec<float>;
+using VD = Vec<double>;
+
+__device__ __forceinline__ u64 pk(float x, float y)
+{
+    u64 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ void unpk(u64 v, float &x, float &y) { asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v)); }
+__device__ __forceinline__ u64 mul2(u64 x, u64 y)
+{
+    u64 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(x), "l"(y));
+    return r;
+}
+__device__ __forceinline__ u64 fma2(u64 x, u64 y, u64 z)
+{
+    u64 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(x), "l"(y), "l"(z));
+    return r;
+}
+__device__ __forceinline__ u64 wt(float s) { return pk(s, s); }
+__device__ __forceinline__ double wt(double s) { return s; }
+__device__ __forceinline__ VF mul(VF x, VF y) { return {mul2(x.a, y.a), mul2(x.b, y.b)}; }
+__device__ __forceinline__ VF mulw(VF x, u64 s) { return {mul2(x.a, s), mul2(x.b, s)}; }
+__device__ __forceinline__ VD mul(VD x, VD y) { return {mul(x.a, y.a), mul(x.b, y.b)}; }
+__device__ __forceinline__ VD mulw(VD x, double s) { return {mul(x.a, s), mul(x.b, s)}; }
+__device__ __forceinline__ VF vzero(float) { return {0ull, 0ull}; }
+__device__ __forceinline__ VD vzero(double) { return {0., 0.}; }
+__device__ __forceinline__ VF vld(const float *p)
+{
+    const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(p);
+    return {v.x, v.y};
+}
+__device__ __forceinline__ VD vld(const double *p)
+{
+    const double2 v = *reinterpret_cast<const double2 *>(p);
+    return {v.x, v.y};
+}
+__device__ __forceinline__ VF vldg(const float *p)
+{
+    const ulonglong2 v = __ldg(reinterpret_cast<const ulonglong2 *>(p));
+    return {v.x, v.y};
+}
+__device__ __forceinline__ VD vldg(const double *p)
+{
+    const double2 v = __ldg(reinterpret_cast<const double2 *>(p));
+    return {v.x, v.y};
+}
+__device__ __forceinline__ void vst(float *p, VF v) { *reinterpret_cast<ulonglong2 *>(p) = make_ulonglong2(v.a, v.b); }
+__device__ __forceinline__ void vst(double *p, VD v) { *reinterpret_cast<double2 *>(p) = make_double2(v.a, v.b); }
+__device__ __forceinline__ void vget(VF v, float (&e)[4])
+{
+    unpk(v.a, e[0], e[1]);
+    unpk(v.b, e[2], e[3]);
+}
+__device__ __forceinline__ void vget(VD v, double (&e)[2])
+{
+    e[0] = v.a;
+    e[1] = v.b;
+}
+__device__ __forceinline__ VF vset(const float (&e)[4]) { return {pk(e[0], e[1]), pk(e[2], e[3])}; }
+__device__ __forceinline__ VD vset(const double (&e)[2]) { return {e[0], e[1]}; }
+
+// the stencil weights and the vector sums. A packed FP32 sum is fma(x, 1, y) with a 1 the compiler
+// cannot see through (and a difference fma(y, -1, x)): a mul.rn.f32x2 whose result feeds an
+// add.rn.f32x2 came out contracted into one rounding, and these cannot be.
+template <class C> struct St;
+template <>
+struct St<float> {
+    u64 w[4], one, mone;
+    __device__ __forceinline__ St(const float (&st)[4], bool truth)
+    {
+#pragma unroll
+        for (int k = 0; k < 4; k++) w[k] = wt(st[k]);
+        one = wt(truth ? 1.f : 2.f);
+        mone = wt(truth ? -1.f : 2.f);
+    }
+    __device__ __forceinline__ VF add(VF x, VF y) const { return {fma2(x.a, one, y.a), fma2(x.b, one, y.b)}; }
+    __device__ __forceinline__ VF sub(VF x, VF y) const { return {fma2(y.a, mone, x.a), fma2(y.b, mone, x.b)}; }
+};
+template <>
+struct St<double> {
+    double w[4];
+    __device__ __forceinline__ St(const double (&st)[4], bool)
+    {
+#pragma unroll
+        for (int k = 0; k < 4; k++) w[k] = st[k];
+    }
+    __device__ __forceinline__ VD add(VD x, VD y) const { return {tw::add(x.a, y.a), tw::add(x.b, y.b)}; }
+    __device__ __forceinline__ VD sub(VD x, VD y) const { return {tw::sub(x.a, y.a), tw::sub(x.b, y.b)}; }
+};
+
+// sum of four taps, each a vector (the leading 0 + is left out: see tma_step.cuh)
+template <class C>
+__device__ __forceinline__ Vec<C> taps(const St<C> &s, Vec<C> t0, Vec<C> t1, Vec<C> t2, Vec<C> t3)
+{
+    Vec<C> v = mulw(t0, s.w[0]);
+    v = s.add(v, mulw(t1, s.w[1]));
+    v = s.add(v, mulw(t2, s.w[2]));
+    return s.add(v, mulw(t3, s.w[3]));
+}
+// y derivative of N-type points from the M-type row p (taps c-2 .. c+1); mid: the vector at c
+__device__ __forceinline__ VF dyN(const St<float> &s, const float *p, VF mid)
+{
+    const u64 l = *reinterpret_cast<const u64 *>(p - 2);
+    float l0, l1, m0, m1, m2, m3;
+    unpk(l, l0, l1);
+    unpk(mid.a, m0, m1);
+    unpk(mid.b, m2, m3);
+    const u64 o0 = pk(l1, m0), o1 = pk(m1, m2), o2 = pk(m3, p[4]);
+    return taps<float>(s, {l, mid.a}, {o0, o1}, mid, {o1, o2});
+}
+__device__ __forceinline__ VD dyN(const St<double> &s, const double *p, VD mid)
+{
+    const VD l = vld(p - 2);
+    const double r = p[2];
+    return taps<double>(s, l, {l.b, mid.a}, mid, {mid.b, r});
+}
+// y derivative of M-type points from the N-type row p (taps c-1 .. c+2)
+// (alt: the column after the vector is *z)
+__device__ __forceinline__ VF dyM(const St<float> &s, const float *p, VF mid, bool alt, const float *z)
+{
+    const u64 r = *reinterpret_cast<const u64 *>(p + 4);
+    float m0, m1, m2, m3, r0, r1;
+    unpk(mid.a, m0, m1);
+    unpk(mid.b, m2, m3);
+    unpk(r, r0, r1);
+    if (alt) r0 = *z;
+    const u64 o0 = pk(p[-1], m0), o1 = pk(m1, m2), o2 = pk(m3, r0);
+    return taps<float>(s, {o0, o1}, mid, {o1, o2}, {mid.b, pk(r0, r1)});
+}
+__device__ __forceinline__ VD dyM(const St<double> &s, const double *p, VD mid, bool alt, const double *z)
+{
+    VD r = vld(p + 2);
+    if (alt) r.a = *z;
+    const double l = p[-1];
+    return taps<double>(s, {l, mid.a}, mid, {mid.b, r.a}, r);
+}
+
+// the closure and penalty weights of the x ends in shared memory, as Vec weights (read there with
+// one broadcast load; indexed by the row they would come from the parameter bank one by one)
+template <class C>
+struct XEnds {
+    using W = typename Vec<C>::W;
+    W dn[6][5], dm[8][5];   // M-type rows 0..2, Mx-3..Mx-1; N-type rows 0..3, Mx-3..Mx
+    W satM[6], satN[2], pM[6];
+};
+template <class C>
+__device__ __forceinline__ void load_ends(XEnds<C> &x, const Ops<C> &o, int tid)
+{
+    if (tid < 15) { x.dn[tid / 5][tid % 5] = wt(o.dnL[tid / 5][tid % 5]); x.dn[3 + tid / 5][tid % 5] = wt(o.dnR[tid / 5][tid % 5]); }
+    if (tid < 20) { x.dm[tid / 5][tid % 5] = wt(o.dmL[tid / 5][tid % 5]); x.dm[4 + tid / 5][tid % 5] = wt(o.dmR[tid / 5][tid % 5]); }
+    if (tid < 3) { x.satM[tid] = wt(o.satML[tid]); x.satM[3 + tid] = wt(o.satMR[tid]); x.pM[tid] = wt(o.pML[tid]); x.pM[3 + tid] = wt(o.pMR[tid]); }
+    if (tid == 0) { x.satN[0] = wt(o.satNL); x.satN[1] = wt(o.satNR); }
+}
+
+// x derivative of an M-type row ix next to an x end (get(r): the N-type neighbour's vector at row r)
+template <class C, class G>
+__device__ __forceinline__ Vec<C> vdxN_end(const XEnds<C> &o, const St<C> &s, int Mx, int ix, G get)
+{
+    const bool L = ix < 3;
+    const auto *c = o.dn[L ? ix : ix - (Mx - 6)];
+    const int r0 = L ? 0 : Mx - 4;
+    Vec<C> v = vzero(C(0));
+#pragma unroll
+    for (int w = 0; w < 5; w++) v = s.add(v, mulw(get(r0 + w), c[w]));
+    return v;
+}
+// the same of an N-type row from its M-type neighbour
+template <class C, class G>
+__device__ __forceinline__ Vec<C> vdxM_end(const XEnds<C> &o, const St<C> &s, int Mx, int ix, G get)
+{
+    const bool L = ix < 4;
+    const auto *c = o.dm[L ? ix : ix - (Mx - 7)];
+    const int r0 = L ? 0 : Mx - 5;
+    Vec<C> v = vzero(C(0));
+#pragma unroll
+    for (int w = 0; w < 5; w++) v = s.add(v, mulw(get(r0 + w), c[w]));
+    return v;
+}
+
+template <int CPST, class C>
+__device__ __forceinline__ void vupdate(const St<C> &t_, Vec<C> &s, Vec<C> &r, Vec<C> &c)
+{
+    if constexpr (CPST == 0) {
+        s = t_.add(s, r);
+    } else if constexpr (CPST == 1 || CPST == 3) {
+        const Vec<C> y = t_.add(r, c), t = t_.add(s, y);
+        c = t_.sub(y, t_.sub(t, s));
+        s = t;
+    } else if constexpr (CPST == 2 || CPST == 4) {
+        const Vec<C> t = t_.add(s, r);
+        r = t_.sub(r, t_.sub(t, s));
+        s = t;
+    } else {
+        const Vec<C> b = (CPST == 5) ? t_.add(r, c) : r;
+        const Vec<C> t = t_.add(s, b);
+        const Vec<C> pa = t_.sub(t, b), pb = t_.sub(t, pa);
+        const Vec<C> d = t_.add(t_.sub(s, pa), t_.sub(b, pb));
+        s = t;
+        if constexpr (CPST == 5) c = d; else r = d;
+    }
+}
+
+// ---- exchange words: 32 value bits and the tag (an FP64 value is two words)
+__device__ __forceinline__ u64 xword(unsigned v, unsigned tag)
+{
+    u64 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(v), "r"(tag));
+    return r;
+}
+__device__ __forceinline__ void xst(u64 *p, float v, unsigned tag)
+{
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(xword(__float_as_uint(v), tag)) : "memory");
+}
+// two words at once (each word is written whole)
+__device__ __forceinline__ void xst2(u64 *p, u64 x, u64 y)
+{
+    asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(x), "l"(y) : "memory");
+}
+__device__ __forceinline__ void xst(u64 *p, double v, unsigned tag)
+{
+    xst2(p, xword((unsigned)__double2loint(v), tag), xword((unsigned)__double2hiint(v), tag));
+}
+__device__ __forceinline__ void xstv(u64 *p, const float (&e)[4], unsigned tag)
+{
+    xst2(p, xword(__float_as_uint(e[0]), tag), xword(__float_as_uint(e[1]), tag));
+    xst2(p + 2, xword(__float_as_uint(e[2]), tag), xword(__float_as_uint(e[3]), tag));
+}
+__device__ __forceinline__ void xstv(u64 *p, const double (&e)[2], unsigned tag)
+{
+    xst(p, e[0], tag);
+    xst(p + 2, e[1], tag);
+}
+__device__ __forceinline__ u64 xld(const u64 *p)
+{
+    u64 v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+constexpr int X_POLLS = 1 << 20;   // polls before a CTA gives up (about a second)
+// one exchanged value: loaded, and whether it is the step's
+template <class C> struct XV;
+template <> struct XV<float> {
+    u64 x;
+    __device__ __forceinline__ void load(const u64 *p) { x = xld(p); }
+    __device__ __forceinline__ bool ok(unsigned tag) const { return (unsigned)(x >> 32) == tag; }
+    __device__ __forceinline__ float get() const { return __uint_as_float((unsigned)x); }
+};
+template <> struct XV<double> {
+    u64 x, y;
+    __device__ __forceinline__ void load(const u64 *p)
+    {
+        x = xld(p);
+        y = xld(p + 1);
+    }
+    __device__ __forceinline__ bool ok(unsigned tag) const { return (unsigned)(x >> 32) == tag && (unsigned)(y >> 32) == tag; }
+    __device__ __forceinline__ double get() const { return __hiloint2double((int)(unsigned)y, (int)(unsigned)x); }
+};
+
+}  // namespace
+
+// one tile's shared memory: rows of NF x RES_P values (the five fields, then their residuals under a
+// compensation code, then with CS the coefficients), so that every neighbour of a point is at a
+// compile-time distance from it. A row's vectors belong to LANES threads; a thread keeps its column
+// and walks down the rows, RES_THREADS / LANES rows apart (tall tiles: two rows at a time).
+template <class C, int CPST, bool ENERGY, bool CS>
+__global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_constant__ ResArgs<C> a)
+{
+    constexpr bool KR = Cpst<CPST>::keep_r, KC = Cpst<CPST>::keep_c, RES = KR || KC;
+    constexpr int N = Vec<C>::N, H = RES_PAD, P = RES_P, LANES = RES_LANES_COLS / N;
+    constexpr int NF = 5 + (RES ? 5 : 0) + (CS ? 5 : 0), RS = NF * P;
+    constexpr int o_r = 5 * P, o_c = (RES ? 10 : 5) * P;   // residual and coefficient rows
+    constexpr int XW = sizeof(C) / 4;                      // exchange words of a value
+    using V = Vec<C>;
+    extern __shared__ __align__(16) unsigned char res_smem[];
+    __shared__ double red[2][3][RES_THREADS / 32];
+    __shared__ int bad_s;
+    __shared__ XEnds<C> ends;
+    const int tid = threadIdx.x;
+    const int Mx = a.Mx, My = a.My;
+    const int tx = blockIdx.x / a.nty, ty = blockIdx.x - tx * a.nty;
+    const int x0 = (int)((long)tx * Mx / a.ntx), x1 = (int)((long)(tx + 1) * Mx / a.ntx);
+    const int nq4 = (My + 4) / 4;   // column quads of the grid (My + 1 columns)
+    const int y0 = 4 * (int)((long)ty * nq4 / a.nty);
+    const bool lastx = tx == a.ntx - 1, lasty = ty == a.nty - 1;
+    const int y1 = lasty ? My : 4 * (int)((long)(ty + 1) * nq4 / a.nty);   // M-type columns end here
+    const int R = x1 - x0, W = y1 - y0;             // owned M-type rows and columns
+    const int RN = R + (lastx ? 1 : 0), WN = W + (lasty ? 1 : 0);
+    C *sm = reinterpret_cast<C *>(res_smem);
+    C *altL = sm + (size_t)a.rows_s * RS, *altR = altL + a.rows_s;
+    auto at = [&](int f, int r, int c) { return sm + (r + H) * RS + f * P + c + H; };
+    auto ntypeY = [](int f) { return f == F_NN || f == F_MN; };
+    auto rows_of = [&](int f) { return (f == F_NN || f == F_NM) ? Mx + 1 : Mx; };
+    auto phys = [&](bool ntype, int c) {   // physical column of the tile's column c
+        int g = y0 + c;
+        if (g < 0) g += My;
+        else if (ntype ? g > My : g >= My) g -= My;
+        return g;
+    };
+    const int it0 = *a.step;
+    if (tid == 0) bad_s = 0;
+    load_ends<C>(ends, a.op, tid);
+
+    // ---- load the tile with its halo
+    for (int k = tid; k < a.rows_s * P; k += RES_THREADS) {
+        const int r = k / P - H, c = k - (r + H) * P - H, g = x0 + r;
+#pragma unroll
+        for (int f = 0; f < 5; f++) {
+            const bool in = g >= 0 && g < rows_of(f) && r < RN + 3 && r >= -3 && c >= -3 && c < WN + 3;
+            const long o = in ? (long)g * a.pitch + phys(ntypeY(f), c) : 0;
+            C *q = at(f, r, c);
+            q[0] = in ? a.in[f][o] : C(0);
+            if constexpr (RES) q[o_r] = in ? a.rin[f][o] : C(0);
+            if constexpr (CS) q[o_c] = in ? a.coef[f][o] : C(0);
+        }
+    }
+    // the N-type seam: an M-type point left of column 0 reads column My where this tile holds
+    // column 0, one right of column My - 1 reads column 0 where it holds column My
+    for (int k = tid; k < a.rows_s; k += RES_THREADS) {
+        const int g = x0 + k - H;
+        const bool in = g >= 0 && g <= Mx && k - H < RN + 3;
+        altL[k] = in && ty == 0 ? a.in[F_NN][(long)g * a.pitch + My] : C(0);
+        altR[k] = in && lasty ? a.in[F_NN][(long)g * a.pitch] : C(0);
+    }
+    const int rb = a.rcv_off[blockIdx.x], re = a.rcv_off[blockIdx.x + 1];
+    const St<C> st(a.op.st, a.n > 0);
+    const bool multi = a.ntx * a.nty > 1;
+    const int lc = W;   // (last tile of a row) the local column of My
+
+    // ---- this thread's column and rows: V on rows [va, vb) and columns -4 .. WN + 1, S on the owned
+    // points. Tiles of few rows give the two kinds of point of a phase to the two halves of the CTA.
+    constexpr int SLOTS = RES_THREADS / LANES;
+    const int va = max(-2, -x0), vb = min(R + 2, Mx + 1 - x0);
+    const int c = (tid % LANES) * N - 4;
+    const bool split = vb - va <= SLOTS / 2;
+    const int slot = split ? (tid / LANES) % (SLOTS / 2) : tid / LANES, dslot = split ? SLOTS / 2 : SLOTS;
+    const bool first = !split || tid < RES_THREADS / 2, second = !split || tid >= RES_THREADS / 2;
+    const bool vcol = c < WN + 2, scol = c >= 0 && c < WN;
+    const int ownN = scol ? min(N, WN - c) : 0, ownM = scol ? max(0, min(N, W - c)) : 0;
+    const bool vpair = !ENERGY && vb - va > SLOTS;   // (the energy's registers leave no room for two rows)
+    const bool seamL = ty == 0 && c == -N, seamR = lasty && c + N > lc && c <= lc + 1;
+    const bool bcol = c < 4 || c + N > WN - 4;   // columns the neighbours (or the seam) read
+    int sq = -1;                                 // the source's column among this thread's
+    if (a.src_grid >= 0)
+        for (int q = 0; q < N; q++)
+            if (c + q >= -3 && c + q < WN + 3 && phys(a.src_grid == G_NN || a.src_grid == G_MN, c + q) == a.src_iy) sq = q;
+    auto own_row = [&](int g) { return g == a.src_grid ? a.src_ix - x0 : -(1 << 20); };
+    const int srcMN = own_row(G_MN), srcNM = own_row(G_NM), srcNN = own_row(G_NN), srcMM = own_row(G_MM);
+
+    // ---- this thread's halo words: 3 rows above and below over columns [-3, WN + 3), 3 columns on
+    // each side, the seam columns of the V rows
+    constexpr int XI = 3;   // (RES_THREADS x XI covers the largest tile: resident_plan)
+    int xs[XI], xm[XI], xg[XI], xh[XI];   // shared index of NN, of MM0 (-1: none), words of NN, of MM0
+    {
+        const int hw = WN + 6, ht = tx > 0 ? 3 : 0, hb = lastx ? 0 : 3, nvr = vb - va;
+        const int n1 = (ht + hb) * hw, n2 = n1 + RN * 6, n3 = n2 + (ty == 0 ? nvr : 0), n4 = n3 + (lasty ? nvr : 0);
+#pragma unroll
+        for (int m = 0; m < XI; m++) {
+            const int h = tid + m * RES_THREADS;
+            xs[m] = xm[m] = -1;
+            xg[m] = xh[m] = 0;
+            if (!multi || h >= n4) continue;
+            if (h < n2) {
+                int r, cc;
+                if (h < n1) {
+                    const int q = h / hw;
+                    cc = h - q * hw - 3;
+                    r = q < ht ? q - 3 : RN + (q - ht);
+                } else {
+                    r = (h - n1) / 6;
+                    cc = h - n1 - 6 * r;
+                    cc = cc < 3 ? cc - 3 : WN + cc - 3;
+                }
+                const int g = x0 + r, cm = (lasty && cc >= WN) ? cc - 1 : cc;   // (M-type halos start at W)
+                xs[m] = (int)(at(F_NN, r, cc) - sm);
+                xg[m] = (g * a.xcols + phys(true, cc)) * XW;
+                if (g < Mx) {
+                    xm[m] = (int)(at(F_MM0, r, cm) - sm);
+                    xh[m] = (g * a.xcols + phys(false, cm)) * XW;
+                }
+            } else {
+                const bool left = h < n3;
+                const int r = va + (left ? h - n2 : h - n3);
+                xs[m] = (int)((left ? altL : altR) + r + H - sm);
+                xg[m] = ((x0 + r) * a.xcols + (left ? My : 0)) * XW;
+            }
+        }
+    }
+    double ep_prev = 0.;
+    __syncthreads();
+
+    for (int k = 0; k < a.n; k++) {
+        const int it = it0 + k;
+        const bool last = k == a.n - 1;
+        double ek = 0., ep0 = 0., ep1 = 0.;
+        auto source = [&](V &v) {
+            if (sq >= 0) {
+                const double inc = a.src_inc[it];
+                C e[N];
+                vget(v, e);
+#pragma unroll
+                for (int q = 0; q < N; q++)
+                    if (q == sq) e[q] = (C)add((double)e[q], inc);
+                v = vset(e);
+            }
+        };
+        // the energy weights of this thread's points of a row (loaded before the points are computed)
+        struct WV { double w[N]; };
+        auto weights = [&](int f, int r, bool own) {
+            WV v;
+            const double2 *p = reinterpret_cast<const double2 *>(a.w[f] + (long)(x0 + r) * a.pitch + y0 + c);
+#pragma unroll
+            for (int q = 0; q < N; q += 2) {
+                const double2 x = own ? __ldg(p + q / 2) : make_double2(0., 0.);
+                v.w[q] = x.x;
+                v.w[q + 1] = x.y;
+            }
+            return v;
+        };
+        // ---- V: velocities
+        // one row; ld(f, o): this column's vector of field f, o rows on
+        auto vrow = [&](int r, C *q, auto ld) {
+                const int j = x0 + r;
+                const bool orow = r >= 0 && r < RN;
+                auto coefv = [&](int f) -> V {
+                    if constexpr (CS) return vld(q + f * P + o_c);
+                    else return vldg(a.coefx[f - F_MN] + (long)j * a.xpitch + y0 + c + 4);
+                };
+                const V nnj = ld(F_NN, 0);
+                if (first && j < Mx) {   // MN: x from NN, y from MM syy
+                    [[maybe_unused]] WV wv;
+                    if constexpr (ENERGY) wv = weights(F_MN, r, orow && ownN > 0);
+                    const V P_ = coefv(F_MN);
+                    V r_ = vzero(C(0)), cc = r_, vx;
+                    if constexpr (KR) r_ = vld(q + F_MN * P + o_r);
+                    if constexpr (KC) cc = vld(q + F_MN * P + o_r);
+                    if (j >= 3 && j < Mx - 3) {
+                        vx = taps<C>(st, ld(F_NN, -1), nnj, ld(F_NN, 1), ld(F_NN, 2));
+                        r_ = st.add(r_, mul(vx, P_));
+                    } else {   // closure and SAT
+                        vx = vdxN_end<C>(ends, st, Mx, j, [&](int g) { return vld(at(F_NN, g - x0, c)); });
+                        r_ = st.add(r_, mul(vx, P_));
+                        const bool L = j < 3;
+                        const V send = mulw(vld(at(F_NN, L ? -x0 : Mx - x0, c)), wt(a.op.pN));
+                        r_ = st.add(r_, mul(mulw(send, ends.satM[L ? j : j - (Mx - 6)]), P_));
+                    }
+                    r_ = st.add(r_, mul(dyN(st, q + F_MM1 * P, vld(q + F_MM1 * P)), P_));
+                    V s = vld(q + F_MN * P);
+                    vupdate<CPST, C>(st, s, r_, cc);
+                    if (r == srcMN) source(s);
+                    vst(q + F_MN * P, s);
+                    if constexpr (RES) vst(q + F_MN * P + o_r, KR ? r_ : cc);
+                    if constexpr (ENERGY) {
+                        C e[N];
+                        vget(s, e);
+#pragma unroll
+                        for (int i = 0; i < N; i++)
+                            if (orow && i < ownN) ek = add(ek, mul(mul((double)e[i], wv.w[i]), (double)e[i]));
+                    }
+                }
+                if (second) {   // NM: x from MM sxx, y from NN
+                    [[maybe_unused]] WV wv;
+                    if constexpr (ENERGY) wv = weights(F_NM, r, orow && ownM > 0);
+                    const V P_ = coefv(F_NM);
+                    V r_ = vzero(C(0)), cc = r_, vx;
+                    if constexpr (KR) r_ = vld(q + F_NM * P + o_r);
+                    if constexpr (KC) cc = vld(q + F_NM * P + o_r);
+                    if (j >= 4 && j < Mx - 3) {
+                        vx = taps<C>(st, ld(F_MM0, -2), ld(F_MM0, -1), ld(F_MM0, 0), ld(F_MM0, 1));
+                        r_ = st.add(r_, mul(vx, P_));
+                    } else {
+                        vx = vdxM_end<C>(ends, st, Mx, j, [&](int g) { return vld(at(F_MM0, g - x0, c)); });
+                        r_ = st.add(r_, mul(vx, P_));
+                        if (j == 0 || j == Mx) {   // SAT
+                            const bool L = j == 0;
+                            V send = vzero(C(0));
+#pragma unroll
+                            for (int w = 0; w < 3; w++)
+                                send = st.add(send, mulw(vld(at(F_MM0, (L ? w : Mx - 3 + w) - x0, c)), ends.pM[(L ? 0 : 3) + w]));
+                            r_ = st.add(r_, mul(mulw(send, ends.satN[L ? 0 : 1]), P_));
+                        }
+                    }
+                    // (left of column 0 the next column is My, not the tile's column 0)
+                    V vy = dyM(st, q + F_NN * P, nnj, seamL, altL + r + H);
+                    if (seamR) {   // the columns from My on: the one there is column 0
+                        const C *p = at(F_NN, r, lc);
+                        const C z = altR[r + H], p1 = p[1], p2 = p[2];
+                        auto tap4 = [&](C t0, C t1, C t2, C t3) {
+                            C v = mul(t0, a.op.st[0]);
+                            v = add(v, mul(t1, a.op.st[1]));
+                            v = add(v, mul(t2, a.op.st[2]));
+                            return add(v, mul(t3, a.op.st[3]));
+                        };
+                        const C w0 = tap4(p[-1], z, p1, p2), w1 = tap4(z, p1, p2, p[3]);
+                        C e[N];
+                        vget(vy, e);
+#pragma unroll
+                        for (int i = 0; i < N; i++) e[i] = c + i == lc ? w0 : (c + i == lc + 1 ? w1 : e[i]);
+                        vy = vset(e);
+                    }
+                    r_ = st.add(r_, mul(vy, P_));
+                    V s = vld(q + F_NM * P);
+                    vupdate<CPST, C>(st, s, r_, cc);
+                    if (r == srcNM) source(s);
+                    vst(q + F_NM * P, s);
+                    if constexpr (RES) vst(q + F_NM * P + o_r, KR ? r_ : cc);
+                    if constexpr (ENERGY) {
+                        C e[N];
+                        vget(s, e);
+#pragma unroll
+                        for (int i = 0; i < N; i++)
+                            if (orow && i < ownM) ek = add(ek, mul(mul((double)e[i], wv.w[i]), (double)e[i]));
+                    }
+                }
+        };
+        if (vcol) {
+            if (vpair) {   // two rows at a time: their x stencils share all but one row
+                for (int r = va + 2 * slot; r < vb; r += 2 * SLOTS) {
+                    C *q = at(0, r, c);
+                    V nn[5], m0[5];
+#pragma unroll
+                    for (int w = 0; w < 5; w++) {
+                        nn[w] = vld(q + F_NN * P + (w - 1) * RS);
+                        m0[w] = vld(q + F_MM0 * P + (w - 2) * RS);
+                    }
+                    vrow(r, q, [&](int f, int o) { return f == F_NN ? nn[o + 1] : m0[o + 2]; });
+                    if (r + 1 < vb) vrow(r + 1, q + RS, [&](int f, int o) { return f == F_NN ? nn[o + 2] : m0[o + 3]; });
+                }
+            } else {
+                for (int r = va + slot; r < vb; r += dslot) {
+                    C *q = at(0, r, c);
+                    vrow(r, q, [&](int f, int o) { return vld(q + f * P + o * RS); });
+                }
+            }
+        }
+        __syncthreads();
+        for (int q = rb + tid; q < re; q += RES_THREADS) {   // velocity receivers (the velocities rest during S)
+            const int *e = a.rcv + 4 * q;
+            if (e[0] == F_MN || e[0] == F_NM)
+                a.traces[(long)e[3] * a.max_steps + it] = (double)*at(e[0], e[1] - x0, e[2] - y0);
+        }
+        // ---- S: stresses of the owned points; those near an edge also to the exchange words
+        const unsigned tag = a.tag0 + (unsigned)k + 1u;
+        u64 *xb = a.xbuf + (size_t)(tag & 1u) * 3 * a.xarr;
+        auto send = [&](int r, int own, int f3, const V &v) {
+            C e[N];
+            vget(v, e);
+            u64 *p = xb + f3 * a.xarr + ((x0 + r) * a.xcols + y0 + c) * XW;
+            if (own >= N) {
+                xstv(p, e, tag);
+            } else {
+#pragma unroll
+                for (int q = 0; q < N - 1; q++)
+                    if (q < own) xst(p + q * XW, e[q], tag);
+            }
+        };
+        auto srow = [&](int r, C *q, auto ld) {
+                const int i = x0 + r;
+                [[maybe_unused]] const long go = (long)i * a.pitch + y0 + c;
+                auto coefv = [&](int f) -> V {
+                    if constexpr (CS) return vld(q + f * P + o_c);
+                    else return vldg(a.coef[f] + go);
+                };
+                const bool border = !last && multi && (bcol || r < 3 || r >= R - 3);
+                if (first) {   // NN: x from MN, y from NM
+                    [[maybe_unused]] WV wv;
+                    if constexpr (ENERGY) wv = weights(F_NN, r, true);
+                    const V P_ = coefv(F_NN);
+                    V r_ = vzero(C(0)), cc = r_, vx;
+                    if constexpr (KR) r_ = vld(q + F_NN * P + o_r);
+                    if constexpr (KC) cc = vld(q + F_NN * P + o_r);
+                    if (i >= 4 && i < Mx - 3)
+                        vx = taps<C>(st, ld(F_MN, -2), ld(F_MN, -1), ld(F_MN, 0), ld(F_MN, 1));
+                    else
+                        vx = vdxM_end<C>(ends, st, Mx, i, [&](int g) { return vld(at(F_MN, g - x0, c)); });
+                    r_ = st.add(r_, mul(vx, P_));
+                    r_ = st.add(r_, mul(dyN(st, q + F_NM * P, ld(F_NM, 0)), P_));
+                    const V old = vld(q + F_NN * P);
+                    V s = old;
+                    vupdate<CPST, C>(st, s, r_, cc);
+                    if (r == srcNN) source(s);
+                    vst(q + F_NN * P, s);
+                    if constexpr (RES) vst(q + F_NN * P + o_r, KR ? r_ : cc);
+                    if (border) send(r, ownN, 0, s);
+                    if constexpr (ENERGY) {
+                        C e[N], o[N];
+                        vget(s, e);
+                        vget(old, o);
+#pragma unroll
+                        for (int m = 0; m < N; m++)
+                            if (m < ownN) {
+                                if (k == 0) ep0 = add(ep0, mul(mul((double)o[m], wv.w[m]), (double)o[m]));
+                                ep1 = add(ep1, mul(mul((double)e[m], wv.w[m]), (double)e[m]));
+                            }
+                    }
+                }
+                if (second && r < R && ownM > 0) {   // MM: x from NM, y from MN
+                    [[maybe_unused]] WV wv3, wv4;
+                    if constexpr (ENERGY) { wv3 = weights(F_MM0, r, true); wv4 = weights(F_MM1, r, true); }
+                    const V L = coefv(F_MM0), M2 = coefv(F_MM1);
+                    V r0 = vzero(C(0)), r1 = r0, k0 = r0, k1 = r0, vx;
+                    if constexpr (KR) { r0 = vld(q + F_MM0 * P + o_r); r1 = vld(q + F_MM1 * P + o_r); }
+                    if constexpr (KC) { k0 = vld(q + F_MM0 * P + o_r); k1 = vld(q + F_MM1 * P + o_r); }
+                    if (i >= 3 && i < Mx - 3)
+                        vx = taps<C>(st, ld(F_NM, -1), ld(F_NM, 0), ld(F_NM, 1), ld(F_NM, 2));
+                    else
+                        vx = vdxN_end<C>(ends, st, Mx, i, [&](int g) { return vld(at(F_NM, g - x0, c)); });
+                    r0 = st.add(r0, mul(vx, L));
+                    r1 = st.add(r1, mul(vx, L));
+                    r0 = st.add(r0, mul(vx, M2));
+                    const V vy = dyM(st, q + F_MN * P, ld(F_MN, 0), false, nullptr);
+                    r0 = st.add(r0, mul(vy, L));
+                    r1 = st.add(r1, mul(vy, L));
+                    r1 = st.add(r1, mul(vy, M2));
+                    const V o0 = vld(q + F_MM0 * P), o1 = vld(q + F_MM1 * P);
+                    V s0 = o0, s1 = o1;
+                    vupdate<CPST, C>(st, s0, r0, k0);
+                    vupdate<CPST, C>(st, s1, r1, k1);
+                    if (r == srcMM) {
+                        source(s0);
+                        source(s1);
+                    }
+                    vst(q + F_MM0 * P, s0);
+                    vst(q + F_MM1 * P, s1);
+                    if constexpr (RES) {
+                        vst(q + F_MM0 * P + o_r, KR ? r0 : k0);
+                        vst(q + F_MM1 * P + o_r, KR ? r1 : k1);
+                    }
+                    if (border) {
+                        send(r, ownM, 1, s0);
+                        send(r, ownM, 2, s1);
+                    }
+                    if constexpr (ENERGY) {
+                        C e0[N], e1[N], p0[N], p1[N];
+                        vget(s0, e0);
+                        vget(s1, e1);
+                        vget(o0, p0);
+                        vget(o1, p1);
+#pragma unroll
+                        for (int m = 0; m < N; m++)
+                            if (m < ownM) {
+                                const double w3 = wv3.w[m], w4 = wv4.w[m];
+                                auto pot = [&](double b0, double b1, double &E) {
+                                    E = add(E, mul(mul(b0, w3), b0));
+                                    E = add(E, mul(mul(b1, w3), b1));
+                                    E = add(E, mul(mul(b0, w4), b1));
+                                };
+                                if (k == 0) pot((double)p0[m], (double)p1[m], ep0);
+                                pot((double)e0[m], (double)e1[m], ep1);
+                            }
+                    }
+                }
+        };
+        if (scol) {
+            if (vpair) {
+                for (int r = 2 * slot; r < RN; r += 2 * SLOTS) {
+                    C *q = at(0, r, c);
+                    V mn[5], nm[5];
+#pragma unroll
+                    for (int w = 0; w < 5; w++) {
+                        mn[w] = vld(q + F_MN * P + (w - 2) * RS);
+                        nm[w] = vld(q + F_NM * P + (w - 1) * RS);
+                    }
+                    srow(r, q, [&](int f, int o) { return f == F_MN ? mn[o + 2] : nm[o + 1]; });
+                    if (r + 1 < RN) srow(r + 1, q + RS, [&](int f, int o) { return f == F_MN ? mn[o + 3] : nm[o + 2]; });
+                }
+            } else {
+                for (int r = slot; r < RN; r += dslot) {
+                    C *q = at(0, r, c);
+                    srow(r, q, [&](int f, int o) { return vld(q + f * P + o * RS); });
+                }
+            }
+        }
+        if constexpr (ENERGY) {   // each warp's sums; the CTA's are added up after the barrier
+            double v3[3] = {ep0, ek, ep1};
+#pragma unroll
+            for (int q = 0; q < 3; q++) {
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) v3[q] += __shfl_down_sync(0xffffffffu, v3[q], o);
+                if ((tid & 31) == 0) red[k & 1][q][tid >> 5] = v3[q];
+            }
+        }
+        __syncthreads();
+        for (int q = rb + tid; q < re; q += RES_THREADS) {   // stress receivers (the owned stresses rest until S)
+            const int *e = a.rcv + 4 * q;
+            if (e[0] != F_MN && e[0] != F_NM)
+                a.traces[(long)e[3] * a.max_steps + it] = (double)*at(e[0], e[1] - x0, e[2] - y0);
+        }
+        if constexpr (ENERGY) {
+            if (tid < 3 && it < a.max_steps) {
+                double v = 0.;
+                for (int w = 0; w < RES_THREADS / 32; w++) v += red[k & 1][tid][w];
+                // the stresses before this step are those after the last one
+                if (tid == 0 && k > 0) v = ep_prev;
+                if (v != 0.) atomicAdd(a.energy + (long)tid * a.max_steps + it, 0.5 * v);
+                ep_prev = __shfl_sync(0x7u, v, 2);
+            }
+        }
+        if (last) break;
+        // ---- X: the halo's stresses
+        if (multi) {
+            // a thread's words are polled together: one round trip when the neighbours are done (an
+            // item at a time in FP64 and with the energy on, where the registers are short)
+            constexpr int B = sizeof(C) == 8 || ENERGY ? 1 : XI;
+            bool ok = true;
+#pragma unroll
+            for (int b = 0; b < XI; b += B) {
+                if (!ok || xs[b] < 0) break;
+                XV<C> v[B][3];
+                ok = false;
+                for (int n = 0; n < X_POLLS && !ok; n++) {
+#pragma unroll
+                    for (int m = 0; m < B; m++) {
+                        if (xs[b + m] >= 0) v[m][0].load(xb + xg[b + m]);
+                        if (xm[b + m] >= 0) {
+                            v[m][1].load(xb + a.xarr + xh[b + m]);
+                            v[m][2].load(xb + 2 * a.xarr + xh[b + m]);
+                        }
+                    }
+                    ok = true;
+#pragma unroll
+                    for (int m = 0; m < B; m++) {
+                        if (xs[b + m] >= 0) ok = ok && v[m][0].ok(tag);
+                        if (xm[b + m] >= 0) ok = ok && v[m][1].ok(tag) && v[m][2].ok(tag);
+                    }
+                }
+                if (ok) {
+#pragma unroll
+                    for (int m = 0; m < B; m++) {
+                        if (xs[b + m] >= 0) sm[xs[b + m]] = v[m][0].get();
+                        if (xm[b + m] >= 0) {
+                            sm[xm[b + m]] = v[m][1].get();
+                            sm[xm[b + m] + P] = v[m][2].get();
+                        }
+                    }
+                }
+            }
+            if (!ok) bad_s = 1;
+        } else {   // one tile: the periodic columns from the tile itself
+            for (int idx = tid; idx < RN * 6; idx += RES_THREADS) {
+                const int r = idx / 6, q = idx - 6 * r;
+                const int cn = q < 3 ? q - 3 : WN + q - 3, cm = cn >= WN ? cn - 1 : cn;
+                *at(F_NN, r, cn) = *at(F_NN, r, phys(true, cn));
+                if (r < R) {
+                    *at(F_MM0, r, cm) = *at(F_MM0, r, phys(false, cm));
+                    *at(F_MM1, r, cm) = *at(F_MM1, r, phys(false, cm));
+                }
+            }
+            for (int r = tid; r < RN; r += RES_THREADS) {
+                altL[r + H] = *at(F_NN, r, lc);
+                altR[r + H] = *at(F_NN, r, 0);
+            }
+        }
+        __syncthreads();
+        if (bad_s) break;
+    }
+    // ---- the state after the run. (A value that stopped being finite at any step has stayed so: an
+    // update adds to it.)
+    C nf = C(0);   // stays 0 until a value is not finite (v * 0 is NaN then)
+    for (int f = 0; f < 5; f++) {
+        const int rows = f == F_NN || f == F_NM ? RN : R, cols = ntypeY(f) ? WN : W;
+        for (int k = tid; k < rows * RES_LANES_COLS; k += RES_THREADS) {
+            const int r = k / RES_LANES_COLS, cc = k - r * RES_LANES_COLS;
+            if (cc >= cols) continue;
+            const C *q = at(f, r, cc);
+            const long o = (long)(x0 + r) * a.pitch + y0 + cc;
+            nf = nf + q[0] * C(0);
+            a.out[f][o] = q[0];
+            if constexpr (RES) a.rout[f][o] = q[o_r];
+        }
+    }
+    if (tid == 0 && bad_s) atomicOr(a.flags, FLAG_TIMEOUT);
+    if (nf != C(0)) atomicOr(a.flags, FLAG_NONFINITE);
+    // the last CTA advances the step counter, after every CTA has read it
+    __syncthreads();
+    if (tid == 0) {
+        __threadfence();
+        if (atomicAdd(a.done, 1) == (int)gridDim.x - 1) {
+            *a.done = 0;
+            *a.step_w = it0 + a.n;
+            __threadfence();
+        }
+    }
+}
+
+// ------------------------------------------------------------------------------- launcher
+template <class C, class F>
+cudaError_t resident_kernel(int cpst, bool energy, bool cs, F f)
+{
+    // codes 1 / 3 and 2 / 4 are the same update; coefficients stay in L2 for the plain update only
+    if (cpst == 0) {
+        if (cs) return energy ? f(k_resident<C, 0, true, true>) : f(k_resident<C, 0, false, true>);
+        return energy ? f(k_resident<C, 0, true, false>) : f(k_resident<C, 0, false, false>);
+    }
+    if (cpst == 1 || cpst == 3) return energy ? f(k_resident<C, 3, true, true>) : f(k_resident<C, 3, false, true>);
+    if (cpst == 2 || cpst == 4) return energy ? f(k_resident<C, 4, true, true>) : f(k_resident<C, 4, false, true>);
+    if (cpst == 5) return energy ? f(k_resident<C, 5, true, true>) : f(k_resident<C, 5, false, true>);
+    return energy ? f(k_resident<C, 6, true, true>) : f(k_resident<C, 6, false, true>);
+}
+
+template <class C>
+cudaError_t prepare_resident(int cpst, bool energy, const ResPlan &p)
+{
+    return resident_kernel<C>(cpst, energy, p.cs, [&](auto k) {
+        return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
+    });
+}
+
+template <class C>
+cudaError_t launch_resident(const ResArgs<C> &a, int cpst, bool energy, const ResPlan &p, cudaStream_t st)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(p.ntx * p.nty);
+    cfg.blockDim = dim3(RES_THREADS);
+    cfg.dynamicSmemBytes = p.smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];   // CTAs poll their neighbours' words: all must be resident
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = p.ntx * p.nty > 1 ? 1 : 0;
+    return resident_kernel<C>(cpst, energy, p.cs, [&](auto k) { return cudaLaunchKernelEx(&cfg, k, a); });
+}
+
+}  // namespace tw

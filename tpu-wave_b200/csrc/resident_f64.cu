@@ -1,0 +1,7 @@
+// On-chip runs of the elastic step (resident.cuh) for FP64 fields.
+#include "resident.cuh"
+
+namespace tw {
+template cudaError_t prepare_resident<double>(int, bool, const ResPlan &);
+template cudaError_t launch_resident<double>(const ResArgs<double> &, int, bool, const ResPlan &, cudaStream_t);
+}  // namespace tw

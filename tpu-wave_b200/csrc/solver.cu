@@ -123,6 +123,17 @@ struct tw_solver {
     // warps, receivers as one flat list in d_rcv_list
     bool afused = false;
     bool pfuse = false;               // double-buffered periodic acoustic: may join a fused batch
+    // grids that fit on the chip: a run of tw_step is one launch (resident.cuh); the handle's other
+    // step kernels serve single steps elsewhere (the adjoint's sweeps, captured streams)
+    ResPlan res_plan;                 // ntx 0: the grid does not fit
+    unsigned res_tag = 0;             // steps run this way since the exchange words were cleared
+    unsigned long long *xbuf = nullptr;
+    size_t xbuf_bytes = 0;
+    void *coefx[2] = {};              // (coefficients in L2) 1/rho with periodic columns around
+    long xpitch = 0;
+    bool coefx_dirty = true;
+    int *d_rcv_off_r = nullptr, *d_rcv_list_r = nullptr;
+    int rcv_list_cap_r = 0;
     int bnd = 0;                      // BND_X_IF | BND_Y_SAT (stepper.cuh): two-launch kernels
     tw_solver *link[2] = {};          // during tw_slab_run: the slabs above / below
     int n_rcv_list = 0;
@@ -220,6 +231,7 @@ tw_solver::~tw_solver()
     for (int k = 0; k < 5; k++) { release(f2[k]); release(res2[k]); }
     release(d_done); release(d_rcv_off); release(d_rcv_list); release(model);
     release(d_rcv_off_w); release(d_rcv_list_w);
+    release(xbuf); release(coefx[0]); release(coefx[1]); release(d_rcv_off_r); release(d_rcv_list_r);
     release(src_inc); release(d_step); release(d_flags); release(d_rcv); release(d_err);
     release(d_traces); release(d_energy);
     for (int k = 0; k < 5; k++) release(coefq[k]);
@@ -548,6 +560,65 @@ void enqueue(tw_solver *s, int n, cudaStream_t st)
     else enqueue_steps<float, float>(s, n, st);
 }
 
+// n steps on chip, from the current buffers into the other ones
+template <class C>
+int run_resident(tw_solver *s, int n, cudaStream_t st)
+{
+    const ResPlan &p = s->res_plan;
+    if (s->res_tag > 0xffffffffu - (unsigned)n - 2u) {   // the tags would wrap: start over
+        TW_CUDA(cudaMemsetAsync(s->xbuf, 0, s->xbuf_bytes, st));
+        s->res_tag = 0;
+    }
+    if (!p.cs && s->coefx_dirty) {
+        for (int k = 0; k < 2; k++)
+            launch_pad_columns<C>((const C *)s->coef[F_MN + k], s->pitch, (C *)s->coefx[k], s->xpitch, s->rows[F_MN + k],
+                                  (int)s->d.My, k == 0, st);
+        s->coefx_dirty = false;
+    }
+    ResArgs<C> a{};
+    void *const *fin = s->parity ? s->f2 : s->f, *const *fout = s->parity ? s->f : s->f2;
+    void *const *rin = s->parity ? s->res2 : s->res, *const *rout = s->parity ? s->res : s->res2;
+    for (int k = 0; k < 5; k++) {
+        a.in[k] = (const C *)fin[k];
+        a.out[k] = (C *)fout[k];
+        a.rin[k] = (const C *)rin[k];
+        a.rout[k] = (C *)rout[k];
+        a.coef[k] = (const C *)s->coef[k];
+        a.w[k] = s->w[k];
+    }
+    a.coefx[0] = (const C *)s->coefx[0];
+    a.coefx[1] = (const C *)s->coefx[1];
+    a.xpitch = s->xpitch;
+    a.pitch = s->pitch;
+    a.Mx = (int)s->d.Mx;
+    a.My = (int)s->d.My;
+    a.op = make_ops<C>((double)s->d.num_dx / (double)s->d.den_dx, s->d.dt, false);
+    a.ntx = p.ntx;
+    a.nty = p.nty;
+    a.rows_s = p.rows_s;
+    a.n = n;
+    a.tag0 = s->res_tag;
+    a.xbuf = s->xbuf;
+    a.xcols = (int)(s->d.My + 2) & ~1;   // (even: pairs of words are written whole)
+    a.xarr = (s->d.Mx + 1) * (long)a.xcols * (long)(sizeof(C) / 4);
+    a.src_inc = s->src_inc;
+    a.src_grid = s->src_grid;
+    a.src_ix = (int)s->src_ix;
+    a.src_iy = (int)s->src_iy;
+    a.step = a.step_w = s->d_step;
+    a.done = s->d_done;
+    a.flags = s->d_flags;
+    a.max_steps = s->d.max_steps;
+    a.energy = s->d_energy;
+    a.rcv_off = s->d_rcv_off_r;
+    a.rcv = s->d_rcv_list_r;
+    a.traces = s->d_traces;
+    TW_CUDA(launch_resident<C>(a, s->d.cpst, s->d.energy != 0, p, st));
+    s->res_tag += (unsigned)n;
+    s->parity ^= 1;
+    return TW_OK;
+}
+
 // stepping coefficients and energy weights from the FP64 material arrays
 int finalize_material(tw_solver *s)
 {
@@ -598,6 +669,7 @@ int finalize_material(tw_solver *s)
                 return cuda_fail(cudaGetLastError(), "coefficient codes");
     s->mat_dirty = false;
     s->mat_ready = true;
+    s->coefx_dirty = true;
     return TW_OK;
 }
 
@@ -701,6 +773,33 @@ int upload_receivers(tw_solver *s)
         int rc = build(false, s->d_rcv_off, &s->d_rcv_list, &s->rcv_list_cap);
         if (rc == TW_OK && s->tma) rc = build(true, s->d_rcv_off_w, &s->d_rcv_list_w, &s->rcv_list_cap_w);
         if (rc != TW_OK) return rc;
+    }
+    if (s->res_plan.ntx > 0) {   // the same by tile of the on-chip run
+        const int nt = s->res_plan.ntx * s->res_plan.nty;
+        std::vector<std::vector<int>> per(nt);
+        for (int r = 0; r < n; r++) {
+            const int *q = &s->rcv_tab[4 * r];
+            const int t = resident_tile(s->res_plan, s->d.Mx, s->d.My, q[2], q[3]);
+            for (int f = 0; f < 2; f++)
+                if (q[f] >= 0) per[t].insert(per[t].end(), {q[f], q[2], q[3], 2 * r + f});
+        }
+        std::vector<int> off(nt + 1, 0), list;
+        for (int t = 0; t < nt; t++) {
+            off[t + 1] = off[t] + (int)per[t].size() / 4;
+            list.insert(list.end(), per[t].begin(), per[t].end());
+        }
+        if ((int)list.size() > s->rcv_list_cap_r) {
+            s->release(s->d_rcv_list_r);
+            s->d_rcv_list_r = nullptr;
+            int cap = 64;
+            while (cap < (int)list.size()) cap *= 2;
+            if (s->alloc((void **)&s->d_rcv_list_r, sizeof(int) * cap) != TW_OK) return TW_ERR_NOMEM;
+            s->rcv_list_cap_r = cap;
+        }
+        TW_CUDA(cudaMemcpyAsync(s->d_rcv_off_r, off.data(), sizeof(int) * off.size(), cudaMemcpyHostToDevice, s->st));
+        if (!list.empty())
+            TW_CUDA(cudaMemcpyAsync(s->d_rcv_list_r, list.data(), sizeof(int) * list.size(), cudaMemcpyHostToDevice, s->st));
+        TW_CUDA(cudaStreamSynchronize(s->st));   // (the host vectors leave scope)
     }
     if (s->pfuse) {   // (field slot, row, column, trace row) per recorded field, for the fused steps
         std::vector<int> list;
@@ -1139,6 +1238,33 @@ int create_impl(tw_solver **out, const tw_grid_desc *desc, const SlabSpec &sl)
             cudaMemsetAsync(s->d_rcv_off_w, 0, sizeof(int) * (nw + 1), s->st);
         }
     }
+    // on-chip runs: FP32 / FP64 storage and coefficients, the reference's boundaries, a handle of its
+    // own (not a slab), a grid that fits on the SMs. TW_TMA / TW_RESIDENT=0 select the other
+    // kernels for comparisons, TW_RES_NTX / TW_RES_NTY a tiling.
+    if (s->fused && !s->slab && !s->bnd && !d.coef_fp16 && (d.precision == TW_FP64 || d.precision == TW_FP32) &&
+        !std::getenv("TW_TMA") && env_int("TW_RESIDENT", 1) != 0) {
+        int n_sm = 0, smem_max = 0, coop = 0;
+        cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, d.device);
+        cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, d.device);
+        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, d.device);
+        const ResPlan p = coop ? resident_plan(Mx, My, s->esz, cp, n_sm, (size_t)std::max(0, smem_max - 2048)) : ResPlan{};
+        if (p.ntx > 0) {
+            e = d.precision == TW_FP64 ? prepare_resident<double>(d.cpst, d.energy != 0, p) : prepare_resident<float>(d.cpst, d.energy != 0, p);
+            if (e != cudaSuccess) return fail(cuda_fail(e, "cudaFuncSetAttribute"));
+            if (p.ntx * p.nty > 1) {
+                s->xbuf_bytes = (size_t)6 * (Mx + 1) * ((My + 2) & ~1L) * 2 * s->esz;
+                if ((rc_ = s->alloc((void **)&s->xbuf, s->xbuf_bytes)) != TW_OK) return fail(rc_);
+                cudaMemsetAsync(s->xbuf, 0, s->xbuf_bytes, s->st);
+            }
+            if (!p.cs) {
+                s->xpitch = (My + 16 + 3) / 4 * 4;
+                for (int k = 0; k < 2; k++)
+                    if ((rc_ = s->alloc(&s->coefx[k], (size_t)s->rows[F_MN + k] * s->xpitch * s->esz)) != TW_OK) return fail(rc_);
+            }
+            if ((rc_ = s->alloc((void **)&s->d_rcv_off_r, sizeof(int) * (p.ntx * p.nty + 1))) != TW_OK) return fail(rc_);
+            s->res_plan = p;
+        }
+    }
     if (!s->elastic && s->periodic && !d.energy) {
         // periodic acoustic with energy off: a second copy of the state, for the fused step of a
         // batch and, on grids of 2^20 points or more, of the handle alone (below that the
@@ -1394,6 +1520,16 @@ int tw_step(tw_solver *s, int n)
     if (s->steps_done + (long)n > s->d.max_steps) return TW_ERR_RECORD_FULL;
     if (n == 0) return TW_OK;
     TW_CUDA(cudaSetDevice(s->d.device));
+    if (s->res_plan.ntx > 0) {
+        // (a captured run would be replayed with the tags of its first run)
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        TW_CUDA(cudaStreamIsCapturing(s->st, &cap));
+        if (cap == cudaStreamCaptureStatusNone) {
+            const int rc = s->d.precision == TW_FP64 ? run_resident<double>(s, n, s->st) : run_resident<float>(s, n, s->st);
+            if (rc == TW_OK) s->steps_done += n;
+            return rc;
+        }
+    }
     // a graph of G steps captured once and replayed; leftover steps are launched directly. The
     // graph is captured on the first call of any length when the records hold G steps, so that
     // a short first call (a warm-up) leaves the next long call only replays and direct launches.
