@@ -257,6 +257,33 @@ int quantize_coefficients16(float *coef, unsigned short *codes, int rows, int co
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
+// ---------------------------------------------------------------- readback
+// bound by the host link behind it: one value a thread, rows over the grid
+template <class S>
+__global__ void __launch_bounds__(256) k_to_f64(const S *in, const S *lo, long pitch, double *out, long rows, long cols)
+{
+    for (long r = blockIdx.y; r < rows; r += gridDim.y)
+        for (long c = blockIdx.x * (long)blockDim.x + threadIdx.x; c < cols; c += (long)gridDim.x * blockDim.x) {
+            const long i = r * pitch + c;
+            if constexpr (sizeof(S) == 2) {
+                const float h = to_c<float>(in[i]);
+                out[r * cols + c] = (double)(lo ? add(h, to_c<float>(lo[i])) : h);
+            } else {
+                out[r * cols + c] = (double)in[i];
+            }
+        }
+}
+template <class S>
+void launch_to_f64(const S *in, const S *lo, long pitch, double *out, long rows, long cols, cudaStream_t st)
+{
+    const dim3 g((unsigned)((cols + 255) / 256 < 1024 ? (cols + 255) / 256 : 1024), (unsigned)(rows < 16384 ? rows : 16384));
+    k_to_f64<S><<<g, 256, 0, st>>>(in, lo, pitch, out, rows, cols);
+}
+template void launch_to_f64<double>(const double *, const double *, long, double *, long, long, cudaStream_t);
+template void launch_to_f64<float>(const float *, const float *, long, double *, long, long, cudaStream_t);
+template void launch_to_f64<__nv_bfloat16>(const __nv_bfloat16 *, const __nv_bfloat16 *, long, double *, long, long, cudaStream_t);
+template void launch_to_f64<__half>(const __half *, const __half *, long, double *, long, long, cudaStream_t);
+
 // ---------------------------------------------------------------- discrete energy (FP64)
 __device__ __forceinline__ double warp_sum(double v)
 {

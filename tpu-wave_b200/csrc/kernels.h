@@ -72,6 +72,10 @@ void launch_material_finalize(const MaterialArgs &m, cudaStream_t st);
 int quantize_coefficients16(float *coef, unsigned short *codes, int rows, int cols, long pitch, unsigned *d_mm,
                             float *lo, float *step, cudaStream_t st);
 
+// rows x cols values of a pitched array as compact doubles (with `lo`: the FP32 sums hi + lo)
+template <class S>
+void launch_to_f64(const S *in, const S *lo, long pitch, double *out, long rows, long cols, cudaStream_t st);
+
 template <class S, class C>
 struct EnergyArgs {
     const S *a[4];            // up to four terms sum_i a_i w_i b_i over rows x My
