@@ -11,7 +11,7 @@ several; energies to 1e-12 (FP64 sums in another order).
 import numpy as np
 import pytest
 
-from cases import elastic_case, product_elastic
+from cases import acoustic_periodic_case, elastic_case, product_acoustic_periodic, product_elastic
 from oracle import oracle as orc
 from test_tma_gpu import _rcv
 
@@ -129,3 +129,110 @@ def test_a_value_that_is_not_finite_is_reported(tw):
     s.run(3)
     assert not s.read_field(tw.MM).any()
     s.close()
+
+
+AC_GRIDS = [(24, 20, (1, 1)), (24, 21, (3, 1)), (25, 22, (1, 2)), (40, 35, (5, 4)), (97, 61, (1, 2)), (64, 57, (2, 1)), (130, 171, None)]
+
+
+@pytest.mark.parametrize("cpst", ["0", "3", "6"])
+@pytest.mark.parametrize("prec", ["f32", "f64"])
+@pytest.mark.parametrize("Mx,My,tiles", AC_GRIDS)
+def test_acoustic_periodic_run(Mx, My, tiles, prec, cpst, monkeypatch):
+    case = acoustic_periodic_case(Mx, My, seed=Mx + My, cpst=cpst, Nt=7)
+    rng = np.random.default_rng(Mx * My)
+    f0 = [rng.standard_normal(s).astype(np.float32).astype(np.float64) for s in ((Mx + 1, My), (Mx, My + 1), (Mx, My))]
+    r0 = [a * 1e-6 for a in f0] if cpst != "0" else None
+    if tiles is not None:
+        monkeypatch.setenv("TW_RES_NTX", str(tiles[0]))
+        monkeypatch.setenv("TW_RES_NTY", str(tiles[1]))
+    got = product_acoustic_periodic(case, prec, fields0=f0, resid0=r0, energy=False)
+    monkeypatch.setenv("TW_RESIDENT", "0")
+    one = product_acoustic_periodic(case, prec, fields0=f0, resid0=r0, energy=False)
+    two = product_acoustic_periodic(case, prec, fields0=f0, resid0=r0, energy=True)   # the two-launch kernels
+    for k, v in got["fields"].items():
+        assert np.array_equal(v, one["fields"][k]) and np.array_equal(v, two["fields"][k]), k
+    assert np.array_equal(got["traces"], one["traces"]) and np.array_equal(got["traces"], two["traces"])
+    for a, b in zip(got.get("resid") or [], one.get("resid") or []):
+        assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("cpst", ["00", "3C", "3R", "6C", "6R"])
+@pytest.mark.parametrize("prec", ["f32", "f64"])
+@pytest.mark.parametrize("Mx,My,tiles", AC_GRIDS)
+def test_acoustic_free_surface_run(Mx, My, tiles, prec, cpst, monkeypatch):
+    """These handles hold one copy of the state: a run ends in the buffer it began in."""
+    den = max(Mx, My)
+    rcvs = [_rcv("M", "M", r, c, den) for r in (0, 8, Mx - 1) for c in (0, 8, My - 1)]
+    case = elastic_case(Mx, My, seed=5, cpst=cpst, Nt=7, rcvs=rcvs, den_dx=den, acoustic=True)
+    rng = np.random.default_rng(Mx * My)
+    f0 = [rng.standard_normal(s).astype(np.float32).astype(np.float64) for s in ((Mx, My + 1), (Mx + 1, My), (Mx, My))]
+    if tiles is not None:
+        monkeypatch.setenv("TW_RES_NTX", str(tiles[0]))
+        monkeypatch.setenv("TW_RES_NTY", str(tiles[1]))
+    got = product_elastic(case, prec, acoustic=True, fields0=f0, energy=False)
+    monkeypatch.setenv("TW_RESIDENT", "0")
+    one = product_elastic(case, prec, acoustic=True, fields0=f0, energy=False)
+    _same(got, one, False)
+
+
+@pytest.mark.parametrize("bc", ["periodic", "free"])
+def test_acoustic_runs_in_several_calls_and_in_a_batch(tw, bc, monkeypatch):
+    """Single steps, runs and batch steps mixed on the same handles equal the per-point kernels."""
+    Mx, My = 60, 75
+
+    def run(calls, resident, batch_at=None):
+        monkeypatch.setenv("TW_RESIDENT", "1" if resident else "0")
+        shots = []
+        for k in range(2):
+            s = tw.Solver(Mx, My, 1, My, 1e-3, physics=tw.ACOUSTIC, bc_x=tw.PERIODIC if bc == "periodic" else tw.SAT_FREE,
+                          precision="f32", max_steps=40, energy=False)
+            rng = np.random.default_rng(k)
+            s.set_material_grid(tw.NM, 0, rng.uniform(1, 2, (Mx + 1, My)))
+            s.set_material_grid(tw.MN, 0, rng.uniform(1, 2, (Mx, My + 1)))
+            s.set_material_grid(tw.MM, 0, rng.uniform(1, 2, (Mx, My)))
+            s.set_source(tw.NM if bc == "periodic" else tw.MM, 1, 1)
+            s.add_receivers(tw.MM, [0, 30, 59], [0, 8, 74])
+            s.write_field(tw.MM, 0, rng.standard_normal((Mx, My)))
+            shots.append(s)
+        b = tw.Batch(shots)
+        for i, n in enumerate(calls):
+            if i == batch_at:
+                b.step(3)
+            for s in shots:
+                s.step(n)
+        b.sync()
+        out = [[s.read_field(g) for g in (tw.MN, tw.NM, tw.MM)] + [s.read_receivers()] for s in shots]
+        b.close()
+        for s in shots:
+            s.close()
+        return out
+
+    for calls, at in (([20], None), ([1, 7, 2, 1, 6], None), ([5, 1, 8], 1), ([4, 4], 1)):
+        for x, y in zip(run(calls, True, at), run(calls, False, at)):
+            for p, q in zip(x, y):
+                assert np.array_equal(p, q), (calls, at)
+
+
+def test_handles_of_different_sizes_side_by_side(tw):
+    """Handles share the kernels: one made later, smaller, must not take shared memory from another."""
+    sizes = [(300, 330), (24, 20), (700, 640), (40, 60)]
+    shots = []
+    for Mx, My in sizes:
+        s = tw.Solver(Mx, My, 1, My, 1e-4, precision="f32", max_steps=8, energy=False)
+        rng = np.random.default_rng(Mx)
+        P = (Mx + 2, My + 2)
+        s.set_material_model(rng.uniform(1.8, 2.7, P), rng.uniform(1.5, 4.5, P), rng.uniform(1., 2., P))
+        s.write_field(tw.MM, 0, rng.standard_normal((Mx, My)))
+        shots.append(s)
+    alone = []
+    for s in shots:
+        s.run(4)
+        alone.append(s.read_field(tw.MM, 0))
+    assert all(np.isfinite(a).all() and np.abs(a).max() > 0 for a in alone)
+    for s in shots:   # queued together, on a stream each
+        s.step(2)
+    for s in shots:
+        s.step(2)
+    for s in shots:
+        s.sync()
+        s.close()

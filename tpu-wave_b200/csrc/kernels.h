@@ -215,10 +215,13 @@ void launch_tma(FusedArgs<S, C> a, const TmaMaps &maps, bool energy, cudaStream_
 constexpr int TMA_QW = TMA_W + 8;    // columns of a 16-bit coefficient box: from 8 before the strip's core
                                      // (a 16-byte boundary) to 4 beyond the 128 loaded field columns
 
-// on-chip runs of the elastic step (resident.cuh): many steps in one cooperative launch, ntx x nty
-// tiles of the grid, one CTA each, FP32 / FP64 storage, free-surface x ends, periodic y
+// on-chip runs (resident.cuh): many steps in one cooperative launch, ntx x nty tiles of the grid, one
+// CTA each, FP32 / FP64 storage, periodic y; elastic and acoustic with free-surface x ends, acoustic
+// with periodic x
+enum { RES_ELASTIC = 0, RES_AC_FREE = 1, RES_AC_PER = 2 };
 constexpr int RES_THREADS = 512;
 constexpr int RES_PAD = 4;            // rows / columns around a tile in shared memory
+constexpr int RES_STATIC = 2048;      // shared memory left to the kernel's own variables
 constexpr int RES_LANES_COLS = 64;    // columns a row's threads cover: 4 on the left, then up to RES_W
 constexpr int RES_W = 58;             // most columns of a tile (column My included)
 constexpr int RES_P = 68;             // values of a shared row (FP32 rows of 5 fields 1360 bytes apart: 13 or
@@ -241,7 +244,8 @@ struct ResArgs {
     int rows_s;               // rows of a tile's shared memory
     int n;                    // steps of this run
     unsigned tag0;            // steps the handle has run this way before: tags of the exchange words
-    unsigned long long *xbuf; // exchange words: [2][NN, MM0, MM1][(Mx + 1) x xcols], FP64 two words a value
+    unsigned long long *xbuf; // exchange words: [2][NN, MM0, MM1 (acoustic: MM0)][(Mx + 1) x xcols], FP64 two
+                              // words a value
     long xarr;                // words of one array
     int xcols;
     const double *src_inc;
@@ -264,12 +268,12 @@ struct ResPlan {
     size_t smem = 0;
 };
 // the tiling of a grid over n_sm SMs with smem_max bytes each
-ResPlan resident_plan(long Mx, long My, int esize, bool comp, int n_sm, size_t smem_max);
+ResPlan resident_plan(long Mx, long My, int esize, int fields, bool comp, int n_sm, size_t smem_max);
 // tile index of a point (host side receiver lists)
 int resident_tile(const ResPlan &p, long Mx, long My, int row, int col);
-template <class C>
-cudaError_t prepare_resident(int cpst, bool energy, const ResPlan &p);
-template <class C>
+template <class C, int PHYS>
+cudaError_t prepare_resident(int cpst, bool energy, const ResPlan &p, int smem_max);
+template <class C, int PHYS>
 cudaError_t launch_resident(const ResArgs<C> &a, int cpst, bool energy, const ResPlan &p, cudaStream_t st);
 // rows of `in` (cols periodic M- or N-type columns) with 4 more columns on the left and 8 on the right
 template <class C>

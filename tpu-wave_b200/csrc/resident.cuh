@@ -1,6 +1,6 @@
-// On-chip runs of the elastic step: many steps in one cooperative launch, each CTA keeping one
-// tile of the grid in shared memory, for grids that fit on the chip's SMs (FP32: up to about 1.1
-// million cells).
+// On-chip runs of the elastic and acoustic steps: many steps in one cooperative launch, each CTA keeping one
+// tile of the grid in shared memory, for grids that fit on the chip's SMs (FP32: elastic up to
+// about 1.1 million cells, acoustic 1.15 million).
 //
 // Such a grid is bound by latency, not by bytes: one launch a step leaves the machine idle
 // between launches, and a launch's first loads and its boundary strips are a serial chain of some
@@ -9,7 +9,8 @@
 // and the instructions of the largest tile. Us a step, one launch a step -> here (B200, FP32, energy
 // off): 48 x 40 29.1 -> 2.4, 200 x 150 27.2 -> 2.5, 509 x 317 28.9 -> 3.4, 700 x 700 30.7 -> 7.4, 1024 x 1024
 // 38.1 -> 15.7; with the energy 509 x 317 33.9 -> 4.8; FP64 509 x 317 30.9 -> 5.0, 700 x 700 32.7 -> 13.1;
-// '6C' 509 x 317 32.9 -> 3.9.
+// '6C' 509 x 317 32.9 -> 3.9. Acoustic FP32 (two launches and the receivers' before): periodic 256 x 256
+// 5.3 -> 1.8, 512 x 512 7.5 -> 2.3, 1000 x 1000 16.3 -> 4.6; free surface 512 x 512 8.5 -> 2.5.
 //
 // A tile owns rows [x0, x1) and columns [y0, y1) (the last tiles also the N-type row Mx and column
 // My). It holds the stresses with a halo of 3 points on each side and the velocities with 2, which
@@ -322,13 +323,19 @@ template <> struct XV<double> {
 // compensation code, then with CS the coefficients), so that every neighbour of a point is at a
 // compile-time distance from it. A row's vectors belong to LANES threads; a thread keeps its column
 // and walks down the rows, RES_THREADS / LANES rows apart (tall tiles: two rows at a time).
-template <class C, int CPST, bool ENERGY, bool CS>
+// PHYS: RES_ELASTIC, or acoustic (MN, NM and the pressure in MM0; only the pressure is exchanged, its halo
+// is a cross, nothing reads beyond an N-type seam): RES_AC_FREE the x free surfaces, RES_AC_PER
+// periodic x, whose halo rows are the rows at the other end.
+template <class C, int CPST, bool ENERGY, bool CS, int PHYS>
 __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_constant__ ResArgs<C> a)
 {
     constexpr bool KR = Cpst<CPST>::keep_r, KC = Cpst<CPST>::keep_c, RES = KR || KC;
     constexpr int N = Vec<C>::N, H = RES_PAD, P = RES_P, LANES = RES_LANES_COLS / N;
-    constexpr int NF = 5 + (RES ? 5 : 0) + (CS ? 5 : 0), RS = NF * P;
-    constexpr int o_r = 5 * P, o_c = (RES ? 10 : 5) * P;   // residual and coefficient rows
+    constexpr bool EL = PHYS == RES_ELASTIC, PERX = PHYS == RES_AC_PER;
+    constexpr int NB = EL ? 5 : 3;                         // fields
+    constexpr int NF = NB + (RES ? NB : 0) + (CS ? NB : 0), RS = NF * P;
+    constexpr int iNN = 0, iMN = EL ? 1 : 0, iNM = iMN + 1, iM0 = iNM + 1, iM1 = EL ? iM0 + 1 : iM0;   // (acoustic: syy is p)
+    constexpr int o_r = NB * P, o_c = (RES ? 2 : 1) * NB * P;   // residual and coefficient rows
     constexpr int XW = sizeof(C) / 4;                      // exchange words of a value
     using V = Vec<C>;
     extern __shared__ __align__(16) unsigned char res_smem[];
@@ -347,13 +354,22 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_consta
     const int RN = R + (lastx ? 1 : 0), WN = W + (lasty ? 1 : 0);
     C *sm = reinterpret_cast<C *>(res_smem);
     C *altL = sm + (size_t)a.rows_s * RS, *altR = altL + a.rows_s;
-    auto at = [&](int f, int r, int c) { return sm + (r + H) * RS + f * P + c + H; };
+    auto at = [&](int i, int r, int c) { return sm + (r + H) * RS + i * P + c + H; };   // i: iNN .. iM1
+    auto slot_of = [](int i) { return EL ? i : (i == iM0 ? (int)F_MM0 : i + F_MN); };
+    auto index_of = [](int f) { return EL ? f : (f == F_MM0 ? iM0 : f - F_MN); };
     auto ntypeY = [](int f) { return f == F_NN || f == F_MN; };
     auto rows_of = [&](int f) { return (f == F_NN || f == F_NM) ? Mx + 1 : Mx; };
     auto phys = [&](bool ntype, int c) {   // physical column of the tile's column c
         int g = y0 + c;
         if (g < 0) g += My;
         else if (ntype ? g > My : g >= My) g -= My;
+        return g;
+    };
+    auto physr = [&](bool ntype, int g) {   // physical row of grid row g (periodic x)
+        if (PERX) {
+            if (g < 0) g += Mx;
+            else if (ntype ? g > Mx : g >= Mx) g -= Mx;
+        }
         return g;
     };
     const int it0 = *a.step;
@@ -364,10 +380,11 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_consta
     for (int k = tid; k < a.rows_s * P; k += RES_THREADS) {
         const int r = k / P - H, c = k - (r + H) * P - H, g = x0 + r;
 #pragma unroll
-        for (int f = 0; f < 5; f++) {
-            const bool in = g >= 0 && g < rows_of(f) && r < RN + 3 && r >= -3 && c >= -3 && c < WN + 3;
-            const long o = in ? (long)g * a.pitch + phys(ntypeY(f), c) : 0;
-            C *q = at(f, r, c);
+        for (int i = 0; i < NB; i++) {
+            const int f = slot_of(i), gr = physr(f == F_NN || f == F_NM, g);
+            const bool in = gr >= 0 && gr < rows_of(f) && r < RN + 3 && r >= -3 && c >= -3 && c < WN + 3;
+            const long o = in ? (long)gr * a.pitch + phys(ntypeY(f), c) : 0;
+            C *q = at(i, r, c);
             q[0] = in ? a.in[f][o] : C(0);
             if constexpr (RES) q[o_r] = in ? a.rin[f][o] : C(0);
             if constexpr (CS) q[o_c] = in ? a.coef[f][o] : C(0);
@@ -375,7 +392,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_consta
     }
     // the N-type seam: an M-type point left of column 0 reads column My where this tile holds
     // column 0, one right of column My - 1 reads column 0 where it holds column My
-    for (int k = tid; k < a.rows_s; k += RES_THREADS) {
+    for (int k = tid; EL && k < a.rows_s; k += RES_THREADS) {
         const int g = x0 + k - H;
         const bool in = g >= 0 && g <= Mx && k - H < RN + 3;
         altL[k] = in && ty == 0 ? a.in[F_NN][(long)g * a.pitch + My] : C(0);
@@ -389,7 +406,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_consta
     // ---- this thread's column and rows: V on rows [va, vb) and columns -4 .. WN + 1, S on the owned
     // points. Tiles of few rows give the two kinds of point of a phase to the two halves of the CTA.
     constexpr int SLOTS = RES_THREADS / LANES;
-    const int va = max(-2, -x0), vb = min(R + 2, Mx + 1 - x0);
+    const int va = PERX ? -1 : max(-2, -x0), vb = PERX ? R + 2 : min(R + 2, Mx + 1 - x0);
     const int c = (tid % LANES) * N - 4;
     const bool split = vb - va <= SLOTS / 2;
     const int slot = split ? (tid / LANES) % (SLOTS / 2) : tid / LANES, dslot = split ? SLOTS / 2 : SLOTS;
@@ -405,14 +422,18 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_consta
             if (c + q >= -3 && c + q < WN + 3 && phys(a.src_grid == G_NN || a.src_grid == G_MN, c + q) == a.src_iy) sq = q;
     auto own_row = [&](int g) { return g == a.src_grid ? a.src_ix - x0 : -(1 << 20); };
     const int srcMN = own_row(G_MN), srcNM = own_row(G_NM), srcNN = own_row(G_NN), srcMM = own_row(G_MM);
+    // (periodic x: the halo rows hold the points of the other end)
+    auto is_srcNM = [&](int r) { return PERX ? a.src_grid == G_NM && physr(true, x0 + r) == a.src_ix : r == srcNM; };
 
     // ---- this thread's halo words: 3 rows above and below over columns [-3, WN + 3), 3 columns on
     // each side, the seam columns of the V rows
     constexpr int XI = 3;   // (RES_THREADS x XI covers the largest tile: resident_plan)
     int xs[XI], xm[XI], xg[XI], xh[XI];   // shared index of NN, of MM0 (-1: none), words of NN, of MM0
     {
-        const int hw = WN + 6, ht = tx > 0 ? 3 : 0, hb = lastx ? 0 : 3, nvr = vb - va;
-        const int n1 = (ht + hb) * hw, n2 = n1 + RN * 6, n3 = n2 + (ty == 0 ? nvr : 0), n4 = n3 + (lasty ? nvr : 0);
+        // (acoustic: the pressure's rows and columns, M type)
+        const int Rh = EL ? RN : R, Wh = EL ? WN : W, hw = Wh + 6, ht = PERX || tx > 0 ? 3 : 0, hb = PERX || !lastx ? 3 : 0;
+        const int nvr = EL ? vb - va : 0;
+        const int n1 = (ht + hb) * hw, n2 = n1 + Rh * 6, n3 = n2 + (ty == 0 ? nvr : 0), n4 = n3 + (lasty ? nvr : 0);
 #pragma unroll
         for (int m = 0; m < XI; m++) {
             const int h = tid + m * RES_THREADS;
@@ -424,18 +445,24 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_consta
                 if (h < n1) {
                     const int q = h / hw;
                     cc = h - q * hw - 3;
-                    r = q < ht ? q - 3 : RN + (q - ht);
+                    r = q < ht ? q - 3 : Rh + (q - ht);
                 } else {
                     r = (h - n1) / 6;
                     cc = h - n1 - 6 * r;
-                    cc = cc < 3 ? cc - 3 : WN + cc - 3;
+                    cc = cc < 3 ? cc - 3 : Wh + cc - 3;
                 }
-                const int g = x0 + r, cm = (lasty && cc >= WN) ? cc - 1 : cc;   // (M-type halos start at W)
-                xs[m] = (int)(at(F_NN, r, cc) - sm);
-                xg[m] = (g * a.xcols + phys(true, cc)) * XW;
-                if (g < Mx) {
-                    xm[m] = (int)(at(F_MM0, r, cm) - sm);
-                    xh[m] = (g * a.xcols + phys(false, cm)) * XW;
+                const int g = physr(false, x0 + r);
+                if constexpr (EL) {
+                    const int cm = (lasty && cc >= WN) ? cc - 1 : cc;   // (M-type halos start at W)
+                    xs[m] = (int)(at(iNN, r, cc) - sm);
+                    xg[m] = (g * a.xcols + phys(true, cc)) * XW;
+                    if (g < Mx) {
+                        xm[m] = (int)(at(iM0, r, cm) - sm);
+                        xh[m] = (g * a.xcols + phys(false, cm)) * XW;
+                    }
+                } else {
+                    xs[m] = (int)(at(iM0, r, cc) - sm);
+                    xg[m] = (g * a.xcols + phys(false, cc)) * XW;
                 }
             } else {
                 const bool left = h < n3;
@@ -482,33 +509,34 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_consta
                 const int j = x0 + r;
                 const bool orow = r >= 0 && r < RN;
                 auto coefv = [&](int f) -> V {
-                    if constexpr (CS) return vld(q + f * P + o_c);
-                    else return vldg(a.coefx[f - F_MN] + (long)j * a.xpitch + y0 + c + 4);
+                    if constexpr (CS) return vld(q + index_of(f) * P + o_c);
+                    else return vldg(a.coefx[f - F_MN] + (long)physr(f == F_NM, j) * a.xpitch + y0 + c + 4);
                 };
-                const V nnj = ld(F_NN, 0);
-                if (first && j < Mx) {   // MN: x from NN, y from MM syy
+                const V nnj = EL ? ld(iNN, 0) : vzero(C(0));
+                if (first && (EL ? j < Mx : r >= 0 && r < R)) {   // MN: x from NN, y from MM syy
                     [[maybe_unused]] WV wv;
                     if constexpr (ENERGY) wv = weights(F_MN, r, orow && ownN > 0);
                     const V P_ = coefv(F_MN);
                     V r_ = vzero(C(0)), cc = r_, vx;
-                    if constexpr (KR) r_ = vld(q + F_MN * P + o_r);
-                    if constexpr (KC) cc = vld(q + F_MN * P + o_r);
-                    if (j >= 3 && j < Mx - 3) {
-                        vx = taps<C>(st, ld(F_NN, -1), nnj, ld(F_NN, 1), ld(F_NN, 2));
+                    if constexpr (KR) r_ = vld(q + iMN * P + o_r);
+                    if constexpr (KC) cc = vld(q + iMN * P + o_r);
+                    if constexpr (!EL) {   // (no shear: the y derivative alone)
+                    } else if (j >= 3 && j < Mx - 3) {
+                        vx = taps<C>(st, ld(iNN, -1), nnj, ld(iNN, 1), ld(iNN, 2));
                         r_ = st.add(r_, mul(vx, P_));
                     } else {   // closure and SAT
-                        vx = vdxN_end<C>(ends, st, Mx, j, [&](int g) { return vld(at(F_NN, g - x0, c)); });
+                        vx = vdxN_end<C>(ends, st, Mx, j, [&](int g) { return vld(at(iNN, g - x0, c)); });
                         r_ = st.add(r_, mul(vx, P_));
                         const bool L = j < 3;
-                        const V send = mulw(vld(at(F_NN, L ? -x0 : Mx - x0, c)), wt(a.op.pN));
+                        const V send = mulw(vld(at(iNN, L ? -x0 : Mx - x0, c)), wt(a.op.pN));
                         r_ = st.add(r_, mul(mulw(send, ends.satM[L ? j : j - (Mx - 6)]), P_));
                     }
-                    r_ = st.add(r_, mul(dyN(st, q + F_MM1 * P, vld(q + F_MM1 * P)), P_));
-                    V s = vld(q + F_MN * P);
+                    r_ = st.add(r_, mul(dyN(st, q + iM1 * P, vld(q + iM1 * P)), P_));
+                    V s = vld(q + iMN * P);
                     vupdate<CPST, C>(st, s, r_, cc);
                     if (r == srcMN) source(s);
-                    vst(q + F_MN * P, s);
-                    if constexpr (RES) vst(q + F_MN * P + o_r, KR ? r_ : cc);
+                    vst(q + iMN * P, s);
+                    if constexpr (RES) vst(q + iMN * P + o_r, KR ? r_ : cc);
                     if constexpr (ENERGY) {
                         C e[N];
                         vget(s, e);
@@ -522,27 +550,28 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_consta
                     if constexpr (ENERGY) wv = weights(F_NM, r, orow && ownM > 0);
                     const V P_ = coefv(F_NM);
                     V r_ = vzero(C(0)), cc = r_, vx;
-                    if constexpr (KR) r_ = vld(q + F_NM * P + o_r);
-                    if constexpr (KC) cc = vld(q + F_NM * P + o_r);
-                    if (j >= 4 && j < Mx - 3) {
-                        vx = taps<C>(st, ld(F_MM0, -2), ld(F_MM0, -1), ld(F_MM0, 0), ld(F_MM0, 1));
+                    if constexpr (KR) r_ = vld(q + iNM * P + o_r);
+                    if constexpr (KC) cc = vld(q + iNM * P + o_r);
+                    if (PERX || (j >= 4 && j < Mx - 3)) {
+                        vx = taps<C>(st, ld(iM0, -2), ld(iM0, -1), ld(iM0, 0), ld(iM0, 1));
                         r_ = st.add(r_, mul(vx, P_));
                     } else {
-                        vx = vdxM_end<C>(ends, st, Mx, j, [&](int g) { return vld(at(F_MM0, g - x0, c)); });
+                        vx = vdxM_end<C>(ends, st, Mx, j, [&](int g) { return vld(at(iM0, g - x0, c)); });
                         r_ = st.add(r_, mul(vx, P_));
                         if (j == 0 || j == Mx) {   // SAT
                             const bool L = j == 0;
                             V send = vzero(C(0));
 #pragma unroll
                             for (int w = 0; w < 3; w++)
-                                send = st.add(send, mulw(vld(at(F_MM0, (L ? w : Mx - 3 + w) - x0, c)), ends.pM[(L ? 0 : 3) + w]));
+                                send = st.add(send, mulw(vld(at(iM0, (L ? w : Mx - 3 + w) - x0, c)), ends.pM[(L ? 0 : 3) + w]));
                             r_ = st.add(r_, mul(mulw(send, ends.satN[L ? 0 : 1]), P_));
                         }
                     }
+                    if constexpr (EL) {
                     // (left of column 0 the next column is My, not the tile's column 0)
-                    V vy = dyM(st, q + F_NN * P, nnj, seamL, altL + r + H);
+                    V vy = dyM(st, q + iNN * P, nnj, seamL, altL + r + H);
                     if (seamR) {   // the columns from My on: the one there is column 0
-                        const C *p = at(F_NN, r, lc);
+                        const C *p = at(iNN, r, lc);
                         const C z = altR[r + H], p1 = p[1], p2 = p[2];
                         auto tap4 = [&](C t0, C t1, C t2, C t3) {
                             C v = mul(t0, a.op.st[0]);
@@ -558,11 +587,12 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_consta
                         vy = vset(e);
                     }
                     r_ = st.add(r_, mul(vy, P_));
-                    V s = vld(q + F_NM * P);
+                    }
+                    V s = vld(q + iNM * P);
                     vupdate<CPST, C>(st, s, r_, cc);
-                    if (r == srcNM) source(s);
-                    vst(q + F_NM * P, s);
-                    if constexpr (RES) vst(q + F_NM * P + o_r, KR ? r_ : cc);
+                    if (is_srcNM(r)) source(s);
+                    vst(q + iNM * P, s);
+                    if constexpr (RES) vst(q + iNM * P + o_r, KR ? r_ : cc);
                     if constexpr (ENERGY) {
                         C e[N];
                         vget(s, e);
@@ -579,11 +609,11 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_consta
                     V nn[5], m0[5];
 #pragma unroll
                     for (int w = 0; w < 5; w++) {
-                        nn[w] = vld(q + F_NN * P + (w - 1) * RS);
-                        m0[w] = vld(q + F_MM0 * P + (w - 2) * RS);
+                        nn[w] = EL ? vld(q + iNN * P + (w - 1) * RS) : vzero(C(0));
+                        m0[w] = vld(q + iM0 * P + (w - 2) * RS);
                     }
-                    vrow(r, q, [&](int f, int o) { return f == F_NN ? nn[o + 1] : m0[o + 2]; });
-                    if (r + 1 < vb) vrow(r + 1, q + RS, [&](int f, int o) { return f == F_NN ? nn[o + 2] : m0[o + 3]; });
+                    vrow(r, q, [&](int f, int o) { return EL && f == iNN ? nn[o + 1] : m0[o + 2]; });
+                    if (r + 1 < vb) vrow(r + 1, q + RS, [&](int f, int o) { return EL && f == iNN ? nn[o + 2] : m0[o + 3]; });
                 }
             } else {
                 for (int r = va + slot; r < vb; r += dslot) {
@@ -596,11 +626,11 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_consta
         for (int q = rb + tid; q < re; q += RES_THREADS) {   // velocity receivers (the velocities rest during S)
             const int *e = a.rcv + 4 * q;
             if (e[0] == F_MN || e[0] == F_NM)
-                a.traces[(long)e[3] * a.max_steps + it] = (double)*at(e[0], e[1] - x0, e[2] - y0);
+                a.traces[(long)e[3] * a.max_steps + it] = (double)*at(index_of(e[0]), e[1] - x0, e[2] - y0);
         }
         // ---- S: stresses of the owned points; those near an edge also to the exchange words
         const unsigned tag = a.tag0 + (unsigned)k + 1u;
-        u64 *xb = a.xbuf + (size_t)(tag & 1u) * 3 * a.xarr;
+        u64 *xb = a.xbuf + (size_t)(tag & 1u) * (EL ? 3 : 1) * a.xarr;
         auto send = [&](int r, int own, int f3, const V &v) {
             C e[N];
             vget(v, e);
@@ -617,29 +647,30 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_consta
                 const int i = x0 + r;
                 [[maybe_unused]] const long go = (long)i * a.pitch + y0 + c;
                 auto coefv = [&](int f) -> V {
-                    if constexpr (CS) return vld(q + f * P + o_c);
+                    if constexpr (CS) return vld(q + index_of(f) * P + o_c);
                     else return vldg(a.coef[f] + go);
                 };
                 const bool border = !last && multi && (bcol || r < 3 || r >= R - 3);
+                if constexpr (EL) {
                 if (first) {   // NN: x from MN, y from NM
                     [[maybe_unused]] WV wv;
                     if constexpr (ENERGY) wv = weights(F_NN, r, true);
                     const V P_ = coefv(F_NN);
                     V r_ = vzero(C(0)), cc = r_, vx;
-                    if constexpr (KR) r_ = vld(q + F_NN * P + o_r);
-                    if constexpr (KC) cc = vld(q + F_NN * P + o_r);
+                    if constexpr (KR) r_ = vld(q + iNN * P + o_r);
+                    if constexpr (KC) cc = vld(q + iNN * P + o_r);
                     if (i >= 4 && i < Mx - 3)
-                        vx = taps<C>(st, ld(F_MN, -2), ld(F_MN, -1), ld(F_MN, 0), ld(F_MN, 1));
+                        vx = taps<C>(st, ld(iMN, -2), ld(iMN, -1), ld(iMN, 0), ld(iMN, 1));
                     else
-                        vx = vdxM_end<C>(ends, st, Mx, i, [&](int g) { return vld(at(F_MN, g - x0, c)); });
+                        vx = vdxM_end<C>(ends, st, Mx, i, [&](int g) { return vld(at(iMN, g - x0, c)); });
                     r_ = st.add(r_, mul(vx, P_));
-                    r_ = st.add(r_, mul(dyN(st, q + F_NM * P, ld(F_NM, 0)), P_));
-                    const V old = vld(q + F_NN * P);
+                    r_ = st.add(r_, mul(dyN(st, q + iNM * P, ld(iNM, 0)), P_));
+                    const V old = vld(q + iNN * P);
                     V s = old;
                     vupdate<CPST, C>(st, s, r_, cc);
                     if (r == srcNN) source(s);
-                    vst(q + F_NN * P, s);
-                    if constexpr (RES) vst(q + F_NN * P + o_r, KR ? r_ : cc);
+                    vst(q + iNN * P, s);
+                    if constexpr (RES) vst(q + iNN * P + o_r, KR ? r_ : cc);
                     if (border) send(r, ownN, 0, s);
                     if constexpr (ENERGY) {
                         C e[N], o[N];
@@ -658,20 +689,20 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_consta
                     if constexpr (ENERGY) { wv3 = weights(F_MM0, r, true); wv4 = weights(F_MM1, r, true); }
                     const V L = coefv(F_MM0), M2 = coefv(F_MM1);
                     V r0 = vzero(C(0)), r1 = r0, k0 = r0, k1 = r0, vx;
-                    if constexpr (KR) { r0 = vld(q + F_MM0 * P + o_r); r1 = vld(q + F_MM1 * P + o_r); }
-                    if constexpr (KC) { k0 = vld(q + F_MM0 * P + o_r); k1 = vld(q + F_MM1 * P + o_r); }
+                    if constexpr (KR) { r0 = vld(q + iM0 * P + o_r); r1 = vld(q + iM1 * P + o_r); }
+                    if constexpr (KC) { k0 = vld(q + iM0 * P + o_r); k1 = vld(q + iM1 * P + o_r); }
                     if (i >= 3 && i < Mx - 3)
-                        vx = taps<C>(st, ld(F_NM, -1), ld(F_NM, 0), ld(F_NM, 1), ld(F_NM, 2));
+                        vx = taps<C>(st, ld(iNM, -1), ld(iNM, 0), ld(iNM, 1), ld(iNM, 2));
                     else
-                        vx = vdxN_end<C>(ends, st, Mx, i, [&](int g) { return vld(at(F_NM, g - x0, c)); });
+                        vx = vdxN_end<C>(ends, st, Mx, i, [&](int g) { return vld(at(iNM, g - x0, c)); });
                     r0 = st.add(r0, mul(vx, L));
                     r1 = st.add(r1, mul(vx, L));
                     r0 = st.add(r0, mul(vx, M2));
-                    const V vy = dyM(st, q + F_MN * P, ld(F_MN, 0), false, nullptr);
+                    const V vy = dyM(st, q + iMN * P, ld(iMN, 0), false, nullptr);
                     r0 = st.add(r0, mul(vy, L));
                     r1 = st.add(r1, mul(vy, L));
                     r1 = st.add(r1, mul(vy, M2));
-                    const V o0 = vld(q + F_MM0 * P), o1 = vld(q + F_MM1 * P);
+                    const V o0 = vld(q + iM0 * P), o1 = vld(q + iM1 * P);
                     V s0 = o0, s1 = o1;
                     vupdate<CPST, C>(st, s0, r0, k0);
                     vupdate<CPST, C>(st, s1, r1, k1);
@@ -679,11 +710,11 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_consta
                         source(s0);
                         source(s1);
                     }
-                    vst(q + F_MM0 * P, s0);
-                    vst(q + F_MM1 * P, s1);
+                    vst(q + iM0 * P, s0);
+                    vst(q + iM1 * P, s1);
                     if constexpr (RES) {
-                        vst(q + F_MM0 * P + o_r, KR ? r0 : k0);
-                        vst(q + F_MM1 * P + o_r, KR ? r1 : k1);
+                        vst(q + iM0 * P + o_r, KR ? r0 : k0);
+                        vst(q + iM1 * P + o_r, KR ? r1 : k1);
                     }
                     if (border) {
                         send(r, ownM, 1, s0);
@@ -709,6 +740,27 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_consta
                             }
                     }
                 }
+                } else {
+                if (r < R && ownM > 0 && (!split || (r & 1) == (second ? 1 : 0))) {   // pressure: x from NM, y from MN
+                    const V K_ = coefv(F_MM0);
+                    V r_ = vzero(C(0)), cc = r_, vx;
+                    if constexpr (KR) r_ = vld(q + iM0 * P + o_r);
+                    if constexpr (KC) cc = vld(q + iM0 * P + o_r);
+                    if (PERX || (i >= 3 && i < Mx - 3))
+                        vx = taps<C>(st, ld(iNM, -1), ld(iNM, 0), ld(iNM, 1), ld(iNM, 2));
+                    else
+                        vx = vdxN_end<C>(ends, st, Mx, i, [&](int g) { return vld(at(iNM, g - x0, c)); });
+                    r_ = st.add(r_, mul(vx, K_));
+                    const C *mnp = q + iMN * P;
+                    r_ = st.add(r_, mul(dyM(st, mnp, vld(mnp), false, nullptr), K_));
+                    V s = vld(q + iM0 * P);
+                    vupdate<CPST, C>(st, s, r_, cc);
+                    if (r == srcMM) source(s);
+                    vst(q + iM0 * P, s);
+                    if constexpr (RES) vst(q + iM0 * P + o_r, KR ? r_ : cc);
+                    if (border) send(r, ownM, 0, s);
+                }
+                }
         };
         if (scol) {
             if (vpair) {
@@ -717,11 +769,11 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_consta
                     V mn[5], nm[5];
 #pragma unroll
                     for (int w = 0; w < 5; w++) {
-                        mn[w] = vld(q + F_MN * P + (w - 2) * RS);
-                        nm[w] = vld(q + F_NM * P + (w - 1) * RS);
+                        mn[w] = EL ? vld(q + iMN * P + (w - 2) * RS) : vzero(C(0));
+                        nm[w] = vld(q + iNM * P + (w - 1) * RS);
                     }
-                    srow(r, q, [&](int f, int o) { return f == F_MN ? mn[o + 2] : nm[o + 1]; });
-                    if (r + 1 < RN) srow(r + 1, q + RS, [&](int f, int o) { return f == F_MN ? mn[o + 3] : nm[o + 2]; });
+                    srow(r, q, [&](int f, int o) { return EL && f == iMN ? mn[o + 2] : nm[o + 1]; });
+                    if (r + 1 < RN) srow(r + 1, q + RS, [&](int f, int o) { return EL && f == iMN ? mn[o + 3] : nm[o + 2]; });
                 }
             } else {
                 for (int r = slot; r < RN; r += dslot) {
@@ -743,7 +795,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_consta
         for (int q = rb + tid; q < re; q += RES_THREADS) {   // stress receivers (the owned stresses rest until S)
             const int *e = a.rcv + 4 * q;
             if (e[0] != F_MN && e[0] != F_NM)
-                a.traces[(long)e[3] * a.max_steps + it] = (double)*at(e[0], e[1] - x0, e[2] - y0);
+                a.traces[(long)e[3] * a.max_steps + it] = (double)*at(index_of(e[0]), e[1] - x0, e[2] - y0);
         }
         if constexpr (ENERGY) {
             if (tid < 3 && it < a.max_steps) {
@@ -771,7 +823,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_consta
 #pragma unroll
                     for (int m = 0; m < B; m++) {
                         if (xs[b + m] >= 0) v[m][0].load(xb + xg[b + m]);
-                        if (xm[b + m] >= 0) {
+                        if (EL && xm[b + m] >= 0) {
                             v[m][1].load(xb + a.xarr + xh[b + m]);
                             v[m][2].load(xb + 2 * a.xarr + xh[b + m]);
                         }
@@ -780,14 +832,14 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_consta
 #pragma unroll
                     for (int m = 0; m < B; m++) {
                         if (xs[b + m] >= 0) ok = ok && v[m][0].ok(tag);
-                        if (xm[b + m] >= 0) ok = ok && v[m][1].ok(tag) && v[m][2].ok(tag);
+                        if (EL && xm[b + m] >= 0) ok = ok && v[m][1].ok(tag) && v[m][2].ok(tag);
                     }
                 }
                 if (ok) {
 #pragma unroll
                     for (int m = 0; m < B; m++) {
                         if (xs[b + m] >= 0) sm[xs[b + m]] = v[m][0].get();
-                        if (xm[b + m] >= 0) {
+                        if (EL && xm[b + m] >= 0) {
                             sm[xm[b + m]] = v[m][1].get();
                             sm[xm[b + m] + P] = v[m][2].get();
                         }
@@ -795,19 +847,26 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_consta
                 }
             }
             if (!ok) bad_s = 1;
-        } else {   // one tile: the periodic columns from the tile itself
+        } else if constexpr (EL) {   // one tile: the periodic columns from the tile itself
             for (int idx = tid; idx < RN * 6; idx += RES_THREADS) {
                 const int r = idx / 6, q = idx - 6 * r;
                 const int cn = q < 3 ? q - 3 : WN + q - 3, cm = cn >= WN ? cn - 1 : cn;
-                *at(F_NN, r, cn) = *at(F_NN, r, phys(true, cn));
+                *at(iNN, r, cn) = *at(iNN, r, phys(true, cn));
                 if (r < R) {
-                    *at(F_MM0, r, cm) = *at(F_MM0, r, phys(false, cm));
-                    *at(F_MM1, r, cm) = *at(F_MM1, r, phys(false, cm));
+                    *at(iM0, r, cm) = *at(iM0, r, phys(false, cm));
+                    *at(iM1, r, cm) = *at(iM1, r, phys(false, cm));
                 }
             }
             for (int r = tid; r < RN; r += RES_THREADS) {
-                altL[r + H] = *at(F_NN, r, lc);
-                altR[r + H] = *at(F_NN, r, 0);
+                altL[r + H] = *at(iNN, r, lc);
+                altR[r + H] = *at(iNN, r, 0);
+            }
+        } else {
+            for (int idx = tid; idx < R * 6 + (PERX ? W * 6 : 0); idx += RES_THREADS) {
+                const bool col = idx < R * 6;
+                const int h = col ? idx : idx - R * 6, r = h / 6, q = h - 6 * r, e = q < 3 ? q - 3 : (col ? W : R) + q - 3;
+                if (col) *at(iM0, r, e) = *at(iM0, r, phys(false, e));
+                else *at(iM0, e, r) = *at(iM0, physr(false, e), r);
             }
         }
         __syncthreads();
@@ -816,12 +875,13 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_consta
     // ---- the state after the run. (A value that stopped being finite at any step has stayed so: an
     // update adds to it.)
     C nf = C(0);   // stays 0 until a value is not finite (v * 0 is NaN then)
-    for (int f = 0; f < 5; f++) {
+    for (int i = 0; i < NB; i++) {
+        const int f = slot_of(i);
         const int rows = f == F_NN || f == F_NM ? RN : R, cols = ntypeY(f) ? WN : W;
         for (int k = tid; k < rows * RES_LANES_COLS; k += RES_THREADS) {
             const int r = k / RES_LANES_COLS, cc = k - r * RES_LANES_COLS;
             if (cc >= cols) continue;
-            const C *q = at(f, r, cc);
+            const C *q = at(i, r, cc);
             const long o = (long)(x0 + r) * a.pitch + y0 + cc;
             nf = nf + q[0] * C(0);
             a.out[f][o] = q[0];
@@ -843,29 +903,37 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_consta
 }
 
 // ------------------------------------------------------------------------------- launcher
-template <class C, class F>
+// codes 1 / 3 and 2 / 4 are the same update; coefficients stay in L2 for the plain update only
+template <class C, int PHYS, bool ENERGY, class F>
+cudaError_t resident_code(int cpst, bool cs, F f)
+{
+    if (cpst == 0) return cs ? f(k_resident<C, 0, ENERGY, true, PHYS>) : f(k_resident<C, 0, ENERGY, false, PHYS>);
+    if (cpst == 2 || cpst == 4) return f(k_resident<C, 4, ENERGY, true, PHYS>);
+    if (cpst == 6) return f(k_resident<C, 6, ENERGY, true, PHYS>);
+    if constexpr (PHYS != RES_AC_PER) {   // (the periodic tree has '0', '3' and '6')
+        if (cpst == 1 || cpst == 3) return f(k_resident<C, 3, ENERGY, true, PHYS>);
+        return f(k_resident<C, 5, ENERGY, true, PHYS>);
+    }
+    return cudaErrorInvalidValue;
+}
+template <class C, int PHYS, class F>
 cudaError_t resident_kernel(int cpst, bool energy, bool cs, F f)
 {
-    // codes 1 / 3 and 2 / 4 are the same update; coefficients stay in L2 for the plain update only
-    if (cpst == 0) {
-        if (cs) return energy ? f(k_resident<C, 0, true, true>) : f(k_resident<C, 0, false, true>);
-        return energy ? f(k_resident<C, 0, true, false>) : f(k_resident<C, 0, false, false>);
-    }
-    if (cpst == 1 || cpst == 3) return energy ? f(k_resident<C, 3, true, true>) : f(k_resident<C, 3, false, true>);
-    if (cpst == 2 || cpst == 4) return energy ? f(k_resident<C, 4, true, true>) : f(k_resident<C, 4, false, true>);
-    if (cpst == 5) return energy ? f(k_resident<C, 5, true, true>) : f(k_resident<C, 5, false, true>);
-    return energy ? f(k_resident<C, 6, true, true>) : f(k_resident<C, 6, false, true>);
+    if constexpr (PHYS == RES_ELASTIC)   // (acoustic energies: the per-point kernels)
+        if (energy) return resident_code<C, PHYS, true>(cpst, cs, f);
+    return resident_code<C, PHYS, false>(cpst, cs, f);
 }
 
-template <class C>
-cudaError_t prepare_resident(int cpst, bool energy, const ResPlan &p)
+// (the opt-in is the kernel's, not a handle's: always the most a plan may ask for)
+template <class C, int PHYS>
+cudaError_t prepare_resident(int cpst, bool energy, const ResPlan &p, int smem_max)
 {
-    return resident_kernel<C>(cpst, energy, p.cs, [&](auto k) {
-        return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
+    return resident_kernel<C, PHYS>(cpst, energy, p.cs, [&](auto k) {
+        return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);
     });
 }
 
-template <class C>
+template <class C, int PHYS>
 cudaError_t launch_resident(const ResArgs<C> &a, int cpst, bool energy, const ResPlan &p, cudaStream_t st)
 {
     cudaLaunchConfig_t cfg{};
@@ -878,7 +946,7 @@ cudaError_t launch_resident(const ResArgs<C> &a, int cpst, bool energy, const Re
     at[0].val.cooperative = 1;
     cfg.attrs = at;
     cfg.numAttrs = p.ntx * p.nty > 1 ? 1 : 0;
-    return resident_kernel<C>(cpst, energy, p.cs, [&](auto k) { return cudaLaunchKernelEx(&cfg, k, a); });
+    return resident_kernel<C, PHYS>(cpst, energy, p.cs, [&](auto k) { return cudaLaunchKernelEx(&cfg, k, a); });
 }
 
 }  // namespace tw

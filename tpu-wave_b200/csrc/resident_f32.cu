@@ -1,38 +1,46 @@
 // On-chip runs of the elastic step (resident.cuh) for FP32 fields, and the tiling of both types.
 #include <algorithm>
 #include <cstdlib>
+#include <vector>
 
 #include "resident.cuh"
 
 namespace tw {
-template cudaError_t prepare_resident<float>(int, bool, const ResPlan &);
-template cudaError_t launch_resident<float>(const ResArgs<float> &, int, bool, const ResPlan &, cudaStream_t);
+template cudaError_t prepare_resident<float, RES_ELASTIC>(int, bool, const ResPlan &, int);
+template cudaError_t launch_resident<float, RES_ELASTIC>(const ResArgs<float> &, int, bool, const ResPlan &, cudaStream_t);
 
-ResPlan resident_plan(long Mx, long My, int esize, bool comp, int n_sm, size_t smem_max)
+ResPlan resident_plan(long Mx, long My, int esize, int fields, bool comp, int n_sm, size_t smem_max)
 {
     ResPlan best;
     double best_cost = 1e30;
     const int N = 16 / esize, nq4 = (int)((My + 4) / 4);
     auto pin = [](const char *name) { const char *v = std::getenv(name); return v ? std::atoi(v) : 0; };
     const int pin_x = pin("TW_RES_NTX"), pin_y = pin("TW_RES_NTY");
+    std::vector<int> widest(n_sm + 1, 0);   // by nty: most columns of a tile (the last one with column My), 0: too few
+    for (int nty = 1; nty <= n_sm; nty++) {
+        int wmin = 1 << 30;
+        for (int t = 0; t < nty; t++) {
+            const int b = 4 * (int)((long)t * nq4 / nty);
+            const int e = t == nty - 1 ? (int)My : 4 * (int)((long)(t + 1) * nq4 / nty);
+            wmin = std::min(wmin, e - b);
+            widest[nty] = std::max(widest[nty], e - b + (t == nty - 1 ? 1 : 0));
+        }
+        if (wmin >= RES_MIN) continue;
+        widest[nty] = 0;
+        break;   // (narrower still from here on)
+    }
     for (int ntx = 1; ntx <= n_sm && Mx / ntx >= RES_MIN; ntx++)
-        for (int nty = 1; ntx * nty <= n_sm; nty++) {
+        for (int nty = 1; ntx * nty <= n_sm && widest[nty]; nty++) {
             if ((pin_x && ntx != pin_x) || (pin_y && nty != pin_y)) continue;
-            int wmax = 0, wmin = 1 << 30;   // columns of the tiles (the last one with column My)
-            for (int t = 0; t < nty; t++) {
-                const int b = 4 * (int)((long)t * nq4 / nty);
-                const int e = t == nty - 1 ? (int)My : 4 * (int)((long)(t + 1) * nq4 / nty);
-                wmin = std::min(wmin, e - b);
-                wmax = std::max(wmax, e - b + (t == nty - 1 ? 1 : 0));
-            }
-            if (wmin < RES_MIN) break;
+            const int wmax = widest[nty];
             if (wmax > RES_W) continue;
             const int R = (int)((Mx + ntx - 1) / ntx);
-            if (6 * (wmax + 6) + (nty > 1 ? 7 : 8) * (R + 1) + 8 > 3 * RES_THREADS) continue;   // halo words (k_resident: XI)
+            // halo words (k_resident: XI), the elastic grids' seam columns among them
+            if (6 * (wmax + 6) + (fields == 3 ? 6 : (nty > 1 ? 7 : 8)) * (R + 1) + 8 > 3 * RES_THREADS) continue;
             const int rows_s = R + 1 + 2 * RES_PAD;
             const size_t one = (size_t)rows_s * RES_P * esize, alt = (size_t)2 * rows_s * esize;
-            const size_t base = one * (5 + (comp ? 5 : 0)) + alt;
-            bool cs = base + 5 * one <= smem_max;
+            const size_t base = one * (fields + (comp ? fields : 0)) + alt;
+            bool cs = base + fields * one <= smem_max;
             if (!cs && (comp || base > smem_max)) continue;
             // modelled cost in rounds of about 0.5 us (within 10 % of the best of a sweep of tilings at 48 x 40
             // to 1024 x 1024): rounds of the CTA's rows in the two phases (short tiles split a phase's two kinds of
@@ -47,7 +55,7 @@ ResPlan resident_plan(long Mx, long My, int esize, bool comp, int n_sm, size_t s
                 best.nty = nty;
                 best.rows_s = rows_s;
                 best.cs = cs;
-                best.smem = base + (cs ? 5 * one : 0);
+                best.smem = base + (cs ? fields * one : 0);
             }
         }
     return best;

@@ -2,6 +2,6 @@
 #include "resident.cuh"
 
 namespace tw {
-template cudaError_t prepare_resident<double>(int, bool, const ResPlan &);
-template cudaError_t launch_resident<double>(const ResArgs<double> &, int, bool, const ResPlan &, cudaStream_t);
+template cudaError_t prepare_resident<double, RES_ELASTIC>(int, bool, const ResPlan &, int);
+template cudaError_t launch_resident<double, RES_ELASTIC>(const ResArgs<double> &, int, bool, const ResPlan &, cudaStream_t);
 }  // namespace tw

@@ -127,6 +127,9 @@ struct tw_solver {
     // grids that fit on the chip: a run of tw_step is one launch (resident.cuh); the handle's other
     // step kernels serve single steps elsewhere (the adjoint's sweeps, captured streams)
     ResPlan res_plan;                 // ntx 0: the grid does not fit
+    // a run of a handle with one buffer ends where it began: a tile is stored after its neighbours have
+    // sent words of their first step, so after they have loaded it (runs of two steps or more)
+    bool res_in_place = false;
     unsigned res_tag = 0;             // steps run this way since the exchange words were cleared
     unsigned long long *xbuf = nullptr;
     size_t xbuf_bytes = 0;
@@ -579,8 +582,9 @@ int run_resident(tw_solver *s, int n, cudaStream_t st)
         s->coefx_dirty = false;
     }
     ResArgs<C> a{};
-    void *const *fin = s->parity ? s->f2 : s->f, *const *fout = s->parity ? s->f : s->f2;
-    void *const *rin = s->parity ? s->res2 : s->res, *const *rout = s->parity ? s->res : s->res2;
+    const int po = s->res_in_place ? s->parity : s->parity ^ 1;   // the buffer of the state after the run
+    void *const *fin = s->parity ? s->f2 : s->f, *const *fout = po ? s->f2 : s->f;
+    void *const *rin = s->parity ? s->res2 : s->res, *const *rout = po ? s->res2 : s->res;
     for (int k = 0; k < 5; k++) {
         a.in[k] = (const C *)fin[k];
         a.out[k] = (C *)fout[k];
@@ -595,7 +599,7 @@ int run_resident(tw_solver *s, int n, cudaStream_t st)
     a.pitch = s->pitch;
     a.Mx = (int)s->d.Mx;
     a.My = (int)s->d.My;
-    a.op = make_ops<C>((double)s->d.num_dx / (double)s->d.den_dx, s->d.dt, false);
+    a.op = make_ops<C>((double)s->d.num_dx / (double)s->d.den_dx, s->d.dt, s->periodic && !s->elastic);
     a.ntx = p.ntx;
     a.nty = p.nty;
     a.rows_s = p.rows_s;
@@ -616,9 +620,13 @@ int run_resident(tw_solver *s, int n, cudaStream_t st)
     a.rcv_off = s->d_rcv_off_r;
     a.rcv = s->d_rcv_list_r;
     a.traces = s->d_traces;
-    TW_CUDA(launch_resident<C>(a, s->d.cpst, s->d.energy != 0, p, st));
+    cudaError_t e;
+    if (s->elastic) e = launch_resident<C, RES_ELASTIC>(a, s->d.cpst, s->d.energy != 0, p, st);
+    else if (s->periodic) e = launch_resident<C, RES_AC_PER>(a, s->d.cpst, false, p, st);
+    else e = launch_resident<C, RES_AC_FREE>(a, s->d.cpst, false, p, st);
+    if (e != cudaSuccess) return cuda_fail(e, "on-chip run");
     s->res_tag += (unsigned)n;
-    s->parity ^= 1;
+    if (!s->res_in_place) s->parity ^= 1;
     return TW_OK;
 }
 
@@ -1305,33 +1313,6 @@ int create_impl(tw_solver **out, const tw_grid_desc *desc, const SlabSpec &sl)
             cudaMemsetAsync(s->d_rcv_off_w, 0, sizeof(int) * (nw + 1), s->st);
         }
     }
-    // on-chip runs: FP32 / FP64 storage and coefficients, the reference's boundaries, a handle of its
-    // own (not a slab), a grid that fits on the SMs. TW_TMA / TW_RESIDENT=0 select the other
-    // kernels for comparisons, TW_RES_NTX / TW_RES_NTY a tiling.
-    if (s->fused && !s->slab && !s->bnd && !d.coef_fp16 && (d.precision == TW_FP64 || d.precision == TW_FP32) &&
-        !std::getenv("TW_TMA") && env_int("TW_RESIDENT", 1) != 0) {
-        int n_sm = 0, smem_max = 0, coop = 0;
-        cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, d.device);
-        cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, d.device);
-        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, d.device);
-        const ResPlan p = coop ? resident_plan(Mx, My, s->esz, cp, n_sm, (size_t)std::max(0, smem_max - 2048)) : ResPlan{};
-        if (p.ntx > 0) {
-            e = d.precision == TW_FP64 ? prepare_resident<double>(d.cpst, d.energy != 0, p) : prepare_resident<float>(d.cpst, d.energy != 0, p);
-            if (e != cudaSuccess) return fail(cuda_fail(e, "cudaFuncSetAttribute"));
-            if (p.ntx * p.nty > 1) {
-                s->xbuf_bytes = (size_t)6 * (Mx + 1) * ((My + 2) & ~1L) * 2 * s->esz;
-                if ((rc_ = s->alloc((void **)&s->xbuf, s->xbuf_bytes)) != TW_OK) return fail(rc_);
-                cudaMemsetAsync(s->xbuf, 0, s->xbuf_bytes, s->st);
-            }
-            if (!p.cs) {
-                s->xpitch = (My + 16 + 3) / 4 * 4;
-                for (int k = 0; k < 2; k++)
-                    if ((rc_ = s->alloc(&s->coefx[k], (size_t)s->rows[F_MN + k] * s->xpitch * s->esz)) != TW_OK) return fail(rc_);
-            }
-            if ((rc_ = s->alloc((void **)&s->d_rcv_off_r, sizeof(int) * (p.ntx * p.nty + 1))) != TW_OK) return fail(rc_);
-            s->res_plan = p;
-        }
-    }
     if (!s->elastic && s->periodic && !d.energy) {
         // periodic acoustic with energy off: a second copy of the state, for the fused step of a
         // batch and, on grids of 2^20 points or more, of the handle alone (below that the
@@ -1354,6 +1335,46 @@ int create_impl(tw_solver **out, const tw_grid_desc *desc, const SlabSpec &sl)
         s->n_int_seg = std::max(1, std::min(target, (int)Mx / 8));
         if ((rc_ = s->alloc((void **)&s->d_done, sizeof(int))) != TW_OK) return fail(rc_);
         cudaMemsetAsync(s->d_done, 0, sizeof(int), s->st);
+    }
+    // on-chip runs: FP32 / FP64 storage and coefficients, the reference's boundaries, a handle of its
+    // own (not a slab), a grid that fits on the SMs. TW_TMA / TW_RESIDENT=0 select the other
+    // kernels for comparisons, TW_RES_NTX / TW_RES_NTY a tiling.
+    // (acoustic: energy off)
+    if ((s->fused || (!s->elastic && !d.energy)) && !s->slab && !s->bnd && !d.coef_fp16 && (d.precision == TW_FP64 || d.precision == TW_FP32) &&
+        !std::getenv("TW_TMA") && env_int("TW_RESIDENT", 1) != 0) {
+        int n_sm = 0, smem_max = 0, coop = 0;
+        cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, d.device);
+        cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, d.device);
+        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, d.device);
+        smem_max = std::max(0, smem_max - RES_STATIC);
+        const ResPlan p = coop ? resident_plan(Mx, My, s->esz, s->elastic ? 5 : 3, cp, n_sm, (size_t)smem_max) : ResPlan{};
+        if (p.ntx > 0) {
+            auto prepare = [&](auto zero) {
+                using C = decltype(zero);
+                if (s->elastic) return prepare_resident<C, RES_ELASTIC>(d.cpst, d.energy != 0, p, smem_max);
+                return s->periodic ? prepare_resident<C, RES_AC_PER>(d.cpst, false, p, smem_max)
+                                   : prepare_resident<C, RES_AC_FREE>(d.cpst, false, p, smem_max);
+            };
+            e = d.precision == TW_FP64 ? prepare(0.0) : prepare(0.0f);
+            if (e != cudaSuccess) return fail(cuda_fail(e, "cudaFuncSetAttribute"));
+            if (p.ntx * p.nty > 1) {
+                s->xbuf_bytes = (size_t)(s->elastic ? 6 : 2) * (Mx + 1) * ((My + 2) & ~1L) * 2 * s->esz;
+                if ((rc_ = s->alloc((void **)&s->xbuf, s->xbuf_bytes)) != TW_OK) return fail(rc_);
+                cudaMemsetAsync(s->xbuf, 0, s->xbuf_bytes, s->st);
+            }
+            if (!p.cs) {
+                s->xpitch = (My + 16 + 3) / 4 * 4;
+                for (int k = 0; k < 2; k++)
+                    if ((rc_ = s->alloc(&s->coefx[k], (size_t)s->rows[F_MN + k] * s->xpitch * s->esz)) != TW_OK) return fail(rc_);
+            }
+            if ((rc_ = s->alloc((void **)&s->d_rcv_off_r, sizeof(int) * (p.ntx * p.nty + 1))) != TW_OK) return fail(rc_);
+            if (!s->d_done) {
+                if ((rc_ = s->alloc((void **)&s->d_done, sizeof(int))) != TW_OK) return fail(rc_);
+                cudaMemsetAsync(s->d_done, 0, sizeof(int), s->st);
+            }
+            s->res_in_place = !s->f2[F_MM0];
+            s->res_plan = p;
+        }
     }
     if ((rc_ = s->alloc((void **)&s->src_inc, sizeof(double) * d.max_steps)) != TW_OK) return fail(rc_);
     if ((rc_ = s->alloc((void **)&s->d_energy, sizeof(double) * 3 * d.max_steps)) != TW_OK) return fail(rc_);
@@ -1587,7 +1608,7 @@ int tw_step(tw_solver *s, int n)
     if (s->steps_done + (long)n > s->d.max_steps) return TW_ERR_RECORD_FULL;
     if (n == 0) return TW_OK;
     TW_CUDA(cudaSetDevice(s->d.device));
-    if (s->res_plan.ntx > 0) {
+    if (s->res_plan.ntx > 0 && (!s->res_in_place || n >= 2)) {
         // (a captured run would be replayed with the tags of its first run)
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         TW_CUDA(cudaStreamIsCapturing(s->st, &cap));
