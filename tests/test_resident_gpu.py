@@ -236,3 +236,39 @@ def test_handles_of_different_sizes_side_by_side(tw):
     for s in shots:
         s.sync()
         s.close()
+
+
+@pytest.mark.parametrize("bc,prec,cpst", [("periodic", "f32", "00"), ("periodic", "f64", "3R"), ("periodic", "f32", "6R"),
+                                          ("free", "f32", "00"), ("free", "f64", "6R")])
+def test_batch_on_chip_matches_the_batch_kernels(tw, bc, prec, cpst, monkeypatch):
+    """Shots of uneven sizes that all fit on the chip step in groups of tiles; more than one group here."""
+    sizes = [(8, 8), (20, 33), (300, 300), (257, 511), (400, 420), (61, 700), (330, 340), (500, 380), (1000, 1030)]
+
+    def run(resident):
+        monkeypatch.setenv("TW_RESIDENT", "1" if resident else "0")
+        shots = []
+        for k, (Mx, My) in enumerate(sizes):
+            s = tw.Solver(Mx, My, 1, My, 1e-4, physics=tw.ACOUSTIC, bc_x=tw.PERIODIC if bc == "periodic" else tw.SAT_FREE,
+                          precision=prec, cpst=cpst, max_steps=16, energy=False)
+            rng = np.random.default_rng(k)
+            for g in (tw.NM, tw.MN, tw.MM):
+                s.set_material_grid(g, 0, rng.uniform(1, 2, s.shape(g)))
+                s.write_field(g, 0, rng.standard_normal(s.shape(g)))
+            s.set_source(tw.MM, Mx // 2, My // 2)
+            s.add_receivers(tw.MM, [0, Mx // 2, Mx - 1], [My - 1, My // 2, 0])
+            s.add_receivers(tw.NM, [Mx - 1], [1])
+            shots.append(s)
+        b = tw.Batch(shots)
+        for n in (5, 1, 6, 2):
+            b.step(n)
+        b.sync()
+        out = [[s.read_field(g) for g in (tw.MN, tw.NM, tw.MM)] + [s.read_receivers()] for s in shots]
+        b.close()
+        for s in shots:
+            s.close()
+        return out
+
+    for k, (x, y) in enumerate(zip(run(True), run(False))):
+        assert np.abs(x[3]).max() > 0
+        for p, q in zip(x, y):
+            assert np.array_equal(p, q), k

@@ -221,7 +221,7 @@ constexpr int TMA_QW = TMA_W + 8;    // columns of a 16-bit coefficient box: fro
 enum { RES_ELASTIC = 0, RES_AC_FREE = 1, RES_AC_PER = 2 };
 constexpr int RES_THREADS = 512;
 constexpr int RES_PAD = 4;            // rows / columns around a tile in shared memory
-constexpr int RES_STATIC = 2048;      // shared memory left to the kernel's own variables
+constexpr int RES_STATIC = 4096;      // shared memory left to the kernel's own variables
 constexpr int RES_LANES_COLS = 64;    // columns a row's threads cover: 4 on the left, then up to RES_W
 constexpr int RES_W = 58;             // most columns of a tile (column My included)
 constexpr int RES_P = 68;             // values of a shared row (FP32 rows of 5 fields 1360 bytes apart: 13 or
@@ -267,14 +267,22 @@ struct ResPlan {
     bool cs = true;           // coefficients in shared memory
     size_t smem = 0;
 };
-// the tiling of a grid over n_sm SMs with smem_max bytes each
-ResPlan resident_plan(long Mx, long My, int esize, int fields, bool comp, int n_sm, size_t smem_max);
+// the tiling of a grid over n_sm SMs with smem_max bytes each: the shortest step, or (shared: the
+// SMs run other shots at the same time) the least SM time a step
+ResPlan resident_plan(long Mx, long My, int esize, int fields, bool comp, int n_sm, size_t smem_max, bool shared = false);
 // tile index of a point (host side receiver lists)
 int resident_tile(const ResPlan &p, long Mx, long My, int row, int col);
 template <class C, int PHYS>
 cudaError_t prepare_resident(int cpst, bool energy, const ResPlan &p, int smem_max);
 template <class C, int PHYS>
 cudaError_t launch_resident(const ResArgs<C> &a, int cpst, bool energy, const ResPlan &p, cudaStream_t st);
+// the tiles of several acoustic shots in one launch: shot k's arguments shots[k] and CTAs [first[k],
+// first[k + 1]), both in device memory
+template <class C, int PHYS>
+cudaError_t prepare_resident_shots(int cpst, bool cs, int smem_max);
+template <class C, int PHYS>
+cudaError_t launch_resident_shots(const ResArgs<C> *shots, const int *first, int n, int ctas, size_t smem, int cpst, bool cs,
+                                  cudaStream_t st);
 // rows of `in` (cols periodic M- or N-type columns) with 4 more columns on the left and 8 on the right
 template <class C>
 void launch_pad_columns(const C *in, long pitch, C *out, long xpitch, int rows, int My, int n_type, cudaStream_t st);

@@ -326,8 +326,9 @@ template <> struct XV<double> {
 // PHYS: RES_ELASTIC, or acoustic (MN, NM and the pressure in MM0; only the pressure is exchanged, its halo
 // is a cross, nothing reads beyond an N-type seam): RES_AC_FREE the x free surfaces, RES_AC_PER
 // periodic x, whose halo rows are the rows at the other end.
+// blk: this CTA's tile, of nblk
 template <class C, int CPST, bool ENERGY, bool CS, int PHYS>
-__global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_constant__ ResArgs<C> a)
+__device__ __forceinline__ void resident_run(const ResArgs<C> &a, int blk, int nblk)
 {
     constexpr bool KR = Cpst<CPST>::keep_r, KC = Cpst<CPST>::keep_c, RES = KR || KC;
     constexpr int N = Vec<C>::N, H = RES_PAD, P = RES_P, LANES = RES_LANES_COLS / N;
@@ -344,7 +345,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_consta
     __shared__ XEnds<C> ends;
     const int tid = threadIdx.x;
     const int Mx = a.Mx, My = a.My;
-    const int tx = blockIdx.x / a.nty, ty = blockIdx.x - tx * a.nty;
+    const int tx = blk / a.nty, ty = blk - tx * a.nty;
     const int x0 = (int)((long)tx * Mx / a.ntx), x1 = (int)((long)(tx + 1) * Mx / a.ntx);
     const int nq4 = (My + 4) / 4;   // column quads of the grid (My + 1 columns)
     const int y0 = 4 * (int)((long)ty * nq4 / a.nty);
@@ -398,7 +399,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_consta
         altL[k] = in && ty == 0 ? a.in[F_NN][(long)g * a.pitch + My] : C(0);
         altR[k] = in && lasty ? a.in[F_NN][(long)g * a.pitch] : C(0);
     }
-    const int rb = a.rcv_off[blockIdx.x], re = a.rcv_off[blockIdx.x + 1];
+    const int rb = a.rcv_off[blk], re = a.rcv_off[blk + 1];
     const St<C> st(a.op.st, a.n > 0);
     const bool multi = a.ntx * a.nty > 1;
     const int lc = W;   // (last tile of a row) the local column of My
@@ -894,12 +895,33 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_consta
     __syncthreads();
     if (tid == 0) {
         __threadfence();
-        if (atomicAdd(a.done, 1) == (int)gridDim.x - 1) {
+        if (atomicAdd(a.done, 1) == nblk - 1) {
             *a.done = 0;
             *a.step_w = it0 + a.n;
             __threadfence();
         }
     }
+}
+
+template <class C, int CPST, bool ENERGY, bool CS, int PHYS>
+__global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_constant__ ResArgs<C> a)
+{
+    resident_run<C, CPST, ENERGY, CS, PHYS>(a, blockIdx.x, gridDim.x);
+}
+
+// several shots side by side: shot k's tiles are the CTAs [first[k], first[k + 1]). A small shot alone
+// pays a step's latency whatever its size; several share it. 24 periodic FP32 shots of 256^2 to 1024^2 (8.9
+// million cells): 119 us a step by the batch kernels, 68 here.
+template <class C, int CPST, bool CS, int PHYS>
+__global__ void __launch_bounds__(RES_THREADS, 1) k_resident_shots(const ResArgs<C> *shots, const int *first, int n)
+{
+    __shared__ ResArgs<C> a;
+    int k = 0;
+    while (k + 1 < n && first[k + 1] <= (int)blockIdx.x) k++;
+    const int *src = reinterpret_cast<const int *>(shots + k);
+    for (int i = threadIdx.x; i < (int)(sizeof(a) / sizeof(int)); i += RES_THREADS) reinterpret_cast<int *>(&a)[i] = src[i];
+    __syncthreads();
+    resident_run<C, CPST, false, CS, PHYS>(a, (int)blockIdx.x - first[k], first[k + 1] - first[k]);
 }
 
 // ------------------------------------------------------------------------------- launcher
@@ -947,6 +969,38 @@ cudaError_t launch_resident(const ResArgs<C> &a, int cpst, bool energy, const Re
     cfg.attrs = at;
     cfg.numAttrs = p.ntx * p.nty > 1 ? 1 : 0;
     return resident_kernel<C, PHYS>(cpst, energy, p.cs, [&](auto k) { return cudaLaunchKernelEx(&cfg, k, a); });
+}
+
+// the shots of a group (acoustic, the single-core tree's codes): f with the kernel's pointer
+template <class C, int PHYS, class F>
+cudaError_t resident_shots_kernel(int cpst, bool cs, F f)
+{
+    if (cpst == 0) return cs ? f(k_resident_shots<C, 0, true, PHYS>) : f(k_resident_shots<C, 0, false, PHYS>);
+    if (cpst == 4) return f(k_resident_shots<C, 4, true, PHYS>);
+    return f(k_resident_shots<C, 6, true, PHYS>);
+}
+template <class C, int PHYS>
+cudaError_t prepare_resident_shots(int cpst, bool cs, int smem_max)
+{
+    return resident_shots_kernel<C, PHYS>(cpst, cs, [&](auto k) {
+        return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);
+    });
+}
+template <class C, int PHYS>
+cudaError_t launch_resident_shots(const ResArgs<C> *shots, const int *first, int n, int ctas, size_t smem, int cpst, bool cs,
+                                  cudaStream_t st)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(RES_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return resident_shots_kernel<C, PHYS>(cpst, cs, [&](auto k) { return cudaLaunchKernelEx(&cfg, k, shots, first, n); });
 }
 
 }  // namespace tw

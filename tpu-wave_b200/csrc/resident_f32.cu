@@ -9,7 +9,7 @@ namespace tw {
 template cudaError_t prepare_resident<float, RES_ELASTIC>(int, bool, const ResPlan &, int);
 template cudaError_t launch_resident<float, RES_ELASTIC>(const ResArgs<float> &, int, bool, const ResPlan &, cudaStream_t);
 
-ResPlan resident_plan(long Mx, long My, int esize, int fields, bool comp, int n_sm, size_t smem_max)
+ResPlan resident_plan(long Mx, long My, int esize, int fields, bool comp, int n_sm, size_t smem_max, bool shared)
 {
     ResPlan best;
     double best_cost = 1e30;
@@ -48,7 +48,8 @@ ResPlan resident_plan(long Mx, long My, int esize, int fields, bool comp, int n_
             const int slots = RES_THREADS * N / RES_LANES_COLS;
             auto rounds = [&](int rows) { return rows <= slots / 2 ? 0.7 : (rows <= slots ? 1.0 : 0.75 * ((rows + 1) / 2 + slots - 1) / slots * 2); };
             const double rv = rounds(R + 4), rs = rounds(R + 1);
-            const double cost = 0.3 + rv + 1.2 * rs + (ntx * nty > 1 ? 1.5 + (6.0 * R + 6.0 * wmax) / RES_THREADS / 4 : 0.0) + (cs ? 0.0 : 0.2 * (rv + rs)) + 1e-4 * ntx * nty;
+            const double step = 0.3 + rv + 1.2 * rs + (ntx * nty > 1 ? 1.5 + (6.0 * R + 6.0 * wmax) / RES_THREADS / 4 : 0.0) + (cs ? 0.0 : 0.2 * (rv + rs)) + 1e-4 * ntx * nty;
+            const double cost = shared ? step * ntx * nty : step;
             if (cost < best_cost) {
                 best_cost = cost;
                 best.ntx = ntx;

@@ -566,11 +566,11 @@ void enqueue(tw_solver *s, int n, cudaStream_t st)
     else enqueue_steps<float, float>(s, n, st);
 }
 
-// n steps on chip, from the current buffers into the other ones
+// before n steps on chip: the exchange words' tags must not wrap, and coefficients read from L2 need
+// their periodic columns
 template <class C>
-int run_resident(tw_solver *s, int n, cudaStream_t st)
+int resident_ready(tw_solver *s, const ResPlan &p, int n, cudaStream_t st)
 {
-    const ResPlan &p = s->res_plan;
     if (s->res_tag > 0xffffffffu - (unsigned)n - 2u) {   // the tags would wrap: start over
         TW_CUDA(cudaMemsetAsync(s->xbuf, 0, s->xbuf_bytes, st));
         s->res_tag = 0;
@@ -581,6 +581,22 @@ int run_resident(tw_solver *s, int n, cudaStream_t st)
                                   (int)s->d.My, k == 0, st);
         s->coefx_dirty = false;
     }
+    return TW_OK;
+}
+
+// the padded 1/rho arrays of tiles whose coefficients stay in L2
+int resident_coefx(tw_solver *s)
+{
+    s->xpitch = (s->d.My + 16 + 3) / 4 * 4;
+    for (int k = 0; k < 2; k++)
+        if (!s->coefx[k] && s->alloc(&s->coefx[k], (size_t)s->rows[F_MN + k] * s->xpitch * s->esz) != TW_OK) return TW_ERR_NOMEM;
+    return TW_OK;
+}
+
+// the arguments of n steps on chip from the current buffers, with plan p and its receiver lists
+template <class C>
+ResArgs<C> resident_args(const tw_solver *s, const ResPlan &p, int n, const int *rcv_off, const int *rcv)
+{
     ResArgs<C> a{};
     const int po = s->res_in_place ? s->parity : s->parity ^ 1;   // the buffer of the state after the run
     void *const *fin = s->parity ? s->f2 : s->f, *const *fout = po ? s->f2 : s->f;
@@ -617,17 +633,53 @@ int run_resident(tw_solver *s, int n, cudaStream_t st)
     a.flags = s->d_flags;
     a.max_steps = s->d.max_steps;
     a.energy = s->d_energy;
-    a.rcv_off = s->d_rcv_off_r;
-    a.rcv = s->d_rcv_list_r;
+    a.rcv_off = rcv_off;
+    a.rcv = rcv;
     a.traces = s->d_traces;
+    return a;
+}
+
+// the handle after n steps on chip have been launched
+void resident_done(tw_solver *s, int n)
+{
+    s->res_tag += (unsigned)n;
+    if (!s->res_in_place) s->parity ^= 1;
+}
+
+// n steps on chip
+template <class C>
+int run_resident(tw_solver *s, int n, cudaStream_t st)
+{
+    const ResPlan &p = s->res_plan;
+    const int rc = resident_ready<C>(s, p, n, st);
+    if (rc != TW_OK) return rc;
+    const ResArgs<C> a = resident_args<C>(s, p, n, s->d_rcv_off_r, s->d_rcv_list_r);
     cudaError_t e;
     if (s->elastic) e = launch_resident<C, RES_ELASTIC>(a, s->d.cpst, s->d.energy != 0, p, st);
     else if (s->periodic) e = launch_resident<C, RES_AC_PER>(a, s->d.cpst, false, p, st);
     else e = launch_resident<C, RES_AC_FREE>(a, s->d.cpst, false, p, st);
     if (e != cudaSuccess) return cuda_fail(e, "on-chip run");
-    s->res_tag += (unsigned)n;
-    if (!s->res_in_place) s->parity ^= 1;
+    resident_done(s, n);
     return TW_OK;
+}
+
+// receivers by tile of plan p: offsets and (slot, row, column, trace row) entries
+void resident_receivers(const tw_solver *s, const ResPlan &p, std::vector<int> &off, std::vector<int> &list)
+{
+    const int nt = p.ntx * p.nty, n = (int)(s->rcv_tab.size() / 4);
+    std::vector<std::vector<int>> per(nt);
+    for (int r = 0; r < n; r++) {
+        const int *q = &s->rcv_tab[4 * r];
+        const int t = resident_tile(p, s->d.Mx, s->d.My, q[2], q[3]);
+        for (int f = 0; f < 2; f++)
+            if (q[f] >= 0) per[t].insert(per[t].end(), {q[f], q[2], q[3], 2 * r + f});
+    }
+    off.assign(nt + 1, 0);
+    list.clear();
+    for (int t = 0; t < nt; t++) {
+        off[t + 1] = off[t] + (int)per[t].size() / 4;
+        list.insert(list.end(), per[t].begin(), per[t].end());
+    }
 }
 
 // stepping coefficients and energy weights from the FP64 material arrays
@@ -786,19 +838,8 @@ int upload_receivers(tw_solver *s)
         if (rc != TW_OK) return rc;
     }
     if (s->res_plan.ntx > 0) {   // the same by tile of the on-chip run
-        const int nt = s->res_plan.ntx * s->res_plan.nty;
-        std::vector<std::vector<int>> per(nt);
-        for (int r = 0; r < n; r++) {
-            const int *q = &s->rcv_tab[4 * r];
-            const int t = resident_tile(s->res_plan, s->d.Mx, s->d.My, q[2], q[3]);
-            for (int f = 0; f < 2; f++)
-                if (q[f] >= 0) per[t].insert(per[t].end(), {q[f], q[2], q[3], 2 * r + f});
-        }
-        std::vector<int> off(nt + 1, 0), list;
-        for (int t = 0; t < nt; t++) {
-            off[t + 1] = off[t] + (int)per[t].size() / 4;
-            list.insert(list.end(), per[t].begin(), per[t].end());
-        }
+        std::vector<int> off, list;
+        resident_receivers(s, s->res_plan, off, list);
         if ((int)list.size() > s->rcv_list_cap_r) {
             s->release(s->d_rcv_list_r);
             s->d_rcv_list_r = nullptr;
@@ -1362,11 +1403,7 @@ int create_impl(tw_solver **out, const tw_grid_desc *desc, const SlabSpec &sl)
                 if ((rc_ = s->alloc((void **)&s->xbuf, s->xbuf_bytes)) != TW_OK) return fail(rc_);
                 cudaMemsetAsync(s->xbuf, 0, s->xbuf_bytes, s->st);
             }
-            if (!p.cs) {
-                s->xpitch = (My + 16 + 3) / 4 * 4;
-                for (int k = 0; k < 2; k++)
-                    if ((rc_ = s->alloc(&s->coefx[k], (size_t)s->rows[F_MN + k] * s->xpitch * s->esz)) != TW_OK) return fail(rc_);
-            }
+            if (!p.cs && (rc_ = resident_coefx(s)) != TW_OK) return fail(rc_);
             if ((rc_ = s->alloc((void **)&s->d_rcv_off_r, sizeof(int) * (p.ntx * p.nty + 1))) != TW_OK) return fail(rc_);
             if (!s->d_done) {
                 if ((rc_ = s->alloc((void **)&s->d_done, sizeof(int))) != TW_OK) return fail(rc_);
@@ -1486,10 +1523,10 @@ int tw_set_material_grid(tw_solver *s, int grid, int idx, const double *coef, lo
     if (ld < s->ref_cols[grid]) return TW_ERR_INVALID;
     TW_CUDA(cudaSetDevice(s->d.device));
     const long R = s->rows[slot], Cn = s->cols[slot];
-    std::vector<double> tmp((size_t)R * Cn);
-    for (long ix = 0; ix < R; ix++)   // a slab: its rows of the global grid's array
-        for (long iy = 0; iy < Cn; iy++) tmp[ix * Cn + iy] = coef[(ix + s->row_off) * ld + iy];
-    TW_CUDA(cudaMemcpyAsync(s->mat[slot], tmp.data(), sizeof(double) * tmp.size(), cudaMemcpyHostToDevice, s->st));
+    const double *src = coef + s->row_off * ld;   // a slab: its rows of the global grid's array
+    TW_CUDA(ld == Cn ? cudaMemcpyAsync(s->mat[slot], src, sizeof(double) * R * Cn, cudaMemcpyHostToDevice, s->st)
+                     : cudaMemcpy2DAsync(s->mat[slot], sizeof(double) * Cn, src, sizeof(double) * ld, sizeof(double) * Cn, R,
+                                         cudaMemcpyHostToDevice, s->st));
     TW_CUDA(cudaStreamSynchronize(s->st));
     s->mat_set[slot] = true;
     s->mat_dirty = true;
@@ -2558,6 +2595,17 @@ struct tw_batch {
     void *d_ac = nullptr;
     int *d_done = nullptr;
     int n_warps = 0, per_sm = TW_AC_CTAS_PER_SM;
+    // shots that all fit on the chip run there, in groups whose tiles fill the SMs, a launch a group
+    // for all the steps of a call: per shot (in group order) its plan and receiver lists, per group its
+    // shots and shared memory
+    bool resident = false;
+    struct Group { int k0, n, ctas; size_t smem; bool cs; };
+    std::vector<Group> groups;
+    std::vector<int> order;           // shots by group
+    std::vector<ResPlan> plans;       // by position in `order`
+    std::vector<int> rcv_off_at, rcv_at;   // where each shot's lists begin in d_rcv_res
+    void *d_res = nullptr;            // arguments by position
+    int *d_first = nullptr, *d_rcv_res = nullptr;   // CTA offsets (n + 1 per group), receiver lists
     cudaStream_t st = nullptr;
     cudaEvent_t done = nullptr;
     void *d_shots = nullptr, *d_gather = nullptr;
@@ -2576,7 +2624,7 @@ struct tw_batch {
     ~tw_batch()
     {
         drop_graph();
-        cudaFree(d_shots); cudaFree(d_gather); cudaFree(d_tile_shot); cudaFree(d_ac); cudaFree(d_done);
+        cudaFree(d_shots); cudaFree(d_gather); cudaFree(d_tile_shot); cudaFree(d_ac); cudaFree(d_done); cudaFree(d_res); cudaFree(d_first); cudaFree(d_rcv_res);
         if (done) cudaEventDestroy(done);
         if (st) cudaStreamDestroy(st);
     }
@@ -2684,6 +2732,115 @@ int batch_layout(tw_batch *b, const BatchShape &shape)
     return b->precision == TW_FP64 ? batch_layout_t<double, double>(b, shape) : batch_layout_t<float, float>(b, shape);
 }
 
+// plans, groups and receiver lists of a batch whose shots all fit on the chip (resident stays false
+// where one does not: the fused or per-point kernels then step every shot)
+template <class C>
+int batch_resident_layout_t(tw_batch *b)
+{
+    const int n = (int)b->shots.size();
+    int n_sm = 0, smem_max = 0;
+    TW_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, b->device));
+    TW_CUDA(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, b->device));
+    smem_max = std::max(0, smem_max - RES_STATIC);
+    std::vector<ResPlan> plans(n);
+    for (int k = 0; k < n; k++) {
+        const tw_solver *s = b->shots[k];
+        if (s->res_plan.ntx <= 0) return TW_OK;
+        plans[k] = resident_plan(s->d.Mx, s->d.My, s->esz, 3, b->cpst != TW_CPST_00, n_sm, (size_t)smem_max, true);
+        if (plans[k].ntx <= 0) return TW_OK;
+    }
+    // largest first, each into the first group with room
+    std::vector<int> by(n);
+    for (int k = 0; k < n; k++) by[k] = k;
+    auto ctas = [&](int k) { return plans[k].ntx * plans[k].nty; };
+    std::stable_sort(by.begin(), by.end(), [&](int x, int y) { return ctas(x) > ctas(y); });
+    std::vector<std::vector<int>> groups;
+    std::vector<int> used;
+    for (int k : by) {
+        size_t g = 0;
+        while (g < groups.size() && (used[g] + ctas(k) > n_sm || plans[groups[g][0]].cs != plans[k].cs)) g++;
+        if (g == groups.size()) {
+            groups.emplace_back();
+            used.push_back(0);
+        }
+        groups[g].push_back(k);
+        used[g] += ctas(k);
+    }
+    std::vector<int> first, lists;
+    for (size_t g = 0; g < groups.size(); g++) {
+        tw_batch::Group G{(int)b->order.size(), (int)groups[g].size(), 0, 0, plans[groups[g][0]].cs};
+        for (int k : groups[g]) {
+            tw_solver *s = b->shots[k];
+            if (!s->xbuf) {   // (a shot of one tile when alone)
+                s->xbuf_bytes = (size_t)2 * (s->d.Mx + 1) * ((s->d.My + 2) & ~1L) * 2 * s->esz;
+                if (s->alloc((void **)&s->xbuf, s->xbuf_bytes) != TW_OK) return TW_ERR_NOMEM;
+                TW_CUDA(cudaMemsetAsync(s->xbuf, 0, s->xbuf_bytes, s->st));
+            }
+            if (!plans[k].cs) {
+                const int rc = resident_coefx(s);
+                if (rc != TW_OK) return rc;
+            }
+            first.push_back(G.ctas);
+            G.ctas += ctas(k);
+            G.smem = std::max(G.smem, plans[k].smem);
+            b->order.push_back(k);
+            b->plans.push_back(plans[k]);
+            std::vector<int> off, list;
+            resident_receivers(s, plans[k], off, list);
+            b->rcv_off_at.push_back((int)lists.size());
+            lists.insert(lists.end(), off.begin(), off.end());
+            while (lists.size() % 4) lists.push_back(0);
+            b->rcv_at.push_back((int)lists.size());
+            lists.insert(lists.end(), list.begin(), list.end());
+        }
+        first.push_back(G.ctas);
+        b->groups.push_back(G);
+    }
+    lists.push_back(0);
+    for (const auto &g : b->groups)
+        TW_CUDA(b->periodic ? (prepare_resident_shots<C, RES_AC_PER>(b->cpst, g.cs, smem_max))
+                            : (prepare_resident_shots<C, RES_AC_FREE>(b->cpst, g.cs, smem_max)));
+    TW_CUDA(cudaMalloc(&b->d_res, sizeof(ResArgs<C>) * n));
+    TW_CUDA(cudaMalloc((void **)&b->d_first, sizeof(int) * first.size()));
+    TW_CUDA(cudaMalloc((void **)&b->d_rcv_res, sizeof(int) * lists.size()));
+    TW_CUDA(cudaMemcpyAsync(b->d_first, first.data(), sizeof(int) * first.size(), cudaMemcpyHostToDevice, b->st));
+    TW_CUDA(cudaMemcpyAsync(b->d_rcv_res, lists.data(), sizeof(int) * lists.size(), cudaMemcpyHostToDevice, b->st));
+    TW_CUDA(cudaStreamSynchronize(b->st));
+    for (tw_solver *s : b->shots) TW_CUDA(cudaStreamSynchronize(s->st));
+    b->resident = true;
+    return TW_OK;
+}
+
+// n steps (2 or more) of every shot, a launch a group
+template <class C>
+int run_batch_resident_t(tw_batch *b, int n)
+{
+    const int ns = (int)b->shots.size();
+    std::vector<ResArgs<C>> args(ns);
+    for (int i = 0; i < ns; i++) {
+        tw_solver *s = b->shots[b->order[i]];
+        const int rc = resident_ready<C>(s, b->plans[i], n, b->st);
+        if (rc != TW_OK) return rc;
+        args[i] = resident_args<C>(s, b->plans[i], n, b->d_rcv_res + b->rcv_off_at[i], b->d_rcv_res + b->rcv_at[i]);
+    }
+    TW_CUDA(cudaMemcpyAsync(b->d_res, args.data(), sizeof(ResArgs<C>) * ns, cudaMemcpyHostToDevice, b->st));
+    int at = 0;
+    for (const auto &g : b->groups) {
+        const ResArgs<C> *a = (const ResArgs<C> *)b->d_res + g.k0;
+        const cudaError_t e = b->periodic ? launch_resident_shots<C, RES_AC_PER>(a, b->d_first + at, g.n, g.ctas, g.smem, b->cpst, g.cs, b->st)
+                                          : launch_resident_shots<C, RES_AC_FREE>(a, b->d_first + at, g.n, g.ctas, g.smem, b->cpst, g.cs, b->st);
+        if (e != cudaSuccess) return cuda_fail(e, "on-chip batch");
+        for (int i = 0; i < g.n; i++) resident_done(b->shots[b->order[g.k0 + i]], n);
+        at += g.n + 1;
+    }
+    return TW_OK;
+}
+
+int run_batch_resident(tw_batch *b, int n)
+{
+    return b->precision == TW_FP64 ? run_batch_resident_t<double>(b, n) : run_batch_resident_t<float>(b, n);
+}
+
 template <class S, class C>
 void enqueue_batch_t(tw_batch *b, int n, cudaStream_t st)
 {
@@ -2751,7 +2908,8 @@ int tw_batch_create(tw_batch **out, tw_solver *const *shots, int n)
     if (e != cudaSuccess) return fail(cuda_fail(e, "tw_batch_create"));
     b->fused = true;
     for (tw_solver *s : b->shots) b->fused = b->fused && s->pfuse;
-    const int rc = b->fused ? batch_fused_layout(b, TW_AC_CTAS_PER_SM) : batch_layout(b, BatchShape{32, 8, 1, 0});
+    int rc = b->fused ? batch_fused_layout(b, TW_AC_CTAS_PER_SM) : batch_layout(b, BatchShape{32, 8, 1, 0});
+    if (rc == TW_OK) rc = b->precision == TW_FP64 ? batch_resident_layout_t<double>(b) : batch_resident_layout_t<float>(b);
     if (rc != TW_OK) return fail(rc);
     *out = b;
     return TW_OK;
@@ -2820,6 +2978,27 @@ int tw_batch_tune(tw_batch *b, int steps, double *best_ms)
     double best = 1e300;
     BatchShape pick = b->shape;
     int rc = TW_OK;
+    if (b->resident && steps >= 2) {   // nothing to choose: the shots' tilings are their plans'
+        for (int q = 0; q < 2 && rc == TW_OK; q++) {
+            for (tw_solver *s : b->shots) cudaMemsetAsync(s->d_step, 0, sizeof(int), b->st);
+            cudaEventRecord(e0, b->st);
+            rc = run_batch_resident(b, steps);
+            cudaEventRecord(e1, b->st);
+            const cudaError_t e = cudaEventSynchronize(e1);
+            if (rc == TW_OK && e != cudaSuccess) rc = cuda_fail(e, "tw_batch_tune");
+            float ms = 0.f;
+            if (rc == TW_OK) cudaEventElapsedTime(&ms, e0, e1);
+            best = ms / steps;
+        }
+        cudaEventDestroy(e0);
+        cudaEventDestroy(e1);
+        for (tw_solver *s : b->shots) {
+            const int r2 = tw_reset(s);
+            if (rc == TW_OK) rc = r2;
+        }
+        if (rc == TW_OK && best_ms) *best_ms = best;
+        return rc;
+    }
     for (const BatchShape &c : cand) {
         if ((rc = b->fused ? batch_fused_layout(b, c.ctas) : batch_layout(b, c)) != TW_OK) break;
         for (tw_solver *s : b->shots) cudaMemsetAsync(s->d_step, 0, sizeof(int), b->st);
@@ -2851,6 +3030,18 @@ int tw_batch_step(tw_batch *b, int n)
     if (n == 0) return TW_OK;
     TW_CUDA(cudaSetDevice(b->device));
     for (tw_solver *s : b->shots) TW_CUDA(cudaStreamSynchronize(s->st));   // queued single-shot work first
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    TW_CUDA(cudaStreamIsCapturing(b->st, &cap));
+    if (b->resident && n >= 2 && cap == cudaStreamCaptureStatusNone) {
+        const int rc = run_batch_resident(b, n);
+        if (rc != TW_OK) return rc;
+        TW_CUDA(cudaEventRecord(b->done, b->st));
+        for (tw_solver *s : b->shots) {
+            TW_CUDA(cudaStreamWaitEvent(s->st, b->done, 0));
+            s->steps_done += n;
+        }
+        return TW_OK;
+    }
     if (b->fused) {   // each shot's current buffer may have changed since the last call
         const int rc = batch_fused_layout(b, b->per_sm);
         if (rc != TW_OK) return rc;
