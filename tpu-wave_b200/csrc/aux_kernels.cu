@@ -146,6 +146,7 @@ __global__ void k_material_finalize(MaterialArgs m)
         const long i = (long)ix * m.cols[g] + iy, o = (long)ix * m.pitch + iy;
         const double rho = m.mat[g][i];
         coef[g][o] = store_coef<C, K>((C)__ddiv_rn(1., rho), m.err);
+        if (m.rho[g - F_MN]) m.rho[g - F_MN][o] = (float)rho;
         if (m.periodic) {
             m.w[g][o] = sc_weight(g);
         } else {

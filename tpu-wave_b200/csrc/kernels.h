@@ -51,6 +51,7 @@ struct MaterialArgs {
     const double *mat[5];     // FP64 NN mu, MN rho, NM rho, MM lambda (kappa), MM 2mu; rows x cols
     void *coef[5];            // stored stepping coefficients (compute type), rows x pitch
     double *w[5];             // energy weights, rows x pitch (w[4] = P2 on MM)
+    float *rho[2];            // the density as the stepper's type rounds it, MN and NM (null: not kept)
     int rows[5], cols[5];
     int Mx, My;
     long pitch;
@@ -160,6 +161,9 @@ struct FusedArgs {
     int *flags;
     int max_steps;
     const double *w[5];       // energy weights (ENERGY only)
+    const float *rho[2];      // (TMA strips) the FP32 density of MN and NM, rows x pitch, and dx dx: the energy
+    double dx2;               // weights of the strips' points follow from them and the coefficients
+    const float *ecoef[3];    // (16-bit codes) mu, lambda, 2mu before they were coded
     double *energy;           // [3][max_steps]: E_p0, E_k, E_p1
     // slabs linked in one process (tw_slab_run): the neighbour above (0) / below (1) receives this
     // slab's local rows [push_row[side], push_row[side] + FS_HALO) of every field (and residual)
@@ -197,13 +201,12 @@ constexpr int TMA_CORE = 120;        // core columns of a TMA strip (thread lane
 constexpr int TMA_Y0 = FS_WARP_CORE; // the first TMA strip starts after the first warp strip
 constexpr int TMA_W = 128;           // columns a TMA strip loads: 4 halo on each side
 constexpr int TMA_ROWS = 4;          // rows per TMA block: one per warp
-constexpr int TMA_NMAP = 15;         // tensor maps: 5 fields, 5 coefficients, 5 energy weights
+constexpr int TMA_NMAP = 10;         // tensor maps: 5 fields, 5 coefficients
 constexpr int TMA_TILE_ROWS = 12;    // the boundary CTAs' tile rows on a TMA handle (free-surface x ends)
 struct TmaMaps {
     alignas(64) unsigned char m[TMA_NMAP][128];   // CUtensorMap objects (opaque, 128 bytes each)
 };
-enum { TM_NN = 0, TM_MN, TM_NM, TM_MM0, TM_MM1, TM_PMN, TM_PNM, TM_MU, TM_LAM, TM_M2,
-       TM_WMN, TM_WNM, TM_WNN, TM_WM3, TM_WM4 };
+enum { TM_NN = 0, TM_MN, TM_NM, TM_MM0, TM_MM1, TM_PMN, TM_PNM, TM_MU, TM_LAM, TM_M2 };
 // how many strips and segments the TMA-staged step uses for a grid (0 strips: not applicable)
 int tma_strips(long My);
 template <class S, class C>

@@ -179,6 +179,8 @@ struct tw_solver {
     int *d_done = nullptr, *d_rcv_off = nullptr, *d_rcv_list = nullptr;
     int rcv_list_cap = 0;
     double *w[5] = {}, *mat[5] = {};
+    float *rho[2] = {};               // (TMA step, energy on) the FP32 density of MN and NM,
+    float *ecoef[3] = {};             // with 16-bit codes also mu, lambda, 2mu before they were coded
     // the padded node model of the last tw_set_material_model (rho, vp, vs), for the model gradient
     double *model = nullptr;
     long model_Mxp = 0, model_Myp = 0;
@@ -241,7 +243,8 @@ tw_solver::~tw_solver()
     release(src_inc); release(d_step); release(d_flags); release(d_rcv); release(d_err);
     release(d_traces); release(d_energy);
     for (int k = 0; k < 5; k++) release(coefq[k]);
-    release(d_mm);
+    release(d_mm); release(rho[0]); release(rho[1]);
+    for (int k = 0; k < 3; k++) release(ecoef[k]);
     cudaStreamSynchronize(st);   // the buffers are back in the pool before the next handle asks
     cudaStreamDestroy(st);
     if (st_side) cudaStreamDestroy(st_side);
@@ -461,6 +464,11 @@ void enqueue_fused_io(tw_solver *s, void *const *fin, void *const *fout, void *c
             a.y_tma_end = s->y_tma_end;
             a.work = s->d_done + 1;
             a.q16 = s->q16 ? 1 : 0;
+            a.rho[0] = s->rho[0];
+            a.rho[1] = s->rho[1];
+            const double dx = (double)s->d.num_dx / (double)s->d.den_dx;
+            a.dx2 = dx * dx;
+            for (int k = 0; k < 3; k++) a.ecoef[k] = s->ecoef[k];
             a.witems = s->tma_witems ? 1 : 0;
             for (int k = 0; k < 5; k++) { a.qlo[k] = s->qlo[k]; a.qstep[k] = s->qstep[k]; }
             launch_tma<S, C>(a, s->tmaps[fin == s->f ? 0 : 1], energy, st, s->st_side, s->ev_fork, s->ev_join);
@@ -695,6 +703,8 @@ int finalize_material(tw_solver *s)
         m.rows[k] = s->rows[k];
         m.cols[k] = s->cols[k];
     }
+    m.rho[0] = s->rho[0];
+    m.rho[1] = s->rho[1];
     m.Mx = (int)s->d.Mx;
     m.My = (int)s->d.My;
     m.pitch = s->pitch;
@@ -725,6 +735,11 @@ int finalize_material(tw_solver *s)
     TW_CUDA(cudaMemcpyAsync(&herr, s->d_err, sizeof(int), cudaMemcpyDeviceToHost, s->st));
     TW_CUDA(cudaStreamSynchronize(s->st));
     if (herr & 2) return TW_ERR_UNSUPPORTED;   // a coefficient outside the normal FP16 range
+    if (s->ecoef[0]) {
+        const int slot[3] = {F_NN, F_MM0, F_MM1};
+        for (int k = 0; k < 3; k++)
+            TW_CUDA(cudaMemcpyAsync(s->ecoef[k], s->coef[slot[k]], (size_t)s->rows[slot[k]] * s->pitch * sizeof(float), cudaMemcpyDeviceToDevice, s->st));
+    }
     if (s->q16)   // the codes, each array's map, and the decoded values in place of the FP32 ones
         for (int k = 0; k < 5; k++)
             if (quantize_coefficients16((float *)s->coef[k], s->coefq[k], s->rows[k], s->cols[k], s->pitch, s->d_mm,
@@ -1272,17 +1287,16 @@ int create_impl(tw_solver **out, const tw_grid_desc *desc, const SlabSpec &sl)
         }
         // the TMA-staged step (tma_step.cuh): FP32 fields and coefficients, plain update, the
         // reference's x ends, a handle of its own (not a linked slab), at least one TMA strip.
-        // With the energy every step it stages 40 bytes of FP64 weights per point and fits 3 CTAs
-        // per SM: faster than the per-warp kernel on grids below 2^25 points (98.4 against 107.5
-        // us at 2048^2, 322.7 against 353.3 at 4096^2), slower above (1181 against 1161 at
-        // 8192^2), so energy-on handles take it below that size. TW_TMA=1 / 0 in the environment
+        // With the energy every step as well (its weights follow from the coefficients and the
+        // density, tma_step.cuh; us a step against the per-warp kernel's: 2048^2 81.2 / 107.9, 4096^2 234.3
+        // / 353.5, 8192^2 808.9 / 1122). TW_TMA=1 / 0 in the environment
         // selects it / the per-warp kernel for every handle (for comparisons); its work items and
         // side segments have TW_TMA_SEG_ROWS / TW_TMA_SIDE_ROWS rows (below).
         const int nts = tma_strips(My);
         const bool want_q16 = d.coef_fp16 == 2;   // (the codes exist only where the TMA step reads them)
         if (d.precision == TW_FP32 && d.cpst == TW_CPST_00 && d.coef_fp16 != 1 && !s->slab && !(s->bnd & BND_X_IF) &&
             s->n_int_seg > 0 && nts > 0 && s->tile_rows == TMA_TILE_ROWS &&   // (the strips' launch holds this tile)
-            (want_q16 || env_int("TW_TMA", (!d.energy || (long)Mx * My < (1L << 25)) ? 1 : 0) != 0)) {
+            (want_q16 || env_int("TW_TMA", 1) != 0)) {
             int n_sm = 148;
             cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, d.device);
             s->tma = true;
@@ -1298,10 +1312,11 @@ int create_impl(tw_solver **out, const tw_grid_desc *desc, const SlabSpec &sl)
             // work items of about TW_TMA_SEG_ROWS rows for the persistent TMA CTAs. Measured, us a
             // step at 16 / 20 / 24 / 32 / 40 rows: 2048^2 61.65 / 61.3 / 63.3 / 63.4 / -, 4096^2
             // 195.6 / 188.5 / 184.8 / 186.9 / -, 8192^2 (side launch) - / - / 664.0 / 679.7 / 690.1,
-            // 8192^2 with 16-bit coefficient codes - / - / 671.4 / 646.3 / 634.0; with the energy
-            // on, 2048^2 99.9 / 97.7 / 97.7 / 95.8 / 102.3
+            // 8192^2 with 16-bit coefficient codes - / - / 671.4 / 646.3 / 634.0; with the energy on
+            // 2048^2 82.7 / 81.6 / 83.3 / 83.0 / 85.5, 4096^2 257.0 / 247.0 / 242.3 / 237.6 / 234.7, 8192^2
+            // (side launch) 910.2 / 874.4 / 851.2 / 823.6 / 808.9
             const bool small = (long)Mx * My <= (1L << 22);
-            const int seg_def = s->tma_witems ? (small ? (d.energy ? 32 : 20) : 24) : (s->q16 ? 40 : 24);
+            const int seg_def = small ? 20 : (d.energy ? 40 : (s->tma_witems ? 24 : (s->q16 ? 40 : 24)));
             const int seg_rows = std::max(8, env_int("TW_TMA_SEG_ROWS", seg_def));
             const int max_seg = std::max(1, s->int_rows / 8);
             s->n_tseg = std::max(1, std::min(max_seg, (s->int_rows + seg_rows / 2) / seg_rows));
@@ -1318,6 +1333,17 @@ int create_impl(tw_solver **out, const tw_grid_desc *desc, const SlabSpec &sl)
                 (e = cudaEventCreateWithFlags(&s->ev_fork, cudaEventDisableTiming)) != cudaSuccess ||
                 (e = cudaEventCreateWithFlags(&s->ev_join, cudaEventDisableTiming)) != cudaSuccess)
                 return fail(cuda_fail(e, "side stream"));
+            if (d.energy)
+                for (int k = 0; k < 2; k++) {
+                    const size_t n = (size_t)s->rows[F_MN + k] * s->pitch;
+                    if ((rc_ = s->alloc((void **)&s->rho[k], n * sizeof(float))) != TW_OK) return fail(rc_);
+                    cudaMemsetAsync(s->rho[k], 0, n * sizeof(float), s->st);
+                }
+            if (d.energy && s->q16) {
+                const int slot[3] = {F_NN, F_MM0, F_MM1};
+                for (int k = 0; k < 3; k++)
+                    if ((rc_ = s->alloc((void **)&s->ecoef[k], (size_t)s->rows[slot[k]] * s->pitch * sizeof(float))) != TW_OK) return fail(rc_);
+            }
             s->tmaps = new (std::nothrow) TmaMaps[2];
             if (!s->tmaps) return fail(TW_ERR_NOMEM);
             if (s->q16) {
@@ -1328,17 +1354,15 @@ int create_impl(tw_solver **out, const tw_grid_desc *desc, const SlabSpec &sl)
                 }
                 if ((rc_ = s->alloc((void **)&s->d_mm, 2 * sizeof(unsigned))) != TW_OK) return fail(rc_);
             }
-            // maps by field slot: the fields of buffer `par`, the coefficients, the energy weights
+            // maps by field slot: the fields of buffer `par`, the coefficients
             const int fmap[5] = {TM_NN, TM_MN, TM_NM, TM_MM0, TM_MM1};
             const int cmap[5] = {TM_MU, TM_PMN, TM_PNM, TM_LAM, TM_M2};
-            const int wmap[5] = {TM_WNN, TM_WMN, TM_WNM, TM_WM3, TM_WM4};
             for (int par = 0; par < 2; par++)
                 for (int k = 0; k < 5; k++) {
                     TmaMaps &m = s->tmaps[par];
                     if ((rc_ = encode_rows(m.m[fmap[k]], par ? s->f2[k] : s->f[k], 4, s->rows[k], s->pitch)) != TW_OK ||
                         (rc_ = s->q16 ? encode_rows(m.m[cmap[k]], s->coefq[k], 2, s->rows[k], s->pitch, TMA_QW)
-                                      : encode_rows(m.m[cmap[k]], s->coef[k], 4, s->rows[k], s->pitch)) != TW_OK ||
-                        (rc_ = encode_rows(m.m[wmap[k]], s->w[k], 8, s->rows[k], s->pitch)) != TW_OK)
+                                      : encode_rows(m.m[cmap[k]], s->coef[k], 4, s->rows[k], s->pitch)) != TW_OK)
                         return fail(rc_);
                 }
         }

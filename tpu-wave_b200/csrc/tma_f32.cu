@@ -16,7 +16,7 @@ int tma_strips(long My)
 template <bool ENERGY, bool Q16 = false>
 static size_t tma_smem()
 {
-    return (size_t)TmaLayout<ENERGY, Q16>::bytes;
+    return (size_t)TmaLayout<Q16>::bytes;
 }
 
 // dynamic shared memory of the side launch: the boundary CTAs' velocity tile or four warp rings

@@ -21,8 +21,8 @@
 // Row bookkeeping of a segment [x0, x1) (stress rows): velocity rows j = x0 - 2 + 4q + warp and
 // stress rows i = j - 2 in step q = 0 .. Q-1, Q = ceil((x1 - x0 + 4) / 4). Arrays whose x
 // stencils reach around the row (NN, MM0, MM1) sit in 3-block rings based at row x0 - 4; the
-// velocity fields and coefficients in 2-block rings based at x0 - 2, the stress coefficients (and
-// energy weights) in 2-block rings based at x0 - 4. Copy group G = 0 carries the first block of
+// velocity fields and coefficients in 2-block rings based at x0 - 2, the stress coefficients in
+// 2-block rings based at x0 - 4. Copy group G = 0 carries the first block of
 // NN, MM0, MM1; group G >= 1 their block G and block G - 1 of every other array. Step q consumes
 // groups q and q + 1; group q + 2 is issued when step q starts, into the slots step q - 1 freed.
 // (Issuing two steps ahead needs 4- and 3-block rings: 3 CTAs fit on an SM instead of 4, and the
@@ -84,12 +84,23 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const void *map, int x, i
         : "memory");
 }
 
+// 1 / d in FP64 for the energy weights: the hardware's approximation and two Newton iterations
+// r += r (1 - d r) (each squares the error), a rounding from the exact value; not finite for d = 0, as
+// the weight is
+__device__ __forceinline__ double recip(double d)
+{
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+    r = fma(r, fma(-d, r, 1.), r);
+    return fma(r, fma(-d, r, 1.), r);
+}
+
 constexpr long long TMA_WAIT_LIMIT = 2000000000LL;   // SM cycles: about one second
 
 // shared memory of a TMA strip CTA (byte offsets from a 128-byte aligned base). Q16: the
 // coefficients arrive as 16-bit codes in rows of TMA_QW columns (from 8 columns before the strip's
 // core), each block padded to a multiple of 128 bytes (TMA destinations are 128-byte aligned)
-template <bool ENERGY, bool Q16 = false>
+template <bool Q16 = false>
 struct TmaLayout {
     // ring lengths in blocks: the arrays whose x stencils reach around the row, the other loaded
     // arrays; NB mbarriers track the copy groups in flight
@@ -99,20 +110,15 @@ struct TmaLayout {
     static constexpr int CROW = Q16 ? TMA_QW * 2 : ROW;                       // one coefficient row
     static constexpr int CBOX = TMA_ROWS * CROW;                              // bytes a coefficient copy lands
     static constexpr int CBLK = (CBOX + 127) / 128 * 128;                     // one coefficient block
-    static constexpr int WROW = TMA_ROWS * TMA_W * 8;  // one block of one FP64 energy-weight array
     static constexpr int PAD = 128;                    // lanes 0 / 31 read up to 8 bytes beyond a row
     static constexpr int o_nn = PAD, o_mm0 = o_nn + R3 * BLK, o_mm1 = o_mm0 + R3 * BLK;
     static constexpr int o_mn = o_mm1 + R3 * BLK, o_nm = o_mn + R2 * BLK, o_pmn = o_nm + R2 * BLK,
                          o_pnm = o_pmn + R2 * CBLK, o_mu = o_pnm + R2 * CBLK, o_lam = o_mu + R2 * CBLK,
                          o_m2 = o_lam + R2 * CBLK;
     static constexpr int o_vmn = o_m2 + R2 * CBLK, o_vnm = o_vmn + 2 * BLK;  // new velocities (2 blocks)
-    // the energy weights, one slot per block and set: the velocity rows' (MN, NM) at o_vw, the
-    // stress rows' (NN, MM P1, P2) at o_sw, each loaded half a step before its use (see below)
-    static constexpr int o_w = o_vnm + 2 * BLK, o_vw = o_w, o_sw = o_w + 2 * WROW;
     // NB mbarriers at o_bar, the item index at o_item, the energy reduction's 3 x FS_WARPS doubles
     // at o_red
-    static constexpr int o_bar = o_w + (ENERGY ? 5 * WROW : 0) + PAD;
-    static constexpr int NBW = NB + (ENERGY ? 2 : 0);   // barriers: the groups', then the two weight sets'
+    static constexpr int o_bar = o_vnm + 2 * BLK + PAD;
     static constexpr int o_item = o_bar + 64, o_red = o_bar + 72;
     static constexpr int bytes = o_red + 8 * 3 * FS_WARPS + 128;              // + alignment slack
     static constexpr unsigned tx0 = 3 * BLK;                                // group 0
@@ -144,7 +150,7 @@ template <bool ENERGY, bool Q16>
 __device__ bool tma_strip_cta(const FusedArgs<float, float> &a, const TmaMaps &maps, int tstrip, int tseg, int it,
                               int rcv_b, int rcv_e, EAcc &E, unsigned char *base)
 {
-    using L = TmaLayout<ENERGY, Q16>;
+    using L = TmaLayout<Q16>;
     constexpr int R3 = L::R3, R2 = L::R2, NB = L::NB;
     using C = float;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -230,31 +236,38 @@ __device__ bool tma_strip_cta(const FusedArgs<float, float> &a, const TmaMaps &m
         }
     };
 
-    // the energy weights of block qq (thread 0): the velocity rows' set is needed in step qq's
-    // first half and loaded during step qq - 1's second half, the stress rows' set is needed in
-    // step qq's second half and loaded during its first half; one slot each suffices, and the
-    // CTA keeps the shared memory of 3 CTAs per SM (a ring of two blocks per array allowed 2)
-    int vw_last = -1, sw_last = -1;   // (thread 0) the last block of each set issued
-    auto issue_vw = [&](int qq) {
-        unsigned long long *b = bar + NB;
-        mbar_expect_tx(b, 2 * L::WROW);
-        const int rv = x0 - 2 + 4 * qq;
-        tma_load_2d(base + L::o_vw, map(TM_WMN), xs, rv, b);
-        tma_load_2d(base + L::o_vw + L::WROW, map(TM_WNM), xs, rv, b);
-        vw_last = qq;
+    // The energy. Its weights are not read: the stress rows' follow from the coefficients at hand
+    // (1/mu on NN; (lambda + 2mu) and -2 lambda over 2mu (2 lambda + 2mu) on MM, in FP64), and the
+    // velocity rows' is the FP32 density behind 1/rho, loaded a step ahead into registers: 8 more bytes
+    // a point where the five FP64 weight arrays were 40, and the CTAs keep the energy-off step's shared
+    // memory, 4 on an SM instead of 3 (us a step, before -> here: 2048^2 95.8 -> 81.2, 4096^2 322 -> 234,
+    // 8192^2, where the per-warp kernel ran, 1122 -> 809; what remains above the energy-off step's 62.3, 184.9
+    // and 666 is FP64 arithmetic and conversions). The strips' rows
+    // and columns all have the interior norm dx dx, applied to the item's sums.
+    double ek = 0., ep0 = 0., ep1 = 0.;
+    float4 rmn = make_float4(0.f, 0.f, 0.f, 0.f), rnm = rmn;
+    auto load_rho = [&](int qq) {
+        const int jj = x0 - 2 + 4 * qq + warp;
+        if (core && jj >= x0 && jj < x1) {
+            rmn = __ldg(reinterpret_cast<const float4 *>(a.rho[0] + jj * pitch + c0));
+            rnm = __ldg(reinterpret_cast<const float4 *>(a.rho[1] + jj * pitch + c0));
+        }
     };
-    auto issue_sw = [&](int qq) {
-        unsigned long long *b = bar + NB + 1;
-        mbar_expect_tx(b, 3 * L::WROW);
-        const int rt = x0 - 4 + 4 * qq;
-        tma_load_2d(base + L::o_sw, map(TM_WNN), xs, rt, b);
-        tma_load_2d(base + L::o_sw + L::WROW, map(TM_WM3), xs, rt, b);
-        tma_load_2d(base + L::o_sw + 2 * L::WROW, map(TM_WM4), xs, rt, b);
-        sw_last = qq;
+    // 16-bit coefficient codes: the weights are those of the coefficients as they were before, kept in
+    // FP32 beside the codes, loaded at the head of the step that uses them
+    float4 emu, elam, em2;
+    auto load_ecoef = [&](int qq) {
+        const int ii = x0 - 4 + 4 * qq + warp;
+        if (core && ii >= x0 && ii < x1) {
+            emu = __ldg(reinterpret_cast<const float4 *>(a.ecoef[0] + ii * pitch + c0));
+            elam = __ldg(reinterpret_cast<const float4 *>(a.ecoef[1] + ii * pitch + c0));
+            em2 = __ldg(reinterpret_cast<const float4 *>(a.ecoef[2] + ii * pitch + c0));
+        }
     };
+    if constexpr (ENERGY) load_rho(0);
 
     if (threadIdx.x == 0) {
-        for (int k = 0; k < L::NBW; k++) mbar_init(bar + k, 1);
+        for (int k = 0; k < L::NB; k++) mbar_init(bar + k, 1);
         mbar_init_fence();
     }
     __syncthreads();
@@ -263,11 +276,6 @@ __device__ bool tma_strip_cta(const FusedArgs<float, float> &a, const TmaMaps &m
         fence_proxy_async();   // the previous item's accesses to this shared memory come first
         for (int G = 0; G <= 2 && G <= Q; G++) issue(G);
         issued = Q < 2 ? Q : 2;
-        if constexpr (ENERGY)
-            if (warp == 0) {
-                issue_vw(0);
-                issue_sw(0);
-            }
     }
     int waited = -1;   // the last group this thread has seen complete
     float nf = 0.f;    // stays 0 unless a stored value is not finite (v * 0 is NaN for Inf / NaN)
@@ -287,8 +295,6 @@ __device__ bool tma_strip_cta(const FusedArgs<float, float> &a, const TmaMaps &m
             return lds4(rowp(off, row) + cl);
         }
     };
-    // this thread's weights in the set at `off` (array k of it), row `warp` of the block
-    auto wrow = [&](int off, int k) { return reinterpret_cast<const double *>(base + off + k * L::WROW) + warp * TMA_W + cl; };
     auto st4 = [&](int f, int row, const float (&v)[4]) {
         *reinterpret_cast<float4 *>(a.out[f] + row * pitch + c0) = make_float4(v[0], v[1], v[2], v[3]);
     };
@@ -306,17 +312,11 @@ __device__ bool tma_strip_cta(const FusedArgs<float, float> &a, const TmaMaps &m
             issue(q + 2);
             issued = q + 2;
         }
-        if constexpr (ENERGY)
-            if (threadIdx.x == 0 && q >= 1) {   // the stress rows' weights: step q - 1 has read their slot
-                fence_proxy_async();
-                issue_sw(q);
-            }
+        if constexpr (ENERGY && Q16) load_ecoef(q);
         for (int G = waited + 1; G <= q + 1 && !bad; G++) {
             bad = !mbar_wait(bar + G % NB, (unsigned)((G / NB) & 1), TMA_WAIT_LIMIT);
             if (!bad) waited = G;
         }
-        if constexpr (ENERGY)
-            if (!bad) bad = !mbar_wait(bar + NB, (unsigned)(q & 1), TMA_WAIT_LIMIT);   // velocity rows' weights
         // 3-block rings: blocks q, q + 1; other loaded rings: block q (slot sl); new-velocity
         // rings: block q (slot s2) and q - 1 (s2p)
         const int s3a = q % R3, s3b = (q + 1) % R3, sl = q % R2, s2 = q & 1, s2p = s2 ^ 1;
@@ -364,9 +364,8 @@ __device__ bool tma_strip_cta(const FusedArgs<float, float> &a, const TmaMaps &m
                     for (int e = 0; e < 4; e++) nf = __fmaf_rn(v[e], 0.f, nf);
                     if (nr > 0 || rmany) record(F_MN, j, v);
                     if constexpr (ENERGY) {
-                        const double *wr = wrow(L::o_vw, 0);
 #pragma unroll
-                        for (int e = 0; e < 4; e++) E.k = add(E.k, mul(mul((double)v[e], wr[e]), (double)v[e]));
+                        for (int e = 0; e < 4; e++) ek = fma(mul((double)v[e], (double)f4(rmn, e)), (double)v[e], ek);
                     }
                 }
             }
@@ -403,9 +402,8 @@ __device__ bool tma_strip_cta(const FusedArgs<float, float> &a, const TmaMaps &m
                     for (int e = 0; e < 4; e++) nf = __fmaf_rn(v[e], 0.f, nf);
                     if (nr > 0 || rmany) record(F_NM, j, v);
                     if constexpr (ENERGY) {
-                        const double *wr = wrow(L::o_vw, 1);
 #pragma unroll
-                        for (int e = 0; e < 4; e++) E.k = add(E.k, mul(mul((double)v[e], wr[e]), (double)v[e]));
+                        for (int e = 0; e < 4; e++) ek = fma(mul((double)v[e], (double)f4(rnm, e)), (double)v[e], ek);
                     }
                 }
             }
@@ -414,13 +412,7 @@ __device__ bool tma_strip_cta(const FusedArgs<float, float> &a, const TmaMaps &m
             bad = true;
             break;
         }
-        if constexpr (ENERGY) {
-            if (threadIdx.x == 0 && q + 1 < Q) {   // the next block's velocity-row weights: this step has read their slot
-                fence_proxy_async();
-                issue_vw(q + 1);
-            }
-            bad = !mbar_wait(bar + NB + 1, (unsigned)(q & 1), TMA_WAIT_LIMIT);   // stress rows' weights
-        }
+        if constexpr (ENERGY) load_rho(q + 1);
         // ---- stresses of row i = j - 2 (window row warp of the 3-block rings; new-velocity rows
         // relative to x0 - 2 + 4q: i is warp - 2)
         if (!bad && core && i >= x0 && i < x1) {
@@ -455,11 +447,11 @@ __device__ bool tma_strip_cta(const FusedArgs<float, float> &a, const TmaMaps &m
                 for (int e = 0; e < 4; e++) nf = __fmaf_rn(v[e], 0.f, nf);
                 if (nr > 0 || rmany) record(F_NN, i, v);
                 if constexpr (ENERGY) {
-                    const double *wr = wrow(L::o_sw, 0);
 #pragma unroll
                     for (int e = 0; e < 4; e++) {
-                        E.p0 = add(E.p0, mul(mul((double)f4(old, e), wr[e]), (double)f4(old, e)));
-                        E.p1 = add(E.p1, mul(mul((double)v[e], wr[e]), (double)v[e]));
+                        const double w = recip((double)f4(Q16 ? emu : mu, e)), o = f4(old, e), n = v[e];
+                        ep0 = fma(mul(o, w), o, ep0);
+                        ep1 = fma(mul(n, w), n, ep1);
                     }
                 }
             }
@@ -507,33 +499,28 @@ __device__ bool tma_strip_cta(const FusedArgs<float, float> &a, const TmaMaps &m
                     record(F_MM1, i, s1);
                 }
                 if constexpr (ENERGY) {
-                    const double *w3r = wrow(L::o_sw, 1), *w4r = wrow(L::o_sw, 2);
 #pragma unroll
                     for (int e = 0; e < 4; e++) {
                         const double a0 = f4(o0, e), a1 = f4(o1, e), b0 = s0[e], b1 = s1[e];
-                        E.p0 = add(E.p0, mul(mul(a0, w3r[e]), a0));
-                        E.p0 = add(E.p0, mul(mul(a1, w3r[e]), a1));
-                        E.p0 = add(E.p0, mul(mul(a0, w4r[e]), a1));
-                        E.p1 = add(E.p1, mul(mul(b0, w3r[e]), b0));
-                        E.p1 = add(E.p1, mul(mul(b1, w3r[e]), b1));
-                        E.p1 = add(E.p1, mul(mul(b0, w4r[e]), b1));
+                        const double l = f4(Q16 ? elam : lam, e), t = f4(Q16 ? em2 : m2c, e), ri = recip(mul(t, fma(2., l, t)));
+                        const double w1 = mul(add(l, t), ri), w2 = mul(mul(-2., l), ri);
+                        ep0 = fma(w1, fma(a0, a0, mul(a1, a1)), fma(w2, mul(a0, a1), ep0));
+                        ep1 = fma(w1, fma(b0, b0, mul(b1, b1)), fma(w2, mul(b0, b1), ep1));
                     }
                 }
             }
         }
-        if constexpr (ENERGY) {
-            if (__syncthreads_or(bad)) {   // (a weight copy that timed out ends the item in every thread)
-                bad = true;
-                break;
-            }
-        } else {
-            __syncthreads();
-        }
+        __syncthreads();
+    }
+    if constexpr (ENERGY) {
+        E.k = fma(ek, a.dx2, E.k);
+        E.p0 = fma(ep0, a.dx2, E.p0);
+        E.p1 = fma(ep1, a.dx2, E.p1);
     }
     if (nf != 0.f) atomicOr(a.flags, FLAG_NONFINITE);
     if (!bad) {   // every copy has landed and every thread is past the last barrier
         if (threadIdx.x == 0)
-            for (int k = 0; k < L::NBW; k++) mbar_inval(bar + k);
+            for (int k = 0; k < L::NB; k++) mbar_inval(bar + k);
         return true;
     }
     {
@@ -545,14 +532,10 @@ __device__ bool tma_strip_cta(const FusedArgs<float, float> &a, const TmaMaps &m
             // was issued)
             for (int G = issued - NB + 1 > 0 ? issued - NB + 1 : 0; G <= issued; G++)
                 mbar_wait(bar + G % NB, (unsigned)((G / NB) & 1), TMA_WAIT_LIMIT);
-            if constexpr (ENERGY) {   // and the last block of each weight set
-                if (vw_last >= 0) mbar_wait(bar + NB, (unsigned)(vw_last & 1), TMA_WAIT_LIMIT);
-                if (sw_last >= 0) mbar_wait(bar + NB + 1, (unsigned)(sw_last & 1), TMA_WAIT_LIMIT);
-            }
         }
         __syncthreads();
         if (threadIdx.x == 0)
-            for (int k = 0; k < L::NBW; k++) mbar_inval(bar + k);
+            for (int k = 0; k < L::NB; k++) mbar_inval(bar + k);
         return false;
     }
 }
@@ -633,14 +616,14 @@ __global__ void __launch_bounds__(FS_THREADS_MAX, fs_min_blocks<float, ENERGY>()
 }
 
 template <bool ENERGY, bool Q16 = false, bool WITEMS = false>
-__global__ void __launch_bounds__(FS_THREADS_MAX, ENERGY ? 3 : 4)
+__global__ void __launch_bounds__(FS_THREADS_MAX, 4)
     k_elastic_tma(FusedArgs<float, float> a, const __grid_constant__ TmaMaps maps)
 {
     extern __shared__ __align__(128) unsigned char tma_smem_raw[];
     unsigned char *base = reinterpret_cast<unsigned char *>((reinterpret_cast<unsigned long>(tma_smem_raw) + 127) & ~127ul);
     const int it = *a.step;
     const int n_side = a.n_zone * a.n_bstrip + a.n_octa;   // receiver lists: the side CTAs' come first
-    int *item_s = reinterpret_cast<int *>(base + TmaLayout<ENERGY, Q16>::o_item);
+    int *item_s = reinterpret_cast<int *>(base + TmaLayout<Q16>::o_item);
     EAcc E;
     // a persistent grid: each CTA takes items until none is left, so CTAs that find their SM busy
     // with side CTAs at first simply take fewer. With WITEMS the whole step is this launch: the
@@ -648,9 +631,9 @@ __global__ void __launch_bounds__(FS_THREADS_MAX, ENERGY ? 3 : 4)
     // (both latency-bound: taken first, so that none trails at the end; spread among the TMA
     // items instead, two loops on one SM were far slower), the rest (segment, strip) items of the
     // TMA strips; without, the side launch runs the boundary CTAs and the warp strips
-    static_assert(FS_WARPS * RingLayout<float, float, 0, ENERGY, float>::warp <= TmaLayout<ENERGY, Q16>::o_bar,
+    static_assert(FS_WARPS * RingLayout<float, float, 0, ENERGY, float>::warp <= TmaLayout<Q16>::o_bar,
                   "the warp strips' rings lie below the TMA strips' barriers");
-    static_assert(sizeof(float) * 2 * TMA_TILE_ROWS * FS_BND_W <= (size_t)TmaLayout<ENERGY, Q16>::o_bar,
+    static_assert(sizeof(float) * 2 * TMA_TILE_ROWS * FS_BND_W <= (size_t)TmaLayout<Q16>::o_bar,
                   "the boundary CTAs' tile lies below the TMA strips' barriers");
     const int n_bnd = a.n_zone * a.n_bstrip;
     for (;;) {
@@ -687,7 +670,7 @@ __global__ void __launch_bounds__(FS_THREADS_MAX, ENERGY ? 3 : 4)
         const int rcv_b = a.rcv_off[n_side + tt], rcv_e = a.rcv_off[n_side + tt + 1];
         if (!tma_strip_cta<ENERGY, Q16>(a, maps, tt % a.n_tstrip, tt / a.n_tstrip, it, rcv_b, rcv_e, E, base)) break;
     }
-    cta_energy<ENERGY>(a, E, reinterpret_cast<double *>(base + TmaLayout<ENERGY, Q16>::o_red), it);
+    cta_energy<ENERGY>(a, E, reinterpret_cast<double *>(base + TmaLayout<Q16>::o_red), it);
     step_done(a, it);
 }
 
