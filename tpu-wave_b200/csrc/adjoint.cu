@@ -13,6 +13,7 @@
 // point r sums, over the forward points that read r, the forward weight of r times their input.
 // Gradients accumulate in FP64.
 #include "kernels.h"
+#include "vec.cuh"
 
 namespace tw {
 
@@ -135,16 +136,114 @@ __device__ __forceinline__ C dyMfromN_T(const Ops<C> &o, int My, int k, G w)
 
 }  // namespace
 
+// Two kinds of block. Away from the closures, the penalties and the periodic seam a thread takes N
+// adjacent columns of one row (16 bytes) with vector loads and the interior weights; the points next to
+// them go one to a thread by the general rules, in the first blocks, so that their long chains of
+// loads do not trail. Point by point everywhere a kernel executed some 300 instructions a point, and that was
+// its time; now the three kernels move their 200 bytes a point (FP32) mostly
+// from L2 (1024 x 1024 FP32, the kernels of an adjoint step each on its own: 83 us point by point, 53 here). Both kinds
+// give the same FP32 values.
+namespace {
+
+// the plain rows [6, r1) and columns [4, c1) (whole vectors), and the other points in a row
+struct AdjLayout {
+    int r1, c1, nq, n_plain, n_edge, edge_blocks, blocks;
+};
+__host__ __device__ inline AdjLayout adj_layout(int Mx, int My, int N)
+{
+    AdjLayout l;
+    l.r1 = Mx - 6 > 6 ? Mx - 6 : 6;
+    const int last = (My - 6 - N) / N * N;   // the last vector whose taps stay 4 columns from My
+    l.c1 = My - 6 - N >= 4 && last >= 4 ? last + N : 4;
+    l.nq = (l.c1 - 4) / N;
+    l.n_plain = (l.r1 - 6) * l.nq;
+    const int rows = (Mx + 1 < 6 ? Mx + 1 : 6) + (Mx + 1 > l.r1 ? Mx + 1 - l.r1 : 0);
+    l.n_edge = rows * (My + 1) + (l.r1 - 6) * (4 + My + 1 - l.c1);
+    l.edge_blocks = (l.n_edge + 255) / 256;
+    l.blocks = l.edge_blocks + (l.n_plain + 255) / 256;
+    return l;
+}
+// the point (or the first column of the vector) of this thread; 0: none, 1: a point, 2: a vector
+__device__ __forceinline__ int adj_item(const AdjLayout &l, int Mx, int My, int N, int &ix, int &c)
+{
+    int h = blockIdx.x * 256 + threadIdx.x;
+    if ((int)blockIdx.x >= l.edge_blocks) {
+        h -= l.edge_blocks * 256;
+        if (h >= l.n_plain) return 0;
+        const int r = h / l.nq;
+        ix = 6 + r;
+        c = 4 + (h - r * l.nq) * N;
+        return 2;
+    }
+    if (h >= l.n_edge) return 0;
+    const int side = 4 + My + 1 - l.c1, n_side = (l.r1 - 6) * side;
+    if (h < n_side) {
+        const int r = h / side, q = h - r * side;
+        ix = 6 + r;
+        c = q < 4 ? q : l.c1 + q - 4;
+    } else {
+        h -= n_side;
+        const int r = h / (My + 1);
+        c = h - r * (My + 1);
+        ix = r < 6 ? r : l.r1 + r - 6;
+    }
+    return 1;
+}
+
+// the vectors of a row at columns c-2 .. c+2
+template <class C> struct Row5 { Vec<C> m2, m1, z, p1, p2; };
+__device__ __forceinline__ Row5<float> row5(const float *p)
+{
+    const u64 l = *reinterpret_cast<const u64 *>(p - 2), r = *reinterpret_cast<const u64 *>(p + 4);
+    const VF z = vld(p);
+    float l0, l1, m0, m1, m2, m3, r0, r1;
+    unpk(l, l0, l1);
+    unpk(z.a, m0, m1);
+    unpk(z.b, m2, m3);
+    unpk(r, r0, r1);
+    const u64 i = pk(m1, m2);
+    return {{l, z.a}, {pk(l1, m0), i}, z, {i, pk(m3, r0)}, {z.b, r}};
+}
+__device__ __forceinline__ Row5<double> row5(const double *p)
+{
+    const VD l = vld(p - 2), z = vld(p), r = vld(p + 2);
+    return {l, {l.b, z.a}, z, {z.b, r.a}, r};
+}
+
+// g[0..N) += the products x[i] y[i] (and u[i] v[i]) in FP64
+template <class C>
+__device__ __forceinline__ void accumulate(double *g, Vec<C> x, Vec<C> y)
+{
+    constexpr int N = Vec<C>::N;
+    C a[N], b[N];
+    vget(x, a);
+    vget(y, b);
+    double2 *q = reinterpret_cast<double2 *>(g);
+#pragma unroll
+    for (int i = 0; i < N; i += 2) {
+        double2 v = q[i / 2];
+        v.x += (double)a[i] * (double)b[i];
+        v.y += (double)a[i + 1] * (double)b[i + 1];
+        q[i / 2] = v;
+    }
+}
+
+template <class C>
+struct AdjWeights {   // the interior weights, forward and reversed
+    St<C> st, sr;
+    __device__ __forceinline__ AdjWeights(const Ops<C> &o, bool truth)
+        : st(o.st, truth), sr({o.st[3], o.st[2], o.st[1], o.st[0]}, truth) {}
+};
+
+}  // namespace
+
 // ---------------------------------------------------------------- phase A
 // W_nn = mu lam_xy, W_xx = lambda (lam_xx + lam_yy) + 2mu lam_xx, W_yy likewise with lam_yy;
 // coefficient gradients from the stress rates of v_{n+1}
 template <class C>
-__global__ void k_adj_a1(AdjArgs<C> a)
+__device__ __forceinline__ void a1_point(const AdjArgs<C> &a, int ix, int iy)
 {
-    const int iy = blockIdx.x * blockDim.x + threadIdx.x;
-    const int ix = blockIdx.y * blockDim.y + threadIdx.y;
     const int Mx = a.Mx, My = a.My;
-    if (ix > Mx || iy > My) return;
     const long p = a.pitch, o = (long)ix * p + iy;
     const C *const *v1 = a.u1;
     {   // NN
@@ -166,14 +265,56 @@ __global__ void k_adj_a1(AdjArgs<C> a)
     }
 }
 
+template <class C>
+__global__ void __launch_bounds__(256) k_adj_a1(const __grid_constant__ AdjArgs<C> a, AdjLayout l)
+{
+    pdl_enter();
+    constexpr int N = Vec<C>::N;
+    int ix, c;
+    const int kind = adj_item(l, a.Mx, a.My, N, ix, c);
+    if (kind == 1) a1_point(a, ix, c);
+    if (kind != 2) return;
+    const AdjWeights<C> W(a.op, a.nt > 0);
+    const St<C> &st = W.st;
+    const long p = a.pitch, o = (long)ix * p + c;
+    const C *mn = a.u1[F_MN] + o, *nm = a.u1[F_NM] + o;
+    const Vec<C> mn0 = vld(mn), nm0 = vld(nm);
+    {
+        const Vec<C> lam = vld(a.lam[F_NN] + o);
+        vst(a.w[F_NN] + o, mul(vld(a.coef[F_NN] + o), lam));
+        const Vec<C> h = st.add(taps<C>(st, vld(mn - 2 * p), vld(mn - p), mn0, vld(mn + p)), dyN(st, nm, nm0));
+        accumulate<C>(a.g[F_NN] + o, lam, h);
+    }
+    const Vec<C> lx = vld(a.lam[F_MM0] + o), ly = vld(a.lam[F_MM1] + o), L = vld(a.coef[F_MM0] + o), M2 = vld(a.coef[F_MM1] + o);
+    const Vec<C> s = st.add(lx, ly), Ls = mul(L, s);
+    vst(a.w[F_MM0] + o, st.add(Ls, mul(M2, lx)));
+    vst(a.w[F_MM1] + o, st.add(Ls, mul(M2, ly)));
+    const Vec<C> hx = taps<C>(st, vld(nm - p), nm0, vld(nm + p), vld(nm + 2 * p));
+    const Vec<C> hy = dyM(st, mn, mn0, false, nullptr);
+    C ex[N], ey[N], es[N], hxe[N], hye[N];
+    vget(lx, ex);
+    vget(ly, ey);
+    vget(s, es);
+    vget(hx, hxe);
+    vget(hy, hye);
+    double2 *g0 = reinterpret_cast<double2 *>(a.g[F_MM0] + o), *g1 = reinterpret_cast<double2 *>(a.g[F_MM1] + o);
+#pragma unroll
+    for (int i = 0; i < N; i += 2) {
+        double2 u = g0[i / 2], v = g1[i / 2];
+        u.x += (double)es[i] * ((double)hxe[i] + (double)hye[i]);
+        u.y += (double)es[i + 1] * ((double)hxe[i + 1] + (double)hye[i + 1]);
+        v.x += (double)ex[i] * (double)hxe[i] + (double)ey[i] * (double)hye[i];
+        v.y += (double)ex[i + 1] * (double)hxe[i + 1] + (double)ey[i + 1] * (double)hye[i + 1];
+        g0[i / 2] = u;
+        g1[i / 2] = v;
+    }
+}
+
 // lam_MN += (dxM)^T W_nn + (dy of MM from MN)^T W_yy;  lam_NM += (dy of NN from NM)^T W_nn + (dxN)^T W_xx
 template <class C>
-__global__ void k_adj_a2(AdjArgs<C> a)
+__device__ __forceinline__ void a2_point(const AdjArgs<C> &a, int ix, int iy)
 {
-    const int iy = blockIdx.x * blockDim.x + threadIdx.x;
-    const int ix = blockIdx.y * blockDim.y + threadIdx.y;
     const int Mx = a.Mx, My = a.My;
-    if (ix > Mx || iy > My) return;
     const long p = a.pitch, o = (long)ix * p + iy;
     if (ix < Mx) {   // MN (Mx x My+1)
         C v = dxM_T<C>(a.op, Mx, ix, [&](int r) { return a.w[F_NN][(long)r * p + iy]; });
@@ -190,12 +331,9 @@ __global__ void k_adj_a2(AdjArgs<C> a)
 // ---------------------------------------------------------------- phase B
 // Z = P lam_v; gradients of 1/rho from the velocity rates of sigma_n
 template <class C>
-__global__ void k_adj_b1(AdjArgs<C> a)
+__device__ __forceinline__ void b1_point(const AdjArgs<C> &a, int ix, int iy)
 {
-    const int iy = blockIdx.x * blockDim.x + threadIdx.x;
-    const int ix = blockIdx.y * blockDim.y + threadIdx.y;
     const int Mx = a.Mx, My = a.My;
-    if (ix > Mx || iy > My) return;
     const long p = a.pitch, o = (long)ix * p + iy;
     const C *const *s0 = a.u0;
     if (ix < Mx) {   // MN
@@ -218,15 +356,51 @@ __global__ void k_adj_b1(AdjArgs<C> a)
     }
 }
 
+// the end of phase A and the first half of B: at a point B's half reads the adjoint velocities A leaves there
+template <class C>
+__global__ void __launch_bounds__(256) k_adj_a2b1(const __grid_constant__ AdjArgs<C> a, AdjLayout l)
+{
+    pdl_enter();
+    constexpr int N = Vec<C>::N;
+    int ix, c;
+    const int kind = adj_item(l, a.Mx, a.My, N, ix, c);
+    if (kind == 1) {
+        a2_point(a, ix, c);
+        b1_point(a, ix, c);
+    }
+    if (kind != 2) return;
+    const AdjWeights<C> W(a.op, a.nt > 0);
+    const St<C> &st = W.st, &sr = W.sr;
+    const long p = a.pitch, o = (long)ix * p + c;
+    const C *wn = a.w[F_NN] + o, *w0 = a.w[F_MM0] + o;
+    const C *nn = a.u0[F_NN] + o, *m0 = a.u0[F_MM0] + o, *m1 = a.u0[F_MM1] + o;
+    const Row5<C> n = row5(wn);
+    const Vec<C> nn0 = vld(nn);
+    {
+        const Row5<C> y = row5(a.w[F_MM1] + o);
+        Vec<C> v = taps<C>(sr, vld(wn - p), n.z, vld(wn + p), vld(wn + 2 * p));
+        v = st.add(v, taps<C>(st, y.p1, y.z, y.m1, y.m2));
+        const Vec<C> lam = st.add(vld(a.lam[F_MN] + o), v);
+        vst(a.lam[F_MN] + o, lam);
+        vst(a.w[F_MN] + o, mul(vld(a.coef[F_MN] + o), lam));
+        const Vec<C> g = st.add(taps<C>(st, vld(nn - p), nn0, vld(nn + p), vld(nn + 2 * p)), dyN(st, m1, vld(m1)));
+        accumulate<C>(a.g[F_MN] + o, lam, g);
+    }
+    Vec<C> v = taps<C>(st, n.p2, n.p1, n.z, n.m1);
+    v = st.add(v, taps<C>(sr, vld(w0 - 2 * p), vld(w0 - p), vld(w0), vld(w0 + p)));
+    const Vec<C> lam = st.add(vld(a.lam[F_NM] + o), v);
+    vst(a.lam[F_NM] + o, lam);
+    vst(a.w[F_NM] + o, mul(vld(a.coef[F_NM] + o), lam));
+    const Vec<C> g = st.add(taps<C>(st, vld(m0 - 2 * p), vld(m0 - p), vld(m0), vld(m0 + p)), dyM(st, nn, nn0, false, nullptr));
+    accumulate<C>(a.g[F_NM] + o, lam, g);
+}
+
 // lam_NN += (dxN)^T Z_mn + SAT_MN^T Z_mn + (dy of NM from NN)^T Z_nm
 // lam_MM0 += (dxM)^T Z_nm + SAT_NM^T Z_nm;  lam_MM1 += (dy of MN from MM)^T Z_mn
 template <class C>
-__global__ void k_adj_b2(AdjArgs<C> a)
+__device__ __forceinline__ void b2_point(const AdjArgs<C> &a, int ix, int iy)
 {
-    const int iy = blockIdx.x * blockDim.x + threadIdx.x;
-    const int ix = blockIdx.y * blockDim.y + threadIdx.y;
     const int Mx = a.Mx, My = a.My;
-    if (ix > Mx || iy > My) return;
     const long p = a.pitch, o = (long)ix * p + iy;
     const C *zmn = a.w[F_MN], *znm = a.w[F_NM];
     {   // NN (Mx+1 x My+1)
@@ -249,11 +423,37 @@ __global__ void k_adj_b2(AdjArgs<C> a)
     }
 }
 
+template <class C>
+__global__ void __launch_bounds__(256) k_adj_b2(const __grid_constant__ AdjArgs<C> a, AdjLayout l)
+{
+    pdl_enter();
+    constexpr int N = Vec<C>::N;
+    int ix, c;
+    const int kind = adj_item(l, a.Mx, a.My, N, ix, c);
+    if (kind == 1) b2_point(a, ix, c);
+    if (kind != 2) return;
+    const AdjWeights<C> W(a.op, a.nt > 0);
+    const St<C> &st = W.st, &sr = W.sr;
+    const long p = a.pitch, o = (long)ix * p + c;
+    const C *zm = a.w[F_MN] + o, *zn = a.w[F_NM] + o;
+    const Row5<C> m = row5(zm), n = row5(zn);
+    {
+        Vec<C> v = taps<C>(sr, vld(zm - 2 * p), vld(zm - p), m.z, vld(zm + p));
+        v = st.add(v, taps<C>(st, n.p1, n.z, n.m1, n.m2));
+        vst(a.lam[F_NN] + o, st.add(vld(a.lam[F_NN] + o), v));
+    }
+    const Vec<C> v = taps<C>(sr, vld(zn - p), n.z, vld(zn + p), vld(zn + 2 * p));
+    vst(a.lam[F_MM0] + o, st.add(vld(a.lam[F_MM0] + o), v));
+    const Vec<C> u = taps<C>(st, m.p2, m.p1, m.z, m.m1);
+    vst(a.lam[F_MM1] + o, st.add(vld(a.lam[F_MM1] + o), u));
+}
+
 // ---------------------------------------------------------------- receivers
 // lam += R^T r_it: every receiver adds its residual at step `it` to the adjoint of its field(s)
 template <class C>
 __global__ void k_adj_inject(AdjArgs<C> a, int it)
 {
+    pdl_enter();
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= a.n_rcv) return;
     const int *e = a.rcv + 4 * q;
@@ -268,17 +468,17 @@ __global__ void k_adj_inject(AdjArgs<C> a, int it)
 template <class C>
 void launch_adjoint_step(const AdjArgs<C> &a, cudaStream_t st)
 {
-    const dim3 b(32, 8), g((a.My + 1 + 31) / 32, (a.Mx + 1 + 7) / 8);
-    k_adj_a1<C><<<g, b, 0, st>>>(a);
-    k_adj_a2<C><<<g, b, 0, st>>>(a);
-    k_adj_b1<C><<<g, b, 0, st>>>(a);
-    k_adj_b2<C><<<g, b, 0, st>>>(a);
+    const AdjLayout l = adj_layout(a.Mx, a.My, 16 / (int)sizeof(C));
+    const dim3 g(l.blocks), b(256);
+    launch_pdl(k_adj_a1<C>, g, b, 0, st, a, l);
+    launch_pdl(k_adj_a2b1<C>, g, b, 0, st, a, l);
+    launch_pdl(k_adj_b2<C>, g, b, 0, st, a, l);
 }
 
 template <class C>
 void launch_adjoint_inject(const AdjArgs<C> &a, int it, cudaStream_t st)
 {
-    if (a.n_rcv > 0) k_adj_inject<C><<<(a.n_rcv + 127) / 128, 128, 0, st>>>(a, it);
+    if (a.n_rcv > 0) launch_pdl(k_adj_inject<C>, dim3((a.n_rcv + 127) / 128), dim3(128), 0, st, a, it);
 }
 
 template void launch_adjoint_step<double>(const AdjArgs<double> &, cudaStream_t);
@@ -287,6 +487,24 @@ template void launch_adjoint_inject<double>(const AdjArgs<double> &, int, cudaSt
 template void launch_adjoint_inject<float>(const AdjArgs<float> &, int, cudaStream_t);
 
 // ---------------------------------------------------------------- model chain rule
+// the gradients of one grid as compact doubles; of the velocity grids with respect to rho (mat, compact):
+// d(1/rho)/d rho = -1/rho^2 at the interpolated FP64 density
+__global__ void __launch_bounds__(256) k_grid_gradient(const double *g, long pitch, const double *mat, double *out, int rows, int cols)
+{
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= cols) return;
+    for (int r = blockIdx.y; r < rows; r += gridDim.y) {
+        const long i = (long)r * cols + c;
+        const double v = g[r * pitch + c];
+        out[i] = mat ? __ddiv_rn(-v, mul(mat[i], mat[i])) : v;
+    }
+}
+
+void launch_grid_gradient(const double *g, long pitch, const double *mat, double *out, int rows, int cols, cudaStream_t st)
+{
+    k_grid_gradient<<<dim3((cols + 255) / 256, rows < 16384 ? rows : 16384), 256, 0, st>>>(g, pitch, mat, out, rows, cols);
+}
+
 // transpose of k_interp: scatter the gradient of one grid's interpolated quantity onto the four
 // model nodes it was interpolated from (FP64 atomics)
 __global__ void k_interp_T(int rows, int cols, int txN, int tyN, int num_dx, int den_dx, int num_dxM, int den_dxM,

@@ -260,6 +260,8 @@ struct ResArgs {
     int max_steps;
     const double *w[5];       // energy weights
     double *energy;
+    C *dump[5];               // (null: none) the state after step k of the run but the last goes to dump + k dump_stride
+    long dump_stride;
     const int *rcv_off;       // receivers by tile
     const int *rcv;           // [n][4]: field slot, row, column, trace row
     double *traces;
@@ -371,6 +373,7 @@ template <class C>
 void launch_adjoint_step(const AdjArgs<C> &a, cudaStream_t st);
 template <class C>
 void launch_adjoint_inject(const AdjArgs<C> &a, int it, cudaStream_t st);
+void launch_grid_gradient(const double *g, long pitch, const double *mat, double *out, int rows, int cols, cudaStream_t st);
 void launch_interp_T(int rows, int cols, int txN, int tyN, int num_dx, int den_dx, int num_dxM, int den_dxM,
                      long Nx_prmt, long Ny_prmt, const double *gin, double *gnode, cudaStream_t st);
 void launch_model_derive_T(const double *rho, const double *vp, const double *vs, long n, const double *g_mu,

@@ -29,172 +29,16 @@
 //
 // Thread layout: an item is one row of 16 bytes' worth of columns (4 FP32, 2 FP64), items are
 // dealt to the threads row by row. Per point the arithmetic and the order of the right-hand-side
-// terms are those of step_kernels.cu: results are bit-identical. FP32 sums and products go two at
-// a time (mul / add / sub .rn.f32x2: each half is rounded on its own, as the scalar instruction).
+// terms are those of step_kernels.cu: results are bit-identical.
 #pragma once
 #include "kernels.h"
 #include "stepper.cuh"
+#include "vec.cuh"
 
 namespace tw {
 
 namespace {
 
-using u64 = unsigned long long;
-using tw::add;   // (the scalar overloads beside the vector ones below)
-using tw::mul;
-
-// ---- vectors of 16 bytes
-template <class C> struct Vec;
-template <> struct Vec<float> {
-    static constexpr int N = 4;
-    using W = u64;   // a weight, in both halves
-    u64 a, b;
-};
-template <> struct Vec<double> {
-    static constexpr int N = 2;
-    using W = double;
-    double a, b;
-};
-using VF = Vec<float>;
-using VD = Vec<double>;
-
-__device__ __forceinline__ u64 pk(float x, float y)
-{
-    u64 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
-    return r;
-}
-__device__ __forceinline__ void unpk(u64 v, float &x, float &y) { asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v)); }
-__device__ __forceinline__ u64 mul2(u64 x, u64 y)
-{
-    u64 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(x), "l"(y));
-    return r;
-}
-__device__ __forceinline__ u64 fma2(u64 x, u64 y, u64 z)
-{
-    u64 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(x), "l"(y), "l"(z));
-    return r;
-}
-__device__ __forceinline__ u64 wt(float s) { return pk(s, s); }
-__device__ __forceinline__ double wt(double s) { return s; }
-__device__ __forceinline__ VF mul(VF x, VF y) { return {mul2(x.a, y.a), mul2(x.b, y.b)}; }
-__device__ __forceinline__ VF mulw(VF x, u64 s) { return {mul2(x.a, s), mul2(x.b, s)}; }
-__device__ __forceinline__ VD mul(VD x, VD y) { return {mul(x.a, y.a), mul(x.b, y.b)}; }
-__device__ __forceinline__ VD mulw(VD x, double s) { return {mul(x.a, s), mul(x.b, s)}; }
-__device__ __forceinline__ VF vzero(float) { return {0ull, 0ull}; }
-__device__ __forceinline__ VD vzero(double) { return {0., 0.}; }
-__device__ __forceinline__ VF vld(const float *p)
-{
-    const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(p);
-    return {v.x, v.y};
-}
-__device__ __forceinline__ VD vld(const double *p)
-{
-    const double2 v = *reinterpret_cast<const double2 *>(p);
-    return {v.x, v.y};
-}
-__device__ __forceinline__ VF vldg(const float *p)
-{
-    const ulonglong2 v = __ldg(reinterpret_cast<const ulonglong2 *>(p));
-    return {v.x, v.y};
-}
-__device__ __forceinline__ VD vldg(const double *p)
-{
-    const double2 v = __ldg(reinterpret_cast<const double2 *>(p));
-    return {v.x, v.y};
-}
-__device__ __forceinline__ void vst(float *p, VF v) { *reinterpret_cast<ulonglong2 *>(p) = make_ulonglong2(v.a, v.b); }
-__device__ __forceinline__ void vst(double *p, VD v) { *reinterpret_cast<double2 *>(p) = make_double2(v.a, v.b); }
-__device__ __forceinline__ void vget(VF v, float (&e)[4])
-{
-    unpk(v.a, e[0], e[1]);
-    unpk(v.b, e[2], e[3]);
-}
-__device__ __forceinline__ void vget(VD v, double (&e)[2])
-{
-    e[0] = v.a;
-    e[1] = v.b;
-}
-__device__ __forceinline__ VF vset(const float (&e)[4]) { return {pk(e[0], e[1]), pk(e[2], e[3])}; }
-__device__ __forceinline__ VD vset(const double (&e)[2]) { return {e[0], e[1]}; }
-
-// the stencil weights and the vector sums. A packed FP32 sum is fma(x, 1, y) with a 1 the compiler
-// cannot see through (and a difference fma(y, -1, x)): a mul.rn.f32x2 whose result feeds an
-// add.rn.f32x2 came out contracted into one rounding, and these cannot be.
-template <class C> struct St;
-template <>
-struct St<float> {
-    u64 w[4], one, mone;
-    __device__ __forceinline__ St(const float (&st)[4], bool truth)
-    {
-#pragma unroll
-        for (int k = 0; k < 4; k++) w[k] = wt(st[k]);
-        one = wt(truth ? 1.f : 2.f);
-        mone = wt(truth ? -1.f : 2.f);
-    }
-    __device__ __forceinline__ VF add(VF x, VF y) const { return {fma2(x.a, one, y.a), fma2(x.b, one, y.b)}; }
-    __device__ __forceinline__ VF sub(VF x, VF y) const { return {fma2(y.a, mone, x.a), fma2(y.b, mone, x.b)}; }
-};
-template <>
-struct St<double> {
-    double w[4];
-    __device__ __forceinline__ St(const double (&st)[4], bool)
-    {
-#pragma unroll
-        for (int k = 0; k < 4; k++) w[k] = st[k];
-    }
-    __device__ __forceinline__ VD add(VD x, VD y) const { return {tw::add(x.a, y.a), tw::add(x.b, y.b)}; }
-    __device__ __forceinline__ VD sub(VD x, VD y) const { return {tw::sub(x.a, y.a), tw::sub(x.b, y.b)}; }
-};
-
-// sum of four taps, each a vector (the leading 0 + is left out: see tma_step.cuh)
-template <class C>
-__device__ __forceinline__ Vec<C> taps(const St<C> &s, Vec<C> t0, Vec<C> t1, Vec<C> t2, Vec<C> t3)
-{
-    Vec<C> v = mulw(t0, s.w[0]);
-    v = s.add(v, mulw(t1, s.w[1]));
-    v = s.add(v, mulw(t2, s.w[2]));
-    return s.add(v, mulw(t3, s.w[3]));
-}
-// y derivative of N-type points from the M-type row p (taps c-2 .. c+1); mid: the vector at c
-__device__ __forceinline__ VF dyN(const St<float> &s, const float *p, VF mid)
-{
-    const u64 l = *reinterpret_cast<const u64 *>(p - 2);
-    float l0, l1, m0, m1, m2, m3;
-    unpk(l, l0, l1);
-    unpk(mid.a, m0, m1);
-    unpk(mid.b, m2, m3);
-    const u64 o0 = pk(l1, m0), o1 = pk(m1, m2), o2 = pk(m3, p[4]);
-    return taps<float>(s, {l, mid.a}, {o0, o1}, mid, {o1, o2});
-}
-__device__ __forceinline__ VD dyN(const St<double> &s, const double *p, VD mid)
-{
-    const VD l = vld(p - 2);
-    const double r = p[2];
-    return taps<double>(s, l, {l.b, mid.a}, mid, {mid.b, r});
-}
-// y derivative of M-type points from the N-type row p (taps c-1 .. c+2)
-// (alt: the column after the vector is *z)
-__device__ __forceinline__ VF dyM(const St<float> &s, const float *p, VF mid, bool alt, const float *z)
-{
-    const u64 r = *reinterpret_cast<const u64 *>(p + 4);
-    float m0, m1, m2, m3, r0, r1;
-    unpk(mid.a, m0, m1);
-    unpk(mid.b, m2, m3);
-    unpk(r, r0, r1);
-    if (alt) r0 = *z;
-    const u64 o0 = pk(p[-1], m0), o1 = pk(m1, m2), o2 = pk(m3, r0);
-    return taps<float>(s, {o0, o1}, mid, {o1, o2}, {mid.b, pk(r0, r1)});
-}
-__device__ __forceinline__ VD dyM(const St<double> &s, const double *p, VD mid, bool alt, const double *z)
-{
-    VD r = vld(p + 2);
-    if (alt) r.a = *z;
-    const double l = p[-1];
-    return taps<double>(s, {l, mid.a}, mid, {mid.b, r.a}, r);
-}
 
 // the closure and penalty weights of the x ends in shared memory, as Vec weights (read there with
 // one broadcast load; indexed by the row they would come from the parameter bank one by one)
@@ -327,7 +171,8 @@ template <> struct XV<double> {
 // is a cross, nothing reads beyond an N-type seam): RES_AC_FREE the x free surfaces, RES_AC_PER
 // periodic x, whose halo rows are the rows at the other end.
 // blk: this CTA's tile, of nblk
-template <class C, int CPST, bool ENERGY, bool CS, int PHYS>
+// DUMP: the state after every step goes to a.dump (the adjoint's recomputed segments)
+template <class C, int CPST, bool ENERGY, bool CS, int PHYS, bool DUMP = false>
 __device__ __forceinline__ void resident_run(const ResArgs<C> &a, int blk, int nblk)
 {
     constexpr bool KR = Cpst<CPST>::keep_r, KC = Cpst<CPST>::keep_c, RES = KR || KC;
@@ -491,6 +336,22 @@ __device__ __forceinline__ void resident_run(const ResArgs<C> &a, int blk, int n
                 v = vset(e);
             }
         };
+        // an owned row's new values into the state this step leaves
+        auto dump = [&](int f, int r, int own, const V &v) {
+            if constexpr (DUMP) {
+                if (last || own <= 0) return;   // (the last state is the run's result)
+                C *o = a.dump[f] + (long)k * a.dump_stride + (long)(x0 + r) * a.pitch + y0 + c;
+                if (own >= N) {
+                    vst(o, v);
+                } else {
+                    C e[N];
+                    vget(v, e);
+#pragma unroll
+                    for (int q = 0; q < N - 1; q++)
+                        if (q < own) o[q] = e[q];
+                }
+            }
+        };
         // the energy weights of this thread's points of a row (loaded before the points are computed)
         struct WV { double w[N]; };
         auto weights = [&](int f, int r, bool own) {
@@ -508,7 +369,7 @@ __device__ __forceinline__ void resident_run(const ResArgs<C> &a, int blk, int n
         // one row; ld(f, o): this column's vector of field f, o rows on
         auto vrow = [&](int r, C *q, auto ld) {
                 const int j = x0 + r;
-                const bool orow = r >= 0 && r < RN;
+                [[maybe_unused]] const bool orow = r >= 0 && r < RN;
                 auto coefv = [&](int f) -> V {
                     if constexpr (CS) return vld(q + index_of(f) * P + o_c);
                     else return vldg(a.coefx[f - F_MN] + (long)physr(f == F_NM, j) * a.xpitch + y0 + c + 4);
@@ -537,6 +398,7 @@ __device__ __forceinline__ void resident_run(const ResArgs<C> &a, int blk, int n
                     vupdate<CPST, C>(st, s, r_, cc);
                     if (r == srcMN) source(s);
                     vst(q + iMN * P, s);
+                    if (orow) dump(F_MN, r, ownN, s);
                     if constexpr (RES) vst(q + iMN * P + o_r, KR ? r_ : cc);
                     if constexpr (ENERGY) {
                         C e[N];
@@ -593,6 +455,7 @@ __device__ __forceinline__ void resident_run(const ResArgs<C> &a, int blk, int n
                     vupdate<CPST, C>(st, s, r_, cc);
                     if (is_srcNM(r)) source(s);
                     vst(q + iNM * P, s);
+                    if (orow) dump(F_NM, r, ownM, s);
                     if constexpr (RES) vst(q + iNM * P + o_r, KR ? r_ : cc);
                     if constexpr (ENERGY) {
                         C e[N];
@@ -671,6 +534,7 @@ __device__ __forceinline__ void resident_run(const ResArgs<C> &a, int blk, int n
                     vupdate<CPST, C>(st, s, r_, cc);
                     if (r == srcNN) source(s);
                     vst(q + iNN * P, s);
+                    dump(F_NN, r, ownN, s);
                     if constexpr (RES) vst(q + iNN * P + o_r, KR ? r_ : cc);
                     if (border) send(r, ownN, 0, s);
                     if constexpr (ENERGY) {
@@ -713,6 +577,8 @@ __device__ __forceinline__ void resident_run(const ResArgs<C> &a, int blk, int n
                     }
                     vst(q + iM0 * P, s0);
                     vst(q + iM1 * P, s1);
+                    dump(F_MM0, r, ownM, s0);
+                    dump(F_MM1, r, ownM, s1);
                     if constexpr (RES) {
                         vst(q + iM0 * P + o_r, KR ? r0 : k0);
                         vst(q + iM1 * P + o_r, KR ? r1 : k1);
@@ -903,10 +769,10 @@ __device__ __forceinline__ void resident_run(const ResArgs<C> &a, int blk, int n
     }
 }
 
-template <class C, int CPST, bool ENERGY, bool CS, int PHYS>
+template <class C, int CPST, bool ENERGY, bool CS, int PHYS, bool DUMP = false>
 __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_constant__ ResArgs<C> a)
 {
-    resident_run<C, CPST, ENERGY, CS, PHYS>(a, blockIdx.x, gridDim.x);
+    resident_run<C, CPST, ENERGY, CS, PHYS, DUMP>(a, blockIdx.x, gridDim.x);
 }
 
 // several shots side by side: shot k's tiles are the CTAs [first[k], first[k + 1]). A small shot alone
@@ -950,11 +816,24 @@ cudaError_t resident_kernel(int cpst, bool energy, bool cs, F f)
 template <class C, int PHYS>
 cudaError_t prepare_resident(int cpst, bool energy, const ResPlan &p, int smem_max)
 {
+    if constexpr (PHYS == RES_ELASTIC)
+        if (cpst == 0) {
+            const auto k = p.cs ? k_resident<C, 0, false, true, PHYS, true> : k_resident<C, 0, false, false, PHYS, true>;
+            const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);
+            if (e != cudaSuccess) return e;
+            if (energy) {   // the gradient's sweeps without the energy
+                const cudaError_t e2 = resident_kernel<C, PHYS>(0, false, p.cs, [&](auto q) {
+                    return cudaFuncSetAttribute(q, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);
+                });
+                if (e2 != cudaSuccess) return e2;
+            }
+        }
     return resident_kernel<C, PHYS>(cpst, energy, p.cs, [&](auto k) {
         return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);
     });
 }
 
+// (a.dump set: elastic, plain update, no energies)
 template <class C, int PHYS>
 cudaError_t launch_resident(const ResArgs<C> &a, int cpst, bool energy, const ResPlan &p, cudaStream_t st)
 {
@@ -968,6 +847,11 @@ cudaError_t launch_resident(const ResArgs<C> &a, int cpst, bool energy, const Re
     at[0].val.cooperative = 1;
     cfg.attrs = at;
     cfg.numAttrs = p.ntx * p.nty > 1 ? 1 : 0;
+    if constexpr (PHYS == RES_ELASTIC)
+        if (a.dump[0]) {
+            const auto k = p.cs ? k_resident<C, 0, false, true, PHYS, true> : k_resident<C, 0, false, false, PHYS, true>;
+            return cudaLaunchKernelEx(&cfg, k, a);
+        }
     return resident_kernel<C, PHYS>(cpst, energy, p.cs, [&](auto k) { return cudaLaunchKernelEx(&cfg, k, a); });
 }
 

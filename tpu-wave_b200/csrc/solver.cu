@@ -654,20 +654,29 @@ void resident_done(tw_solver *s, int n)
     if (!s->res_in_place) s->parity ^= 1;
 }
 
-// n steps on chip
+// n steps on chip; with `in`, from that state into `out` (elastic, no energies), the states between
+// them to first, first + stride, ... (the handle's own state stays as it is)
 template <class C>
-int run_resident(tw_solver *s, int n, cudaStream_t st)
+int run_resident(tw_solver *s, int n, cudaStream_t st, void *const *in = nullptr, void *const *first = nullptr,
+                 void *const *out = nullptr, long stride = 0)
 {
     const ResPlan &p = s->res_plan;
     const int rc = resident_ready<C>(s, p, n, st);
     if (rc != TW_OK) return rc;
-    const ResArgs<C> a = resident_args<C>(s, p, n, s->d_rcv_off_r, s->d_rcv_list_r);
+    ResArgs<C> a = resident_args<C>(s, p, n, s->d_rcv_off_r, s->d_rcv_list_r);
+    for (int k = 0; in && k < 5; k++) {
+        a.in[k] = (const C *)in[k];
+        a.out[k] = (C *)out[k];
+        a.dump[k] = (C *)first[k];
+        a.dump_stride = stride;
+    }
     cudaError_t e;
     if (s->elastic) e = launch_resident<C, RES_ELASTIC>(a, s->d.cpst, s->d.energy != 0, p, st);
     else if (s->periodic) e = launch_resident<C, RES_AC_PER>(a, s->d.cpst, false, p, st);
     else e = launch_resident<C, RES_AC_FREE>(a, s->d.cpst, false, p, st);
     if (e != cudaSuccess) return cuda_fail(e, "on-chip run");
-    resident_done(s, n);
+    if (in) s->res_tag += (unsigned)n;
+    else resident_done(s, n);
     return TW_OK;
 }
 
@@ -2166,14 +2175,15 @@ int copy_state(tw_solver *s, void *const *dst, void *const *src)
 // (sizes are summed on a first pass, then the same calls hand out the pieces), freed on exit
 struct DevBuf {
     cudaStream_t st;
+    int device;
     char *base = nullptr;
     size_t used = 0, size = 0;
     bool sizing = true;
-    explicit DevBuf(cudaStream_t s) : st(s) {}
+    DevBuf(cudaStream_t s, int d) : st(s), device(d) {}
     ~DevBuf()
     {
+        if (base) cudaFreeAsync(base, st);   // (back to the pool: the next gradient maps no memory)
         cudaStreamSynchronize(st);
-        cudaFree(base);
     }
     int get(void **out, size_t bytes)
     {
@@ -2190,7 +2200,10 @@ struct DevBuf {
     }
     int commit()   // allocate and zero the arena, then hand out pieces in the same order
     {
-        cudaError_t e = cudaMalloc((void **)&base, size);
+        cudaError_t e = cudaSuccess;
+        const cudaMemPool_t pool = handle_pool(device, &e);
+        if (e == cudaSuccess) e = cudaMallocFromPoolAsync((void **)&base, size, pool, st);
+        if (e != cudaSuccess) base = nullptr;
         if (e != cudaSuccess) return e == cudaErrorMemoryAllocation ? TW_ERR_NOMEM : cuda_fail(e, "tw_adjoint_gradient");
         e = cudaMemsetAsync(base, 0, size, st);
         if (e != cudaSuccess) return cuda_fail(e, "tw_adjoint_gradient");
@@ -2367,7 +2380,7 @@ int adjoint_t(tw_solver *s, int nt, const double *obs, int K, int slots, double 
     const bool periodic = K > 0;
     const int n_ck = periodic ? (nt + K - 1) / K : 0;
     const int n_rcv = (int)(s->rcv_tab.size() / 4);
-    DevBuf mem(s->st);
+    DevBuf mem(s->st, s->d.device);
     int rc;
     // periodic: checkpoints every K steps and the states of one segment; revolve: the slots, two
     // states of the plan and two scratch states for multi-step advances; both: the final state
@@ -2447,7 +2460,11 @@ int adjoint_t(tw_solver *s, int nt, const double *obs, int K, int slots, double 
         for (int c = 0; c < n_ck; c++) {
             if ((rc = copy_state(s, ck[c].data(), cur().data())) != TW_OK) return rc;
             const int n = std::min(K, nt - c * K);
-            enqueue(s, n, s->st);
+            if (s->res_plan.ntx > 0) {
+                if ((rc = run_resident<C>(s, n, s->st)) != TW_OK) return rc;
+            } else {
+                enqueue(s, n, s->st);
+            }
             s->steps_done += n;
         }
         if ((rc = copy_state(s, fin.data(), cur().data())) != TW_OK) return rc;
@@ -2458,10 +2475,14 @@ int adjoint_t(tw_solver *s, int nt, const double *obs, int K, int slots, double 
         for (int c = n_ck - 1; c >= 0; c--) {
             const int k0 = c * K, k1 = std::min(nt, k0 + K);
             TW_CUDA(cudaMemcpyAsync(s->d_step, &k0, sizeof(int), cudaMemcpyHostToDevice, s->st));
-            if ((rc = copy_state(s, seg[0].data(), ck[c].data())) != TW_OK) return rc;
-            for (int k = k0; k < k1; k++)   // step k: segment state k - k0 -> k - k0 + 1 (recomputed: no energy)
-                enqueue_fused_io<C, C>(s, seg[k - k0].data(), seg[k - k0 + 1].data(), none, none, s->st, false);
-            for (int n = k1 - 1; n >= k0; n--) adjoint_step(n, seg[n - k0].data(), seg[n + 1 - k0].data());
+            if (s->res_plan.ntx > 0) {   // on chip, every state written out (1024^2 FP32: 38 -> 21 us a step)
+                const long stride = K > 1 ? (long)((char *)seg[2][0] - (char *)seg[1][0]) / (long)sizeof(C) : 0;
+                if ((rc = run_resident<C>(s, k1 - k0, s->st, ck[c].data(), seg[1].data(), seg[k1 - k0].data(), stride)) != TW_OK) return rc;
+            } else {
+                for (int k = k0; k < k1; k++)   // step k: segment state k - k0 -> k - k0 + 1 (recomputed: no energy)
+                    enqueue_fused_io<C, C>(s, k == k0 ? ck[c].data() : seg[k - k0].data(), seg[k - k0 + 1].data(), none, none, s->st, false);
+            }
+            for (int n = k1 - 1; n >= k0; n--) adjoint_step(n, n == k0 ? ck[c].data() : seg[n - k0].data(), seg[n + 1 - k0].data());
             TW_CUDA(cudaGetLastError());
         }
     } else {
@@ -2502,25 +2523,14 @@ int adjoint_t(tw_solver *s, int nt, const double *obs, int K, int slots, double 
 
     // gradients with respect to the material on each grid: mu, rho (through 1/rho), lambda, 2mu
     for (int k = 0; k < 5; k++) {
-        TW_CUDA(cudaMemcpy2DAsync(gq[k], sizeof(double) * s->cols[k], a.g[k], sizeof(double) * s->pitch,
-                                  sizeof(double) * s->cols[k], s->rows[k], cudaMemcpyDeviceToDevice, s->st));
+        const size_t bytes = sizeof(double) * (size_t)s->rows[k] * s->cols[k];
+        launch_grid_gradient(a.g[k], s->pitch, k == F_MN || k == F_NM ? s->mat[k] : nullptr, gq[k], s->rows[k], s->cols[k], s->st);
+        TW_CUDA(cudaGetLastError());
+        if (!g_grid || !g_grid[k]) continue;
+        map_pages((char *)g_grid[k], bytes);
+        TW_CUDA(cudaMemcpyAsync(g_grid[k], gq[k], bytes, cudaMemcpyDeviceToHost, s->st));
     }
-    std::vector<double> h, m;
-    for (int k = 0; k < 5; k++) {
-        const size_t n = (size_t)s->rows[k] * s->cols[k];
-        h.resize(n);
-        TW_CUDA(cudaMemcpyAsync(h.data(), gq[k], sizeof(double) * n, cudaMemcpyDeviceToHost, s->st));
-        TW_CUDA(cudaStreamSynchronize(s->st));
-        if (k == F_MN || k == F_NM) {   // d(1/rho)/d rho = -1/rho^2 at the interpolated FP64 density
-            m.resize(n);
-            TW_CUDA(cudaMemcpyAsync(m.data(), s->mat[k], sizeof(double) * n, cudaMemcpyDeviceToHost, s->st));
-            TW_CUDA(cudaStreamSynchronize(s->st));
-            for (size_t i = 0; i < n; i++) h[i] = -h[i] / (m[i] * m[i]);
-            if (want_model) TW_CUDA(cudaMemcpyAsync(gq[k], h.data(), sizeof(double) * n, cudaMemcpyHostToDevice, s->st));
-        }
-        if (g_grid && g_grid[k]) memcpy(g_grid[k], h.data(), sizeof(double) * n);
-        TW_CUDA(cudaStreamSynchronize(s->st));
-    }
+    TW_CUDA(cudaStreamSynchronize(s->st));
     if (g_state)
         for (int k = 0; k < 5; k++) {
             if (!g_state[k]) continue;
