@@ -32,6 +32,7 @@
 // Every wait on an mbarrier gives up after about a second and raises FLAG_TIMEOUT.
 #pragma once
 #include "fused_step.cuh"
+#include "vec.cuh"
 
 namespace tw {
 
@@ -125,22 +126,6 @@ struct TmaLayout {
     static constexpr unsigned tx = 5 * BLK + 5 * CBOX;                      // groups >= 1
 };
 
-__device__ __forceinline__ float4 lds4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
-__device__ __forceinline__ float2 lds2(const float *p) { return *reinterpret_cast<const float2 *>(p); }
-
-// 7 values of a row around this thread's 4 columns: columns c-2 .. c+4 (N-type point from
-// M-type taps c-2..c+1) or c-1 .. c+5 (M-type point from N-type taps c-1..c+2)
-__device__ __forceinline__ void taps_left2(const float *row, int c, float (&t)[7], float4 mid)
-{
-    const float2 l = lds2(row + c - 2);
-    t[0] = l.x; t[1] = l.y; t[2] = mid.x; t[3] = mid.y; t[4] = mid.z; t[5] = mid.w;
-    t[6] = row[c + 4];
-}
-__device__ __forceinline__ void taps_left1(const float *row, int c, float (&t)[7], float4 mid)
-{
-    const float2 r = lds2(row + c + 4);
-    t[0] = row[c - 1]; t[1] = mid.x; t[2] = mid.y; t[3] = mid.z; t[4] = mid.w; t[5] = r.x; t[6] = r.y;
-}
 __device__ __forceinline__ float f4(const float4 &v, int e) { return e == 0 ? v.x : (e == 1 ? v.y : (e == 2 ? v.z : v.w)); }
 
 }  // namespace
@@ -163,7 +148,6 @@ __device__ bool tma_strip_cta(const FusedArgs<float, float> &a, const TmaMaps &m
     const int x1 = a.ir0 + (int)((long)(tseg + 1) * a.int_rows / a.n_tseg);
     const int Q = (x1 - x0 + 7) / 4;
     const long pitch = a.pitch;
-    const Ops<C> &op = a.op;
     unsigned long long *bar = reinterpret_cast<unsigned long long *>(base + L::o_bar);
 
     // this thread's receivers (at most 2 in registers; more fall back to the CTA's list)
@@ -278,31 +262,49 @@ __device__ bool tma_strip_cta(const FusedArgs<float, float> &a, const TmaMaps &m
         issued = Q < 2 ? Q : 2;
     }
     int waited = -1;   // the last group this thread has seen complete
-    float nf = 0.f;    // stays 0 unless a stored value is not finite (v * 0 is NaN for Inf / NaN)
+    VF nf = vzero(0.f);   // stays 0 unless a stored value is not finite (v * 0 is NaN for Inf / NaN)
     bool bad = false;
-    const float st0 = op.st[0], st1 = op.st[1], st2 = op.st[2], st3 = op.st[3];
+    // (sums without the reference's leading 0 +: 0 + x differs from x only for x = -0, and a difference in
+    // the sign of a zero sum vanishes in r = 0 + vx p: bit-identical results)
+    const St<C> st(a.op.st, a.n_tseg > 0);
     auto rowp = [&](int off, int slot) { return reinterpret_cast<const float *>(base + off) + slot * TMA_W; };
+    auto wrowp = [&](int off, int slot) { return reinterpret_cast<float *>(base + off) + slot * TMA_W; };
     // this thread's 4 coefficients of ring row `row` (0..7: block row) of the ring at `off`, of
-    // field slot f: FP32 values, or 16-bit codes decoded as qlo + qstep * code
-    auto coef4 = [&](int off, int row, int f) -> float4 {
+    // field slot f: FP32 values, or 16-bit codes decoded as qlo + qstep * code (a code as a float: the
+    // bits of 2^23 + code, less 2^23)
+    auto coefv = [&](int off, int row, int f) -> VF {
         if constexpr (Q16) {
             const unsigned char *r = base + off + (row >> 2) * L::CBLK + (row & 3) * L::CROW;
             const uint2 u = *reinterpret_cast<const uint2 *>(r + 2 * (cl + 4));
-            const float lo = a.qlo[f], st = a.qstep[f];
-            return make_float4(add(lo, mul(st, (float)(u.x & 0xffffu))), add(lo, mul(st, (float)(u.x >> 16))),
-                               add(lo, mul(st, (float)(u.y & 0xffffu))), add(lo, mul(st, (float)(u.y >> 16))));
+            const u64 lo = wt(a.qlo[f]), sp = wt(a.qstep[f]), m23 = wt(-8388608.f);
+            auto two = [&](unsigned x) {
+                const u64 c = fma2(pk(__uint_as_float(__byte_perm(x, 0x4b000000u, 0x7410)), __uint_as_float(__byte_perm(x, 0x4b000000u, 0x7432))),
+                                   st.one, m23);
+                return fma2(mul2(sp, c), st.one, lo);
+            };
+            return {two(u.x), two(u.y)};
         } else {
-            return lds4(rowp(off, row) + cl);
+            return vld(rowp(off, row) + cl);
         }
     };
-    auto st4 = [&](int f, int row, const float (&v)[4]) {
-        *reinterpret_cast<float4 *>(a.out[f] + row * pitch + c0) = make_float4(v[0], v[1], v[2], v[3]);
+    // an owned row's new values: to the output, the check, the receivers
+    auto keep = [&](int f, int row, const VF &v) {
+        vst(a.out[f] + row * pitch + c0, v);
+        nf = {fma2(v.a, 0ull, nf.a), fma2(v.b, 0ull, nf.b)};
+        if (nr > 0 || rmany) {
+            float e[4];
+            vget(v, e);
+            record(f, row, e);
+        }
     };
-    auto src = [&](int grid, int row, float (&v)[4]) {
+    auto src = [&](int grid, int row, VF &v) {
         if (a.src_grid == grid && row == a.src_ix) {
+            float e4[4];
+            vget(v, e4);
 #pragma unroll
             for (int e = 0; e < 4; e++)
-                if (c0 + e == a.src_iy) v[e] = to_s<C>(add((double)v[e], a.src_inc[it]));
+                if (c0 + e == a.src_iy) e4[e] = to_s<C>(add((double)e4[e], a.src_inc[it]));
+            v = vset(e4);
         }
     };
 
@@ -330,80 +332,45 @@ __device__ bool tma_strip_cta(const FusedArgs<float, float> &a, const TmaMaps &m
             const bool ownV = core && j >= x0 && j < x1;
             // ---- MN (row j): x from NN rows j-1..j+2 (window w+1..w+4), y from syy row j
             if (j <= x1) {
-                const float4 n1 = lds4(w3(L::o_nn, warp + 1) + cl), n2 = lds4(w3(L::o_nn, warp + 2) + cl),
-                             n3 = lds4(w3(L::o_nn, warp + 3) + cl), n4 = lds4(w3(L::o_nn, warp + 4) + cl);
-                const float *m1row = w3(L::o_mm1, warp + 2);
-                float t[7];
-                taps_left2(m1row, cl, t, lds4(m1row + cl));
-                const float4 old = lds4(rowp(L::o_mn, sl * 4 + warp) + cl);
-                const float4 p = coef4(L::o_pmn, sl * 4 + warp, F_MN);
-                float v[4];
-#pragma unroll
-                for (int e = 0; e < 4; e++) {
-                    // the reference sums from 0: 0 + x differs from x only for x = -0, and a
-                    // difference in the sign of a zero sum vanishes in r = 0 + vx * p below (and
-                    // in any later sum that has a non-zero term): bit-identical results
-                    float vx = mul(f4(n1, e), st0);
-                    vx = add(vx, mul(f4(n2, e), st1));
-                    vx = add(vx, mul(f4(n3, e), st2));
-                    vx = add(vx, mul(f4(n4, e), st3));
-                    float vy = mul(t[e], st0);
-                    vy = add(vy, mul(t[e + 1], st1));
-                    vy = add(vy, mul(t[e + 2], st2));
-                    vy = add(vy, mul(t[e + 3], st3));
-                    float r = 0.f;
-                    r = add(r, mul(vx, f4(p, e)));
-                    r = add(r, mul(vy, f4(p, e)));
-                    v[e] = add(f4(old, e), r);
-                }
+                const VF vx = taps<C>(st, vld(w3(L::o_nn, warp + 1) + cl), vld(w3(L::o_nn, warp + 2) + cl),
+                                      vld(w3(L::o_nn, warp + 3) + cl), vld(w3(L::o_nn, warp + 4) + cl));
+                const float *m1row = w3(L::o_mm1, warp + 2) + cl;
+                const VF vy = dyN(st, m1row, vld(m1row));
+                const VF p = coefv(L::o_pmn, sl * 4 + warp, F_MN);
+                VF r = st.add(vzero(0.f), mul(vx, p));
+                r = st.add(r, mul(vy, p));
+                VF v = st.add(vld(rowp(L::o_mn, sl * 4 + warp) + cl), r);
                 src(G_MN, j, v);
-                *reinterpret_cast<float4 *>(const_cast<float *>(rowp(L::o_vmn, s2 * 4 + warp)) + cl) = make_float4(v[0], v[1], v[2], v[3]);
+                vst(wrowp(L::o_vmn, s2 * 4 + warp) + cl, v);
                 if (ownV) {
-                    st4(F_MN, j, v);
-#pragma unroll
-                    for (int e = 0; e < 4; e++) nf = __fmaf_rn(v[e], 0.f, nf);
-                    if (nr > 0 || rmany) record(F_MN, j, v);
+                    keep(F_MN, j, v);
                     if constexpr (ENERGY) {
+                        float e4[4];
+                        vget(v, e4);
 #pragma unroll
-                        for (int e = 0; e < 4; e++) ek = fma(mul((double)v[e], (double)f4(rmn, e)), (double)v[e], ek);
+                        for (int e = 0; e < 4; e++) ek = fma(mul((double)e4[e], (double)f4(rmn, e)), (double)e4[e], ek);
                     }
                 }
             }
             // ---- NM (row j): x from sxx rows j-2..j+1 (window w..w+3), y from NN row j
             if (j >= x0 - 1) {
-                const float4 a0 = lds4(w3(L::o_mm0, warp) + cl), a1 = lds4(w3(L::o_mm0, warp + 1) + cl),
-                             a2 = lds4(w3(L::o_mm0, warp + 2) + cl), a3 = lds4(w3(L::o_mm0, warp + 3) + cl);
-                const float *nrow = w3(L::o_nn, warp + 2);
-                float t[7];
-                taps_left1(nrow, cl, t, lds4(nrow + cl));
-                const float4 old = lds4(rowp(L::o_nm, sl * 4 + warp) + cl);
-                const float4 p = coef4(L::o_pnm, sl * 4 + warp, F_NM);
-                float v[4];
-#pragma unroll
-                for (int e = 0; e < 4; e++) {
-                    float vy = mul(t[e], st0);
-                    vy = add(vy, mul(t[e + 1], st1));
-                    vy = add(vy, mul(t[e + 2], st2));
-                    vy = add(vy, mul(t[e + 3], st3));
-                    float vx = mul(f4(a0, e), st0);
-                    vx = add(vx, mul(f4(a1, e), st1));
-                    vx = add(vx, mul(f4(a2, e), st2));
-                    vx = add(vx, mul(f4(a3, e), st3));
-                    float r = 0.f;
-                    r = add(r, mul(vx, f4(p, e)));
-                    r = add(r, mul(vy, f4(p, e)));
-                    v[e] = add(f4(old, e), r);
-                }
+                const float *nrow = w3(L::o_nn, warp + 2) + cl;
+                const VF vy = dyM(st, nrow, vld(nrow), false, nullptr);
+                const VF vx = taps<C>(st, vld(w3(L::o_mm0, warp) + cl), vld(w3(L::o_mm0, warp + 1) + cl),
+                                      vld(w3(L::o_mm0, warp + 2) + cl), vld(w3(L::o_mm0, warp + 3) + cl));
+                const VF p = coefv(L::o_pnm, sl * 4 + warp, F_NM);
+                VF r = st.add(vzero(0.f), mul(vx, p));
+                r = st.add(r, mul(vy, p));
+                VF v = st.add(vld(rowp(L::o_nm, sl * 4 + warp) + cl), r);
                 src(G_NM, j, v);
-                *reinterpret_cast<float4 *>(const_cast<float *>(rowp(L::o_vnm, s2 * 4 + warp)) + cl) = make_float4(v[0], v[1], v[2], v[3]);
+                vst(wrowp(L::o_vnm, s2 * 4 + warp) + cl, v);
                 if (ownV) {
-                    st4(F_NM, j, v);
-#pragma unroll
-                    for (int e = 0; e < 4; e++) nf = __fmaf_rn(v[e], 0.f, nf);
-                    if (nr > 0 || rmany) record(F_NM, j, v);
+                    keep(F_NM, j, v);
                     if constexpr (ENERGY) {
+                        float e4[4];
+                        vget(v, e4);
 #pragma unroll
-                        for (int e = 0; e < 4; e++) ek = fma(mul((double)v[e], (double)f4(rnm, e)), (double)v[e], ek);
+                        for (int e = 0; e < 4; e++) ek = fma(mul((double)e4[e], (double)f4(rnm, e)), (double)e4[e], ek);
                     }
                 }
             }
@@ -418,91 +385,60 @@ __device__ bool tma_strip_cta(const FusedArgs<float, float> &a, const TmaMaps &m
         if (!bad && core && i >= x0 && i < x1) {
             const int ir = warp - 2;
             {   // NN: x from new MN rows i-2..i+1, y from new NM row i (taps c-2..c+1)
-                const float4 m0 = lds4(vr(L::o_vmn, ir - 2) + cl), m1 = lds4(vr(L::o_vmn, ir - 1) + cl),
-                             m2 = lds4(vr(L::o_vmn, ir) + cl), m3 = lds4(vr(L::o_vmn, ir + 1) + cl);
-                const float *nmrow = vr(L::o_vnm, ir);
-                float t[7];
-                taps_left2(nmrow, cl, t, lds4(nmrow + cl));
-                const float4 old = lds4(w3(L::o_nn, warp) + cl);
-                const float4 mu = coef4(L::o_mu, sl * 4 + warp, F_NN);
-                float v[4];
-#pragma unroll
-                for (int e = 0; e < 4; e++) {
-                    float vx = mul(f4(m0, e), st0);
-                    vx = add(vx, mul(f4(m1, e), st1));
-                    vx = add(vx, mul(f4(m2, e), st2));
-                    vx = add(vx, mul(f4(m3, e), st3));
-                    float vy = mul(t[e], st0);
-                    vy = add(vy, mul(t[e + 1], st1));
-                    vy = add(vy, mul(t[e + 2], st2));
-                    vy = add(vy, mul(t[e + 3], st3));
-                    float r = 0.f;
-                    r = add(r, mul(vx, f4(mu, e)));
-                    r = add(r, mul(vy, f4(mu, e)));
-                    v[e] = add(f4(old, e), r);
-                }
+                const VF vx = taps<C>(st, vld(vr(L::o_vmn, ir - 2) + cl), vld(vr(L::o_vmn, ir - 1) + cl),
+                                      vld(vr(L::o_vmn, ir) + cl), vld(vr(L::o_vmn, ir + 1) + cl));
+                const float *nmrow = vr(L::o_vnm, ir) + cl;
+                const VF vy = dyN(st, nmrow, vld(nmrow));
+                const VF old = vld(w3(L::o_nn, warp) + cl);
+                const VF mu = coefv(L::o_mu, sl * 4 + warp, F_NN);
+                VF r = st.add(vzero(0.f), mul(vx, mu));
+                r = st.add(r, mul(vy, mu));
+                VF v = st.add(old, r);
                 src(G_NN, i, v);
-                st4(F_NN, i, v);
-#pragma unroll
-                for (int e = 0; e < 4; e++) nf = __fmaf_rn(v[e], 0.f, nf);
-                if (nr > 0 || rmany) record(F_NN, i, v);
+                keep(F_NN, i, v);
                 if constexpr (ENERGY) {
+                    float o4[4], e4[4], c4[4];
+                    vget(old, o4);
+                    vget(v, e4);
+                    vget(mu, c4);
 #pragma unroll
                     for (int e = 0; e < 4; e++) {
-                        const double w = recip((double)f4(Q16 ? emu : mu, e)), o = f4(old, e), n = v[e];
+                        const double w = recip((double)(Q16 ? f4(emu, e) : c4[e])), o = o4[e], n = e4[e];
                         ep0 = fma(mul(o, w), o, ep0);
                         ep1 = fma(mul(n, w), n, ep1);
                     }
                 }
             }
             {   // MM: x from new NM rows i-1..i+2, y from new MN row i (taps c-1..c+2)
-                const float4 n0 = lds4(vr(L::o_vnm, ir - 1) + cl), n1 = lds4(vr(L::o_vnm, ir) + cl),
-                             n2 = lds4(vr(L::o_vnm, ir + 1) + cl), n3 = lds4(vr(L::o_vnm, ir + 2) + cl);
-                const float *mnrow = vr(L::o_vmn, ir);
-                float t[7];
-                taps_left1(mnrow, cl, t, lds4(mnrow + cl));
-                const float4 o0 = lds4(w3(L::o_mm0, warp) + cl), o1 = lds4(w3(L::o_mm1, warp) + cl);
-                const float4 lam = coef4(L::o_lam, sl * 4 + warp, F_MM0), m2c = coef4(L::o_m2, sl * 4 + warp, F_MM1);
-                float s0[4], s1[4];
-#pragma unroll
-                for (int e = 0; e < 4; e++) {
-                    float vx = mul(f4(n0, e), st0);
-                    vx = add(vx, mul(f4(n1, e), st1));
-                    vx = add(vx, mul(f4(n2, e), st2));
-                    vx = add(vx, mul(f4(n3, e), st3));
-                    float vy = mul(t[e], st0);
-                    vy = add(vy, mul(t[e + 1], st1));
-                    vy = add(vy, mul(t[e + 2], st2));
-                    vy = add(vy, mul(t[e + 3], st3));
-                    const float L_ = f4(lam, e), M2 = f4(m2c, e);
-                    float r0 = 0.f, r1 = 0.f;
-                    r0 = add(r0, mul(vx, L_));
-                    r1 = add(r1, mul(vx, L_));
-                    r0 = add(r0, mul(vx, M2));
-                    r0 = add(r0, mul(vy, L_));
-                    r1 = add(r1, mul(vy, L_));
-                    r1 = add(r1, mul(vy, M2));
-                    s0[e] = add(f4(o0, e), r0);
-                    s1[e] = add(f4(o1, e), r1);
-                }
+                const VF vx = taps<C>(st, vld(vr(L::o_vnm, ir - 1) + cl), vld(vr(L::o_vnm, ir) + cl),
+                                      vld(vr(L::o_vnm, ir + 1) + cl), vld(vr(L::o_vnm, ir + 2) + cl));
+                const float *mnrow = vr(L::o_vmn, ir) + cl;
+                const VF vy = dyM(st, mnrow, vld(mnrow), false, nullptr);
+                const VF o0 = vld(w3(L::o_mm0, warp) + cl), o1 = vld(w3(L::o_mm1, warp) + cl);
+                const VF lam = coefv(L::o_lam, sl * 4 + warp, F_MM0), m2c = coefv(L::o_m2, sl * 4 + warp, F_MM1);
+                const VF xl = mul(vx, lam), yl = mul(vy, lam);
+                VF r0 = st.add(vzero(0.f), xl), r1 = r0;
+                r0 = st.add(r0, mul(vx, m2c));
+                r0 = st.add(r0, yl);
+                r1 = st.add(r1, yl);
+                r1 = st.add(r1, mul(vy, m2c));
+                VF s0 = st.add(o0, r0), s1 = st.add(o1, r1);
                 src(G_MM, i, s0);
                 src(G_MM, i, s1);
-                st4(F_MM0, i, s0);
-                st4(F_MM1, i, s1);
-#pragma unroll
-                for (int e = 0; e < 4; e++) {
-                    nf = __fmaf_rn(s0[e], 0.f, nf);
-                    nf = __fmaf_rn(s1[e], 0.f, nf);
-                }
-                if (nr > 0 || rmany) {
-                    record(F_MM0, i, s0);
-                    record(F_MM1, i, s1);
-                }
+                keep(F_MM0, i, s0);
+                keep(F_MM1, i, s1);
                 if constexpr (ENERGY) {
+                    float p0[4], p1[4], n0[4], n1[4], l4[4], t4[4];
+                    vget(o0, p0);
+                    vget(o1, p1);
+                    vget(s0, n0);
+                    vget(s1, n1);
+                    vget(lam, l4);
+                    vget(m2c, t4);
 #pragma unroll
                     for (int e = 0; e < 4; e++) {
-                        const double a0 = f4(o0, e), a1 = f4(o1, e), b0 = s0[e], b1 = s1[e];
-                        const double l = f4(Q16 ? elam : lam, e), t = f4(Q16 ? em2 : m2c, e), ri = recip(mul(t, fma(2., l, t)));
+                        const double a0 = p0[e], a1 = p1[e], b0 = n0[e], b1 = n1[e];
+                        const double l = Q16 ? f4(elam, e) : l4[e], t = Q16 ? f4(em2, e) : t4[e], ri = recip(mul(t, fma(2., l, t)));
                         const double w1 = mul(add(l, t), ri), w2 = mul(mul(-2., l), ri);
                         ep0 = fma(w1, fma(a0, a0, mul(a1, a1)), fma(w2, mul(a0, a1), ep0));
                         ep1 = fma(w1, fma(b0, b0, mul(b1, b1)), fma(w2, mul(b0, b1), ep1));
@@ -517,7 +453,11 @@ __device__ bool tma_strip_cta(const FusedArgs<float, float> &a, const TmaMaps &m
         E.p0 = fma(ep0, a.dx2, E.p0);
         E.p1 = fma(ep1, a.dx2, E.p1);
     }
-    if (nf != 0.f) atomicOr(a.flags, FLAG_NONFINITE);
+    {
+        float e[4];
+        vget(nf, e);
+        if (e[0] + e[1] + e[2] + e[3] != 0.f) atomicOr(a.flags, FLAG_NONFINITE);
+    }
     if (!bad) {   // every copy has landed and every thread is past the last barrier
         if (threadIdx.x == 0)
             for (int k = 0; k < L::NB; k++) mbar_inval(bar + k);
