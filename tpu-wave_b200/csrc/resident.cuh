@@ -649,14 +649,18 @@ __device__ __forceinline__ void resident_run(const ResArgs<C> &a, int blk, int n
                 }
             }
         }
-        if constexpr (ENERGY) {   // each warp's sums; the CTA's are added up after the barrier
-            double v3[3] = {ep0, ek, ep1};
+        if constexpr (ENERGY) {   // each warp's sums (side by side); the CTA's are added up after the barrier
+            double v3[3] = {ek, ep1, ep0};
+            const int nv = k == 0 ? 3 : 2;   // (the stresses before a later step are those after the one before it)
 #pragma unroll
-            for (int q = 0; q < 3; q++) {
+            for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) v3[q] += __shfl_down_sync(0xffffffffu, v3[q], o);
-                if ((tid & 31) == 0) red[k & 1][q][tid >> 5] = v3[q];
-            }
+                for (int q = 0; q < 3; q++)
+                    if (q < nv) v3[q] += __shfl_down_sync(0xffffffffu, v3[q], o);
+            if ((tid & 31) == 0)
+#pragma unroll
+                for (int q = 0; q < 3; q++)
+                    if (q < nv) red[k & 1][q][tid >> 5] = v3[q];
         }
         __syncthreads();
         for (int q = rb + tid; q < re; q += RES_THREADS) {   // stress receivers (the owned stresses rest until S)
@@ -665,13 +669,23 @@ __device__ __forceinline__ void resident_run(const ResArgs<C> &a, int blk, int n
                 a.traces[(long)e[3] * a.max_steps + it] = (double)*at(index_of(e[0]), e[1] - x0, e[2] - y0);
         }
         if constexpr (ENERGY) {
-            if (tid < 3 && it < a.max_steps) {
-                double v = 0.;
-                for (int w = 0; w < RES_THREADS / 32; w++) v += red[k & 1][tid][w];
-                // the stresses before this step are those after the last one
-                if (tid == 0 && k > 0) v = ep_prev;
-                if (v != 0.) atomicAdd(a.energy + (long)tid * a.max_steps + it, 0.5 * v);
-                ep_prev = __shfl_sync(0x7u, v, 2);
+            constexpr int NW = RES_THREADS / 32;
+            if (tid >> 5 == NW - 1) {   // the last warp
+                const int l = tid & 31;
+                double v[3];
+#pragma unroll
+                for (int q = 0; q < 3; q++) v[q] = l < NW && (q < 2 || k == 0) ? red[k & 1][q][l] : 0.;
+#pragma unroll
+                for (int o = NW / 2; o > 0; o >>= 1)
+#pragma unroll
+                    for (int q = 0; q < 3; q++) v[q] += __shfl_down_sync(0xffffffffu, v[q], o);
+                if (k > 0) v[2] = ep_prev;
+                ep_prev = v[1];
+                if (l == 0 && it < a.max_steps) {   // records: E_p0, E_k, E_p1
+                    if (v[2] != 0.) atomicAdd(a.energy + it, 0.5 * v[2]);
+                    if (v[0] != 0.) atomicAdd(a.energy + (long)a.max_steps + it, 0.5 * v[0]);
+                    if (v[1] != 0.) atomicAdd(a.energy + 2L * a.max_steps + it, 0.5 * v[1]);
+                }
             }
         }
         if (last) break;
