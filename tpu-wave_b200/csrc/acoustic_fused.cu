@@ -16,6 +16,35 @@ namespace tw {
 
 namespace {
 
+// y derivative of an N-type-y point from M-type taps c-2..c+1 (a: column c0, b: column c1)
+template <class C>
+__device__ __forceinline__ P2<C> dyNfromM(const Ops<C> &o, const P2<C> &v, const P2<C> &p, const P2<C> &n)
+{
+    const C ta[4] = {p.a, p.b, v.a, v.b}, tb[4] = {p.b, v.a, v.b, n.a};
+    P2<C> r{C(0), C(0)};
+#pragma unroll
+    for (int w = 0; w < 4; w++) {
+        r.a = add(r.a, mul(ta[w], o.st[w]));
+        r.b = add(r.b, mul(tb[w], o.st[w]));
+    }
+    return r;
+}
+
+// y derivative of an M-type-y point from N-type taps c-1..c+2
+template <class C>
+__device__ __forceinline__ P2<C> dyMfromN(const Ops<C> &o, const P2<C> &v, const P2<C> &p, const P2<C> &n)
+{
+    const C ta[4] = {p.b, v.a, v.b, n.a}, tb[4] = {v.a, v.b, n.a, n.b};
+    P2<C> r{C(0), C(0)};
+#pragma unroll
+    for (int w = 0; w < 4; w++) {
+        r.a = add(r.a, mul(ta[w], o.st[w]));
+        r.b = add(r.b, mul(tb[w], o.st[w]));
+    }
+    return r;
+}
+
+
 template <class C>
 struct ARow {   // global values one iteration consumes
     P2<C> p1;                 // old pressure row j + 1

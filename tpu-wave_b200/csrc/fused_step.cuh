@@ -30,6 +30,7 @@
 
 #include "kernels.h"
 #include "stepper.cuh"
+#include "vec.cuh"
 
 namespace tw {
 
@@ -66,16 +67,6 @@ __device__ __forceinline__ P2<C> ld2_any(const S *row, int pa, int pb)
     return {to_c<C>(row[pa]), to_c<C>(row[pb])};
 }
 
-template <class C>
-__device__ __forceinline__ P2<C> ldg2_any(const C *row, int pa, int pb)
-{
-    if (pb == pa + 1 && !(pa & 1)) {
-        const typename Vec2<C>::T v = __ldg(reinterpret_cast<const typename Vec2<C>::T *>(row + pa));
-        return {v.x, v.y};
-    }
-    return {__ldg(row + pa), __ldg(row + pb)};
-}
-
 struct EAcc {
     double p0 = 0., k = 0., p1 = 0.;
 };
@@ -90,33 +81,95 @@ __device__ __forceinline__ void lanes(const P2<C> &v, P2<C> &p, P2<C> &n)
     n.b = __shfl_down_sync(FULL, v.b, 1);
 }
 
-// y derivative of an N-type-y point from M-type taps c-2..c+1 (a: column c0, b: column c1)
-template <class C>
-__device__ __forceinline__ P2<C> dyNfromM(const Ops<C> &o, const P2<C> &v, const P2<C> &p, const P2<C> &n)
-{
-    const C ta[4] = {p.a, p.b, v.a, v.b}, tb[4] = {p.b, v.a, v.b, n.a};
-    P2<C> r{C(0), C(0)};
+// arithmetic of a lane's column pair. PACKED: through the packed FP32 instructions (vec.cuh), each half
+// rounded on its own as the scalar instruction; taken by 16-bit storage, whose steps are bound by
+// instructions issued (us a step, scalar -> packed, 1500 x 1023: FP16 pairs 52.5 -> 49.8, BF16 pairs 54.3 -> 51.4). With FP32 storage the register pairs cost more than the packing saves (3R 3000 x 2000 139.0 ->
+// 148.0, '6C' 1000 x 1200 46.6 -> 47.6): scalar there.
+template <class C, bool PACKED>
+struct Pair {
+    C w[4];
+    __device__ __forceinline__ Pair(const C (&st)[4], bool)
+    {
 #pragma unroll
-    for (int w = 0; w < 4; w++) {
-        r.a = add(r.a, mul(ta[w], o.st[w]));
-        r.b = add(r.b, mul(tb[w], o.st[w]));
+        for (int k = 0; k < 4; k++) w[k] = st[k];
     }
-    return r;
+    __device__ __forceinline__ P2<C> add(P2<C> x, P2<C> y) const { return {tw::add(x.a, y.a), tw::add(x.b, y.b)}; }
+    __device__ __forceinline__ P2<C> sub(P2<C> x, P2<C> y) const { return {tw::sub(x.a, y.a), tw::sub(x.b, y.b)}; }
+    __device__ __forceinline__ P2<C> mul(P2<C> x, P2<C> y) const { return {tw::mul(x.a, y.a), tw::mul(x.b, y.b)}; }
+    __device__ __forceinline__ P2<C> nonfinite(P2<C> v, P2<C> nf) const { return {fma(v.a, C(0), nf.a), fma(v.b, C(0), nf.b)}; }
+    __device__ __forceinline__ P2<C> mulw(P2<C> x, int k) const { return {tw::mul(x.a, w[k]), tw::mul(x.b, w[k])}; }
+};
+template <>
+struct Pair<float, true> : St<float> {
+    using St<float>::St;
+    static __device__ __forceinline__ u64 p(P2<float> x) { return pk(x.a, x.b); }
+    static __device__ __forceinline__ P2<float> u(u64 x)
+    {
+        P2<float> r;
+        unpk(x, r.a, r.b);
+        return r;
+    }
+    __device__ __forceinline__ P2<float> add(P2<float> x, P2<float> y) const { return u(fma2(p(x), one, p(y))); }
+    __device__ __forceinline__ P2<float> sub(P2<float> x, P2<float> y) const { return u(fma2(p(y), mone, p(x))); }
+    __device__ __forceinline__ P2<float> mul(P2<float> x, P2<float> y) const { return u(mul2(p(x), p(y))); }
+    __device__ __forceinline__ P2<float> nonfinite(P2<float> v, P2<float> nf) const { return u(fma2(p(v), 0ull, p(nf))); }
+    __device__ __forceinline__ P2<float> mulw(P2<float> x, int k) const { return u(mul2(p(x), w[k])); }
+};
+// sum of four taps. ZERO: with the reference's leading 0 +, which makes a zero sum a positive zero; a
+// right-hand side that starts from 0 does that anyway (0 + vx p), one that starts from a residual does not
+template <bool ZERO, class C, bool PK>
+__device__ __forceinline__ P2<C> taps4(const Pair<C, PK> &o, P2<C> t0, P2<C> t1, P2<C> t2, P2<C> t3)
+{
+    P2<C> v = o.mulw(t0, 0);
+    if constexpr (ZERO) v = o.add(P2<C>{C(0), C(0)}, v);
+    v = o.add(v, o.mulw(t1, 1));
+    v = o.add(v, o.mulw(t2, 2));
+    return o.add(v, o.mulw(t3, 3));
+}
+
+// y derivative of an N-type-y point from M-type taps c-2..c+1 (a: column c0, b: column c1)
+template <bool ZERO, class C, bool PK>
+__device__ __forceinline__ P2<C> dyNfromM(const Pair<C, PK> &o, const P2<C> &v, const P2<C> &p, const P2<C> &n)
+{
+    return taps4<ZERO>(o, p, P2<C>{p.b, v.a}, v, P2<C>{v.b, n.a});
 }
 
 // y derivative of an M-type-y point from N-type taps c-1..c+2
-template <class C>
-__device__ __forceinline__ P2<C> dyMfromN(const Ops<C> &o, const P2<C> &v, const P2<C> &p, const P2<C> &n)
+template <bool ZERO, class C, bool PK>
+__device__ __forceinline__ P2<C> dyMfromN(const Pair<C, PK> &o, const P2<C> &v, const P2<C> &p, const P2<C> &n)
 {
-    const C ta[4] = {p.b, v.a, v.b, n.a}, tb[4] = {v.a, v.b, n.a, n.b};
-    P2<C> r{C(0), C(0)};
-#pragma unroll
-    for (int w = 0; w < 4; w++) {
-        r.a = add(r.a, mul(ta[w], o.st[w]));
-        r.b = add(r.b, mul(tb[w], o.st[w]));
-    }
-    return r;
+    return taps4<ZERO>(o, P2<C>{p.b, v.a}, v, P2<C>{v.b, n.a}, n);
 }
+
+// time_update of a pair
+template <int CPST, class C, bool PK>
+__device__ __forceinline__ void pair_update(const Pair<C, PK> &o, P2<C> &s, P2<C> &r, P2<C> &c)
+{
+    if constexpr (CPST == 0 || CPST == 7) {
+        s = o.add(s, r);
+    } else if constexpr (CPST == 1 || CPST == 3) {
+        const P2<C> y = o.add(r, c), t = o.add(s, y);
+        c = o.sub(y, o.sub(t, s));
+        s = t;
+    } else if constexpr (CPST == 2 || CPST == 4) {
+        const P2<C> t = o.add(s, r);
+        r = o.sub(r, o.sub(t, s));
+        s = t;
+    } else {
+        const P2<C> b = (CPST == 5) ? o.add(r, c) : r;
+        const P2<C> t = o.add(s, b);
+        const P2<C> pa = o.sub(t, b), pb = o.sub(t, pa);
+        const P2<C> d = o.add(o.sub(s, pa), o.sub(b, pb));
+        s = t;
+        if constexpr (CPST == 5) c = d; else r = d;
+    }
+}
+
+// a pair as 16-bit storage rounds it (one conversion of both halves)
+__device__ __forceinline__ void round2(const P2<float> &v, __half2 &h) { h = __floats2half2_rn(v.a, v.b); }
+__device__ __forceinline__ void round2(const P2<float> &v, __nv_bfloat162 &h) { h = __floats2bfloat162_rn(v.a, v.b); }
+__device__ __forceinline__ void round2(const P2<double> &v, double2 &h) { h = {v.a, v.b}; }
+__device__ __forceinline__ void round2(const P2<float> &v, float2 &h) { h = {v.a, v.b}; }
 
 template <class C>
 struct Row {   // global values one interior iteration consumes
@@ -125,6 +178,7 @@ struct Row {   // global values one interior iteration consumes
     P2<C> rmn, rnm;               // compensation of velocity row j
     P2<C> mu, lam, m2;            // coefficients of stress row j-2
     P2<C> rnn, rm0, rm1;          // compensation of stress row j-2
+    C z;                          // NN of row j across the seam
     P2<double> wmn, wnm, wnn, wm3, wm4;
 };
 
@@ -144,17 +198,28 @@ constexpr int fs_min_blocks()
 template <class C, bool ENERGY>
 constexpr int ring_depth() { return (sizeof(C) == 8 || ENERGY) ? 2 : TW_FS_RING; }
 
-template <class S, class C, int CPST, bool ENERGY, class K = C>
+// EDGE: a strip at the periodic seam (see interior_warp): one slot more, and 16-bit pairs as the two
+// 32-bit words that hold their values
+template <class S, class C, int CPST, bool ENERGY, class K, bool EDGE>
 struct RingLayout {
     static constexpr bool KR = Cpst<CPST>::keep_r, KC = Cpst<CPST>::keep_c, SPLIT = Cpst<CPST>::split;
     // slots of the storage type: nn, mm0, mm1, vmn, vnm; their lo parts (split); the residuals
-    // rmn, rnm, rnn, rm0, rm1 (R and C codes)
-    static constexpr int NS = 5 + (SPLIT ? 5 : 0) + ((KR || KC) ? 5 : 0);
+    // rmn, rnm, rnn, rm0, rm1 (R and C codes); at a seam the value of NN across it (and its lo part)
+    static constexpr int NS = 5 + (SPLIT ? 5 : 0) + ((KR || KC) ? 5 : 0) + (EDGE ? 1 : 0);
     static constexpr int NC = 5;                      // pmn, pnm, mu, lam, m2 (coefficient type K)
     static constexpr int NE = ENERGY ? 5 : 0;         // wmn, wnm, wnn, wm3, wm4 (double)
-    static constexpr int s_bytes = 32 * 2 * (int)sizeof(S), c_bytes = 32 * 2 * (int)sizeof(K), e_bytes = 32 * 16;
+    template <class T> static constexpr int slot_size() { return 2 * (EDGE && sizeof(T) == 2 ? 4 : (int)sizeof(T)); }
+    static constexpr int s_lane = slot_size<S>(), c_lane = slot_size<K>();   // bytes a lane
+    static constexpr int s_bytes = 32 * s_lane, c_bytes = 32 * c_lane, e_bytes = 32 * 16;
     static constexpr int stage = NS * s_bytes + NC * c_bytes + NE * e_bytes;
-    static constexpr int warp = stage * ring_depth<C, ENERGY>();
+};
+// the bytes of a warp's ring and the rows that fit into it
+template <class S, class C, int CPST, bool ENERGY, class K>
+struct RingSize {
+    static constexpr int D = ring_depth<C, ENERGY>(), DE = sizeof(S) == 2 ? 2 : D;
+    static constexpr int plain = RingLayout<S, C, CPST, ENERGY, K, false>::stage * D;
+    static constexpr int edge = RingLayout<S, C, CPST, ENERGY, K, true>::stage * DE;
+    static constexpr int warp = plain > edge ? plain : edge;
 };
 
 __device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -185,12 +250,12 @@ __device__ __forceinline__ void store_pair(S *o, S *ro, int c0, int c1, S h0, S 
             *reinterpret_cast<V2 *>(o + c0) = V2{h0, h1};
             if (TWO) *reinterpret_cast<V2 *>(ro + c0) = V2{l0, l1};
         }
-    } else if (o0 && o1 && !(c0 & 1)) {
+    } else if (o1) {   // (owned pairs begin at an even column >= 0; only the last may be half owned)
         *reinterpret_cast<V2 *>(o + c0) = V2{h0, h1};
         if (TWO) *reinterpret_cast<V2 *>(ro + c0) = V2{l0, l1};
-    } else {
-        if (o0) { o[c0] = h0; if (TWO) ro[c0] = l0; }
-        if (o1) { o[c1] = h1; if (TWO) ro[c1] = l1; }
+    } else if (o0) {
+        o[c0] = h0;
+        if (TWO) ro[c0] = l0;
     }
 }
 
@@ -200,7 +265,9 @@ __device__ __forceinline__ void store_pair(S *o, S *ro, int c0, int c1, S h0, S 
 // owned by the core lanes, and loads and stores are single vector accesses
 // PUSH: the slab is linked to its neighbours (tw_slab_run) and stores its rows next to a cut into
 // their halo rows as well
-template <class S, class C, int CPST, bool ENERGY, bool EDGE, class K, bool PUSH>
+// D: rows staged (D - 1 of them ahead)
+template <class S, class C, int CPST, bool ENERGY, bool EDGE, class K, bool PUSH,
+          int D = EDGE ? RingSize<S, C, CPST, ENERGY, K>::DE : RingSize<S, C, CPST, ENERGY, K>::D>
 __device__ void interior_warp(const FusedArgs<S, C> &a, int y0, int seg, int it, int rcv_b, int rcv_e, EAcc &E,
                               unsigned char *ring)
 {
@@ -218,25 +285,27 @@ __device__ void interior_warp(const FusedArgs<S, C> &a, int y0, int seg, int it,
     const int x0 = a.ir0 + (int)((long)seg * a.int_rows / a.n_int_seg);
     const int x1 = a.ir0 + (int)((long)(seg + 1) * a.int_rows / a.n_int_seg);   // rows [x0, x1)
     // NM columns next to the periodic seam read NN by the physical rule (column My and column 0
-    // of an N-type-y grid are distinct points)
-    const bool seam0 = EDGE && (c0 == -2 || c0 == -1 || c0 == My || c0 == My + 1);
-    const bool seam1 = EDGE && (c1 == -2 || c1 == -1 || c1 == My || c1 == My + 1);
+    // of an N-type-y grid are distinct points): left of column 0 the column after -1 is My, from
+    // column My on the one there is 0. That one value a row is staged with the others and takes its
+    // tap's place by a select. (Read from global memory where it was used, up to eight loads and two
+    // round trips a row, it made these strips' items of the TMA step 33.6 us long at 2048^2, the longest
+    // 62.9, the whole step; us a step, before -> here: 2048^2 63.6 -> 58.9, with the energy 82.8 -> 76.9,
+    // 1200 x 1500 40.0 -> 36.5; here FP64 1024^2 45.0 -> 39.6, FP16 pairs 1500 x 1023 59.0 -> 47.7, 3R 3000 x 2000
+    // 145.0 -> 137.7, '6C' 1000 x 1200 49.8 -> 45.2.)
+    const bool z_na = EDGE && c0 == -2;                        // columns -2 and -1: the column after -1
+    const bool z_va = EDGE && c0 == My, z_vb = EDGE && c1 == My;   // columns My and My + 1: column My itself
+    const bool z_pb = EDGE && c0 == My + 1;
+    const bool seam = z_na || z_va || z_vb || z_pb;
+    const int zcol = z_na ? My : 0;
 
+    const Pair<C, sizeof(S) == 2> P(a.op.st, a.n_int_seg > 0);
     auto rowp = [&](const S *base, int r) { return base + r * pitch; };
     auto ld2 = [&](const S *row, int pa, int pb) -> P2<C> {
         if (!EDGE) {
             const typename Vec2<S>::T v = *reinterpret_cast<const typename Vec2<S>::T *>(row + c0);
             return {to_c<C>(v.x), to_c<C>(v.y)};
         }
-        return ld2_any<C>(row, pa, pb);
-    };
-    auto ldg2 = [&](const auto *row, int pa, int pb) {
-        using T = typename std::remove_cv<typename std::remove_pointer<decltype(row)>::type>::type;
-        if (!EDGE) {
-            const typename Vec2<T>::T v = __ldg(reinterpret_cast<const typename Vec2<T>::T *>(row + c0));
-            return P2<T>{v.x, v.y};
-        }
-        return ldg2_any<T>(row, pa, pb);
+        return P2<C>{to_c<C>(row[pa]), to_c<C>(row[pb])};
     };
     // a field value pair as the stencil reads it (hi + lo under the split code)
     auto ld2f = [&](int f, int r, int pa, int pb) -> P2<C> {
@@ -250,11 +319,10 @@ __device__ void interior_warp(const FusedArgs<S, C> &a, int y0, int seg, int it,
     };
     // ---- row staging: issue(j, st) copies row j's values into ring stage st, read(st, in)
     // converts them into `in`
-    using RL = RingLayout<S, C, CPST, ENERGY, K>;
-    constexpr int D = ring_depth<C, ENERGY>();
+    using RL = RingLayout<S, C, CPST, ENERGY, K, EDGE>;
     const int l = lane;
-    auto sslot = [&](int st, int k) { return ring + st * RL::stage + k * RL::s_bytes + l * 2 * (int)sizeof(S); };
-    auto cslot = [&](int st, int k) { return ring + st * RL::stage + RL::NS * RL::s_bytes + k * RL::c_bytes + l * 2 * (int)sizeof(K); };
+    auto sslot = [&](int st, int k) { return ring + st * RL::stage + k * RL::s_bytes + l * RL::s_lane; };
+    auto cslot = [&](int st, int k) { return ring + st * RL::stage + RL::NS * RL::s_bytes + k * RL::c_bytes + l * RL::c_lane; };
     auto coef = [&](int f) { return reinterpret_cast<const K *>(a.coef[f]); };
     auto eslot = [&](int st, int k) {
         return ring + st * RL::stage + RL::NS * RL::s_bytes + RL::NC * RL::c_bytes + k * RL::e_bytes + l * 16;
@@ -264,13 +332,25 @@ __device__ void interior_warp(const FusedArgs<S, C> &a, int y0, int seg, int it,
         using T = typename std::remove_cv<typename std::remove_pointer<decltype(row)>::type>::type;
         if (!EDGE) {
             cp_async<2 * (int)sizeof(T)>(dst, row + c0, pred);
-        } else if constexpr (sizeof(T) >= 4) {
+        } else if constexpr (sizeof(T) == 2) {   // (cp.async copies 4 bytes at least, aligned)
+            cp_async<4>(dst, row + (pa & ~1), pred);
+            cp_async<4>(dst + 4, row + (pb & ~1), pred);
+        } else if (sizeof(S) == 8 && pb == pa + 1 && !(pa & 1)) {   // (3000 x 2000 163.4 -> 157.0; FP32: longer code, 2048^2 58.9 -> 60.5)
+            cp_async<2 * (int)sizeof(T)>(dst, row + pa, pred);
+        } else {
             cp_async<(int)sizeof(T)>(dst, row + pa, pred);
             cp_async<(int)sizeof(T)>(dst + sizeof(T), row + pb, pred);
-        } else {   // 16-bit elements: too small for cp.async, staged through registers
-            T *d = reinterpret_cast<T *>(dst);
-            d[0] = pred ? row[pa] : T(0.f);
-            d[1] = pred ? row[pb] : T(0.f);
+        }
+    };
+    // a pair as put2 left it
+    auto get2 = [&](auto *t, const unsigned char *src, int pa, int pb) {
+        using T = typename std::remove_pointer<decltype(t)>::type;
+        if constexpr (EDGE && sizeof(T) == 2) {
+            const T *d = reinterpret_cast<const T *>(src);
+            return P2<C>{to_c<C>(d[pa & 1]), to_c<C>(d[2 + (pb & 1)])};
+        } else {
+            const typename Vec2<T>::T v = *reinterpret_cast<const typename Vec2<T>::T *>(src);
+            return P2<C>{to_c<C>(v.x), to_c<C>(v.y)};
         }
     };
     auto issue = [&](int j, int st) {
@@ -287,6 +367,16 @@ __device__ void interior_warp(const FusedArgs<S, C> &a, int y0, int seg, int it,
             put2(sslot(st, 8), rowp(a.rin[F_MN], j), pN0, pN1, true);
             put2(sslot(st, 9), rowp(a.rin[F_NM], j), pM0, pM1, true);
             k = 10;
+        }
+        if (EDGE && seam) {
+            const int o = j * pitch + zcol;
+            unsigned char *dst = sslot(st, RL::NS - 1);
+            if constexpr (sizeof(S) >= 4) {
+                cp_async<(int)sizeof(S)>(dst, a.in[F_NN] + o, true);
+            } else {
+                cp_async<4>(dst, a.in[F_NN] + (o & ~1), true);
+                if constexpr (SPLIT) cp_async<4>(dst + 4, a.rin[F_NN] + (o & ~1), true);
+            }
         }
         const int i = j - 2;
         const bool srow = core && i >= x0 && i < x1;
@@ -311,42 +401,47 @@ __device__ void interior_warp(const FusedArgs<S, C> &a, int y0, int seg, int it,
             put2(eslot(st, 4), a.w[F_MM1] + i * pitch, pM0, pM1, srow);
         }
     };
-    auto rdS = [&](int st, int k) {
-        const typename Vec2<S>::T v = *reinterpret_cast<const typename Vec2<S>::T *>(sslot(st, k));
-        return P2<C>{to_c<C>(v.x), to_c<C>(v.y)};
+    // slot k's pair, at N-type (TN) or M-type columns
+    auto rdS = [&](int st, int k, bool TN) {
+        return get2(static_cast<S *>(nullptr), sslot(st, k), TN ? pN0 : pM0, TN ? pN1 : pM1);
     };
-    auto rdC = [&](int st, int k) {
-        const typename Vec2<K>::T v = *reinterpret_cast<const typename Vec2<K>::T *>(cslot(st, k));
-        return P2<C>{to_c<C>(v.x), to_c<C>(v.y)};
+    auto rdC = [&](int st, int k, bool TN) {
+        return get2(static_cast<K *>(nullptr), cslot(st, k), TN ? pN0 : pM0, TN ? pN1 : pM1);
     };
-    auto rdF = [&](int st, int k) {   // a field pair as the stencil reads it
-        P2<C> v = rdS(st, k);
+    auto rdF = [&](int st, int k, bool TN) {   // a field pair as the stencil reads it
+        P2<C> v = rdS(st, k, TN);
         if constexpr (SPLIT) {
-            const P2<C> lo = rdS(st, k + 5);
+            const P2<C> lo = rdS(st, k + 5, TN);
             v.a = add(v.a, lo.a);
             v.b = add(v.b, lo.b);
         }
         return v;
     };
     auto read = [&](int st, int j, Row<C> &in) {
-        in.nn = rdF(st, 0);
-        in.mm0 = rdF(st, 1);
-        in.mm1 = rdF(st, 2);
-        in.vmn = rdF(st, 3);
-        in.vnm = rdF(st, 4);
+        in.nn = rdF(st, 0, true);
+        in.mm0 = rdF(st, 1, false);
+        in.mm1 = rdF(st, 2, false);
+        in.vmn = rdF(st, 3, true);
+        in.vnm = rdF(st, 4, false);
         if constexpr (KR || KC) {
             constexpr int k = SPLIT ? 10 : 5;
-            in.rmn = rdS(st, k + 0);
-            in.rnm = rdS(st, k + 1);
-            in.rnn = rdS(st, k + 2);
-            in.rm0 = rdS(st, k + 3);
-            in.rm1 = rdS(st, k + 4);
+            in.rmn = rdS(st, k + 0, true);
+            in.rnm = rdS(st, k + 1, false);
+            in.rnn = rdS(st, k + 2, true);
+            in.rm0 = rdS(st, k + 3, false);
+            in.rm1 = rdS(st, k + 4, false);
         }
-        in.pmn = rdC(st, 0);
-        in.pnm = rdC(st, 1);
-        in.mu = rdC(st, 2);
-        in.lam = rdC(st, 3);
-        in.m2 = rdC(st, 4);
+        if (EDGE && seam) {
+            const S *d = reinterpret_cast<const S *>(sslot(st, RL::NS - 1));
+            const int h = sizeof(S) == 2 ? zcol & 1 : 0;   // (rows start at even elements)
+            in.z = to_c<C>(d[h]);
+            if constexpr (SPLIT) in.z = add(in.z, to_c<C>(d[2 + h]));
+        }
+        in.pmn = rdC(st, 0, true);
+        in.pnm = rdC(st, 1, false);
+        in.mu = rdC(st, 2, true);
+        in.lam = rdC(st, 3, false);
+        in.m2 = rdC(st, 4, false);
         if constexpr (ENERGY) {
             auto rdE = [&](int k) {
                 const double2 v = *reinterpret_cast<const double2 *>(eslot(st, k));
@@ -388,15 +483,17 @@ __device__ void interior_warp(const FusedArgs<S, C> &a, int y0, int seg, int it,
     // store the owned values of a pair (owned columns are physical: c0 >= 0 for core lanes)
     // the second array holds the residual (R, C codes) or the low part lo = s - hi (split)
     constexpr bool TWO = Cpst<CPST>::any;
+    P2<C> nf{C(0), C(0)};   // stays 0 unless a new value is not finite (v * 0 is NaN for Inf / NaN)
     auto put = [&](int f, int row, const P2<C> &s, const P2<C> &r, const P2<C> &cc, bool o0, bool o1) {
         S *o = a.out[f] + row * pitch;
         S *ro = TWO ? a.rout[f] + row * pitch : nullptr;
-        if ((o0 && !finite(s.a)) || (o1 && !finite(s.b))) atomicOr(a.flags, FLAG_NONFINITE);
-        const S h0 = to_s<S>(s.a), h1 = to_s<S>(s.b);
-        S l0{}, l1{};
-        if constexpr (SPLIT) { l0 = to_s<S>(sub(s.a, to_c<C>(h0))); l1 = to_s<S>(sub(s.b, to_c<C>(h1))); }
-        if constexpr (KR) { l0 = to_s<S>(r.a); l1 = to_s<S>(r.b); }
-        if constexpr (KC) { l0 = to_s<S>(cc.a); l1 = to_s<S>(cc.b); }
+        if (o0) nf = P.nonfinite(s, nf);
+        typename Vec2<S>::T h, lo{};
+        round2(s, h);
+        if constexpr (SPLIT) round2(P.sub(s, {to_c<C>(h.x), to_c<C>(h.y)}), lo);
+        if constexpr (KR) round2(r, lo);
+        if constexpr (KC) round2(cc, lo);
+        const S h0 = h.x, h1 = h.y, l0 = lo.x, l1 = lo.y;
         store_pair<S, EDGE, TWO>(o, ro, c0, c1, h0, h1, l0, l1, o0, o1);
         // a slab linked to its neighbours also stores its rows next to a cut into their halo rows
         // (the same column layout; peer memory on another GPU is written over NVLink)
@@ -424,8 +521,17 @@ __device__ void interior_warp(const FusedArgs<S, C> &a, int y0, int seg, int it,
     auto pair0 = [&](bool keep, const P2<C> &v) { return P2<C>{keep ? v.a : C(0), keep ? v.b : C(0)}; };
     // a new value as storage keeps it (16-bit storage rounds here, before any later use)
     auto q2 = [&](P2<C> &v) {
-        v.a = quant<S, C, CPST>(v.a);
-        v.b = quant<S, C, CPST>(v.b);
+        if constexpr (sizeof(S) < sizeof(C)) {
+            typename Vec2<S>::T h;
+            round2(v, h);
+            const P2<C> hi{to_c<C>(h.x), to_c<C>(h.y)};
+            if constexpr (SPLIT) {
+                round2(P.sub(v, hi), h);
+                v = P.add(hi, {to_c<C>(h.x), to_c<C>(h.y)});
+            } else {
+                v = hi;
+            }
+        }
     };
 
     // windows: NN rows j-2..j+2, MM0 rows j-2..j+1, MM1 rows j-2..j, MN rows j-4..j, NM rows j-3..j
@@ -459,21 +565,13 @@ __device__ void interior_warp(const FusedArgs<S, C> &a, int y0, int seg, int it,
         if (j <= x1) {   // MN: x from NN rows j-1..j+2, y from MM syy row j (row x1 + 1 feeds no stress)
             P2<C> p, n;
             lanes(M1w[2], p, n);
-            const P2<C> vy = dyNfromM(a.op, M1w[2], p, n);
-            P2<C> vx{C(0), C(0)};
-#pragma unroll
-            for (int w = 0; w < 4; w++) {
-                vx.a = add(vx.a, mul(NNw[1 + w].a, a.op.st[w]));
-                vx.b = add(vx.b, mul(NNw[1 + w].b, a.op.st[w]));
-            }
+            const P2<C> vy = dyNfromM<KR>(P, M1w[2], p, n);
+            const P2<C> vx = taps4<KR>(P, NNw[1], NNw[2], NNw[3], NNw[4]);
             P2<C> r = pair0(KR, cur.rmn), cc = pair0(KC, cur.rmn);
-            r.a = add(r.a, mul(vx.a, cur.pmn.a));
-            r.b = add(r.b, mul(vx.b, cur.pmn.b));
-            r.a = add(r.a, mul(vy.a, cur.pmn.a));
-            r.b = add(r.b, mul(vy.b, cur.pmn.b));
+            r = P.add(r, P.mul(vx, cur.pmn));
+            r = P.add(r, P.mul(vy, cur.pmn));
             P2<C> s = cur.vmn;
-            time_update<CPST>(s.a, r.a, cc.a);
-            time_update<CPST>(s.b, r.b, cc.b);
+            pair_update<CPST>(P, s, r, cc);
             src_add(G_MN, j, s, pN0, pN1);
             q2(s);
             MNw[4] = s;
@@ -488,39 +586,20 @@ __device__ void interior_warp(const FusedArgs<S, C> &a, int y0, int seg, int it,
         if (j >= x0 - 1) {   // NM: x from MM sxx rows j-2..j+1, y from NN row j (row x0 - 2 feeds no stress)
             P2<C> p, n;
             lanes(NNw[2], p, n);
-            P2<C> vy = dyMfromN(a.op, NNw[2], p, n);
-            if (seam0 || seam1) {
-                const S *row = rowp(a.in[F_NN], j), *lrow = SPLIT ? rowp(a.rin[F_NN], j) : nullptr;
-                auto nnv = [&](int col) {
-                    C v = to_c<C>(row[col]);
-                    if constexpr (SPLIT) v = add(v, to_c<C>(lrow[col]));
-                    return v;
-                };
-                if (seam0) {
-                    vy.a = C(0);
-#pragma unroll
-                    for (int w = 0; w < 4; w++) vy.a = add(vy.a, mul(nnv(nread(pM0 - 1 + w, My)), a.op.st[w]));
-                }
-                if (seam1) {
-                    vy.b = C(0);
-#pragma unroll
-                    for (int w = 0; w < 4; w++) vy.b = add(vy.b, mul(nnv(nread(pM1 - 1 + w, My)), a.op.st[w]));
-                }
+            P2<C> vy;
+            if constexpr (EDGE) {
+                const P2<C> v = NNw[2];
+                const C pb = z_pb ? cur.z : p.b, va = z_va ? cur.z : v.a, vb = z_vb ? cur.z : v.b, na = z_na ? cur.z : n.a;
+                vy = taps4<KR>(P, P2<C>{pb, va}, P2<C>{va, vb}, P2<C>{v.b, na}, P2<C>{na, n.b});
+            } else {
+                vy = dyMfromN<KR>(P, NNw[2], p, n);
             }
-            P2<C> vx{C(0), C(0)};
-#pragma unroll
-            for (int w = 0; w < 4; w++) {
-                vx.a = add(vx.a, mul(M0w[w].a, a.op.st[w]));
-                vx.b = add(vx.b, mul(M0w[w].b, a.op.st[w]));
-            }
+            const P2<C> vx = taps4<KR>(P, M0w[0], M0w[1], M0w[2], M0w[3]);
             P2<C> r = pair0(KR, cur.rnm), cc = pair0(KC, cur.rnm);
-            r.a = add(r.a, mul(vx.a, cur.pnm.a));
-            r.b = add(r.b, mul(vx.b, cur.pnm.b));
-            r.a = add(r.a, mul(vy.a, cur.pnm.a));
-            r.b = add(r.b, mul(vy.b, cur.pnm.b));
+            r = P.add(r, P.mul(vx, cur.pnm));
+            r = P.add(r, P.mul(vy, cur.pnm));
             P2<C> s = cur.vnm;
-            time_update<CPST>(s.a, r.a, cc.a);
-            time_update<CPST>(s.b, r.b, cc.b);
+            pair_update<CPST>(P, s, r, cc);
             src_add(G_NM, j, s, pM0, pM1);
             q2(s);
             NMw[3] = s;
@@ -537,26 +616,18 @@ __device__ void interior_warp(const FusedArgs<S, C> &a, int y0, int seg, int it,
         if (i >= x0) {
             P2<C> p, n;
             lanes(NMw[1], p, n);
-            const P2<C> vyN = dyNfromM(a.op, NMw[1], p, n);   // NN y from NM row i
+            const P2<C> vyN = dyNfromM<KR>(P, NMw[1], p, n);   // NN y from NM row i
             lanes(MNw[2], p, n);
-            const P2<C> vyM = dyMfromN(a.op, MNw[2], p, n);   // MM y from MN row i
+            const P2<C> vyM = dyMfromN<KR>(P, MNw[2], p, n);   // MM y from MN row i
             if (core) {
                 {   // NN: x from MN rows i-2..i+1
-                    P2<C> vx{C(0), C(0)};
-#pragma unroll
-                    for (int w = 0; w < 4; w++) {
-                        vx.a = add(vx.a, mul(MNw[w].a, a.op.st[w]));
-                        vx.b = add(vx.b, mul(MNw[w].b, a.op.st[w]));
-                    }
+                    const P2<C> vx = taps4<KR>(P, MNw[0], MNw[1], MNw[2], MNw[3]);
                     P2<C> r = pair0(KR, cur.rnn), cc = pair0(KC, cur.rnn);
-                    r.a = add(r.a, mul(vx.a, cur.mu.a));
-                    r.b = add(r.b, mul(vx.b, cur.mu.b));
-                    r.a = add(r.a, mul(vyN.a, cur.mu.a));
-                    r.b = add(r.b, mul(vyN.b, cur.mu.b));
+                    r = P.add(r, P.mul(vx, cur.mu));
+                    r = P.add(r, P.mul(vyN, cur.mu));
                     const P2<C> old = NNw[0];
                     P2<C> s = old;
-                    time_update<CPST>(s.a, r.a, cc.a);
-                    time_update<CPST>(s.b, r.b, cc.b);
+                    pair_update<CPST>(P, s, r, cc);
                     src_add(G_NN, i, s, c0, c1);
                     q2(s);
                     put(F_NN, i, s, r, cc, oN0, oN1);
@@ -572,27 +643,20 @@ __device__ void interior_warp(const FusedArgs<S, C> &a, int y0, int seg, int it,
                     }
                 }
                 {   // MM: x from NM rows i-1..i+2
-                    P2<C> vx{C(0), C(0)};
-#pragma unroll
-                    for (int w = 0; w < 4; w++) {
-                        vx.a = add(vx.a, mul(NMw[w].a, a.op.st[w]));
-                        vx.b = add(vx.b, mul(NMw[w].b, a.op.st[w]));
-                    }
+                    const P2<C> vx = taps4<KR>(P, NMw[0], NMw[1], NMw[2], NMw[3]);
                     P2<C> r0 = pair0(KR, cur.rm0), k0 = pair0(KC, cur.rm0);
                     P2<C> r1 = pair0(KR, cur.rm1), k1 = pair0(KC, cur.rm1);
                     const P2<C> L = cur.lam, M2 = cur.m2;
-                    r0.a = add(r0.a, mul(vx.a, L.a));   r0.b = add(r0.b, mul(vx.b, L.b));
-                    r1.a = add(r1.a, mul(vx.a, L.a));   r1.b = add(r1.b, mul(vx.b, L.b));
-                    r0.a = add(r0.a, mul(vx.a, M2.a));  r0.b = add(r0.b, mul(vx.b, M2.b));
-                    r0.a = add(r0.a, mul(vyM.a, L.a));  r0.b = add(r0.b, mul(vyM.b, L.b));
-                    r1.a = add(r1.a, mul(vyM.a, L.a));  r1.b = add(r1.b, mul(vyM.b, L.b));
-                    r1.a = add(r1.a, mul(vyM.a, M2.a)); r1.b = add(r1.b, mul(vyM.b, M2.b));
+                    r0 = P.add(r0, P.mul(vx, L));
+                    r1 = P.add(r1, P.mul(vx, L));
+                    r0 = P.add(r0, P.mul(vx, M2));
+                    r0 = P.add(r0, P.mul(vyM, L));
+                    r1 = P.add(r1, P.mul(vyM, L));
+                    r1 = P.add(r1, P.mul(vyM, M2));
                     const P2<C> o0 = M0w[0], o1 = M1w[0];
                     P2<C> s0 = o0, s1 = o1;
-                    time_update<CPST>(s0.a, r0.a, k0.a);
-                    time_update<CPST>(s0.b, r0.b, k0.b);
-                    time_update<CPST>(s1.a, r1.a, k1.a);
-                    time_update<CPST>(s1.b, r1.b, k1.b);
+                    pair_update<CPST>(P, s0, r0, k0);
+                    pair_update<CPST>(P, s1, r1, k1);
                     src_add(G_MM, i, s0, c0, c1);
                     src_add(G_MM, i, s1, c0, c1);
                     q2(s0);
@@ -633,6 +697,7 @@ __device__ void interior_warp(const FusedArgs<S, C> &a, int y0, int seg, int it,
         for (int q = 0; q < 3; q++) NMw[q] = NMw[q + 1];
     }
     cp_async_wait_all();
+    if (nf.a + nf.b != C(0)) atomicOr(a.flags, FLAG_NONFINITE);
 }
 
 // ------------------------------------------------------------------------------- boundary CTA
@@ -846,7 +911,7 @@ __global__ void __launch_bounds__(FS_THREADS_MAX, fs_min_blocks<C, ENERGY>()) k_
         if (gw < a.n_int_seg * a.n_wstrip) {
             const int seg = gw / a.n_wstrip, wstrip = gw - seg * a.n_wstrip;
             const int y0 = wstrip * FS_WARP_CORE;
-            unsigned char *ring = smem_raw + (threadIdx.x >> 5) * RingLayout<S, C, CPST, ENERGY, K>::warp;
+            unsigned char *ring = smem_raw + (threadIdx.x >> 5) * RingSize<S, C, CPST, ENERGY, K>::warp;
             if (y0 >= 4 && y0 + 60 <= a.My) interior_warp<S, C, CPST, ENERGY, false, K, MODE == 1>(a, y0, seg, it, rcv_b, rcv_e, E, ring);
             else interior_warp<S, C, CPST, ENERGY, true, K, MODE == 1>(a, y0, seg, it, rcv_b, rcv_e, E, ring);
         }
@@ -891,7 +956,7 @@ template <class S, class C, int CPST, bool ENERGY, class K = C>
 size_t fused_smem_bytes(int tile_rows)
 {
     const size_t tile = sizeof(C) * 2 * (size_t)tile_rows * FS_BND_W;
-    const size_t rings = (size_t)FS_WARPS * RingLayout<S, C, CPST, ENERGY, K>::warp;
+    const size_t rings = (size_t)FS_WARPS * RingSize<S, C, CPST, ENERGY, K>::warp;
     return tile > rings ? tile : rings;
 }
 

@@ -546,7 +546,7 @@ __global__ void __launch_bounds__(FS_THREADS_MAX, fs_min_blocks<float, ENERGY>()
         if (gw < a.n_int_seg * a.n_ostrip) {
             const int seg = gw / a.n_ostrip, os = gw - seg * a.n_ostrip;
             const int y0 = os == 0 ? 0 : a.y_tma_end + (os - 1) * FS_WARP_CORE;
-            unsigned char *ring = side_smem_raw + (threadIdx.x >> 5) * RingLayout<float, float, 0, ENERGY, float>::warp;
+            unsigned char *ring = side_smem_raw + (threadIdx.x >> 5) * RingSize<float, float, 0, ENERGY, float>::warp;
             // (the seam-aware variant for every strip, as in the strips' launch: 1 % faster at 8192^2)
             interior_warp<float, float, 0, ENERGY, true, float, false>(a, y0, seg, it, rcv_b, rcv_e, E, ring);
         }
@@ -571,8 +571,9 @@ __global__ void __launch_bounds__(FS_THREADS_MAX, 4)
     // (both latency-bound: taken first, so that none trails at the end; spread among the TMA
     // items instead, two loops on one SM were far slower), the rest (segment, strip) items of the
     // TMA strips; without, the side launch runs the boundary CTAs and the warp strips
-    static_assert(FS_WARPS * RingLayout<float, float, 0, ENERGY, float>::warp <= TmaLayout<Q16>::o_bar,
-                  "the warp strips' rings lie below the TMA strips' barriers");
+    // (the warp strips' rings lie below the TMA strips' barriers, as many rows deep as fit)
+    constexpr int WD = TmaLayout<Q16>::o_bar / (FS_WARPS * RingLayout<float, float, 0, ENERGY, float, true>::stage);
+    static_assert(WD >= 2, "a warp strip's ring has two rows at least");
     static_assert(sizeof(float) * 2 * TMA_TILE_ROWS * FS_BND_W <= (size_t)TmaLayout<Q16>::o_bar,
                   "the boundary CTAs' tile lies below the TMA strips' barriers");
     const int n_bnd = a.n_zone * a.n_bstrip;
@@ -597,10 +598,10 @@ __global__ void __launch_bounds__(FS_THREADS_MAX, 4)
             if (gw < a.n_int_seg * a.n_ostrip) {
                 const int seg = gw / a.n_ostrip, os = gw - seg * a.n_ostrip;
                 const int y0 = os == 0 ? 0 : a.y_tma_end + (os - 1) * FS_WARP_CORE;
-                unsigned char *ring = base + (threadIdx.x >> 5) * RingLayout<float, float, 0, ENERGY, float>::warp;
+                unsigned char *ring = base + (threadIdx.x >> 5) * (WD * RingLayout<float, float, 0, ENERGY, float, true>::stage);
                 // (the seam-aware variant for every strip: a second, faster variant for the strips
                 // away from the seam made the launch's code larger and the step 4 % slower)
-                interior_warp<float, float, 0, ENERGY, true, float, false>(a, y0, seg, it, rcv_b, rcv_e, E, ring);
+                interior_warp<float, float, 0, ENERGY, true, float, false, WD>(a, y0, seg, it, rcv_b, rcv_e, E, ring);
             }
             __syncthreads();   // every warp is done with its ring before the shared memory is reused
             continue;
