@@ -191,6 +191,7 @@ struct FusedArgs {
     int q16;
     float qlo[5], qstep[5];
     int witems;               // the warp strips run as the first items of the TMA strips' launch
+    int alternate;            // every other step takes the TMA items from the last to the first
 };
 template <class S, class C>
 void launch_fused(const FusedArgs<S, C> &a, int cpst, bool energy, bool coef16, cudaStream_t st);

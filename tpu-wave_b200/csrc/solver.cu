@@ -159,6 +159,7 @@ struct tw_solver {
     // latency-bound items at the head of the queue hold the strips' DRAM stream back), else in the
     // side launch; TW_TMA_WITEMS=1 / 0 selects either for comparisons
     bool tma_witems = false;
+    bool tma_alternate = false;
     int *d_rcv_off_w = nullptr, *d_rcv_list_w = nullptr;
     int rcv_list_cap_w = 0;
     TmaMaps *tmaps = nullptr;
@@ -470,6 +471,7 @@ void enqueue_fused_io(tw_solver *s, void *const *fin, void *const *fout, void *c
             a.dx2 = dx * dx;
             for (int k = 0; k < 3; k++) a.ecoef[k] = s->ecoef[k];
             a.witems = s->tma_witems ? 1 : 0;
+            a.alternate = s->tma_alternate ? 1 : 0;
             for (int k = 0; k < 5; k++) { a.qlo[k] = s->qlo[k]; a.qstep[k] = s->qstep[k]; }
             launch_tma<S, C>(a, s->tmaps[fin == s->f ? 0 : 1], energy, st, s->st_side, s->ev_fork, s->ev_join);
             return;
@@ -1318,6 +1320,11 @@ int create_impl(tw_solver **out, const tw_grid_desc *desc, const SlabSpec &sl)
             s->n_ostrip = 1 + (int)((My + 1 - s->y_tma_end + FS_WARP_CORE - 1) / FS_WARP_CORE);
             // the boundary and warp-strip work in the strips' launch (one launch a step) or beside it
             s->tma_witems = env_int("TW_TMA_WITEMS", (long)Mx * My < (1L << 25) ? 1 : 0) != 0;
+            // every other step takes the TMA items from the last to the first: what the step before read
+            // and wrote last is still in L2. Us a step without / with: 1023 x 2500 48.1 / 45.7, 2048^2 62.8 /
+            // 60.8, with the energy 80.3 / 78.4, 3000^2 110.5 / 109.7; from 4096^2 on L2 holds too little of a
+            // step: 187.9 / 188.4, 8192^2 666 / 676
+            s->tma_alternate = env_int("TW_TMA_ALT", (long)Mx * My < (1L << 24)) != 0;
             // work items of about TW_TMA_SEG_ROWS rows for the persistent TMA CTAs. Measured, us a
             // step at 16 / 20 / 24 / 32 / 40 rows: 2048^2 61.65 / 61.3 / 63.3 / 63.4 / -, 4096^2
             // 195.6 / 188.5 / 184.8 / 186.9 / -, 8192^2 (side launch) - / - / 664.0 / 679.7 / 690.1,
@@ -1331,9 +1338,13 @@ int create_impl(tw_solver **out, const tw_grid_desc *desc, const SlabSpec &sl)
             s->n_tseg = std::max(1, std::min(max_seg, (s->int_rows + seg_rows / 2) / seg_rows));
             (void)n_sm;
             // the warp strips run beside the TMA strips, latency-bound at about two microseconds a
-            // row: short segments (TW_TMA_SIDE_ROWS rows, default 8) keep them shorter than a TMA CTA
-            const int side_rows = std::max(8, env_int("TW_TMA_SIDE_ROWS", 8));
-            s->n_int_seg = std::max(1, std::min(max_seg, s->int_rows / side_rows));
+            // row: short segments (TW_TMA_SIDE_ROWS rows) keep them shorter than a TMA CTA. Below 2^22
+            // points the longest of them is the step's end: us a step at 4 / 5 / 6 / 8 rows, 1200 x 1500 33.2 /
+            // 33.4 / 33.1 / 37.1, 1500^2 37.1 / 36.7 / 37.3 / 39.3 (with the energy 48.7 / 48.0 / 48.0 / 51.7),
+            // 1900^2 54.6 / 53.9 / 53.4 / 54.4; from there on their halo rows cost more: 2048^2 62.4 /
+            // 62.0 / 61.2 / 60.4
+            const int side_rows = std::max(4, env_int("TW_TMA_SIDE_ROWS", (long)Mx * My < (1L << 22) ? 6 : 8));
+            s->n_int_seg = std::max(1, s->int_rows / side_rows);
             s->n_int_cta = (s->n_int_seg * s->n_ostrip + FS_WARPS - 1) / FS_WARPS;
             s->n_tcta = s->n_tseg * s->n_tstrip;
             e = prepare_tma<float, float>();

@@ -607,7 +607,9 @@ __global__ void __launch_bounds__(FS_THREADS_MAX, 4)
             continue;
           }
         }
-        const int tt = t - B - W;
+        // (every other step from the last item to the first: what the step before read and wrote last is
+        // still in L2)
+        const int tt = a.alternate & it & 1 ? a.n_tcta - 1 - (t - B - W) : t - B - W;
         const int rcv_b = a.rcv_off[n_side + tt], rcv_e = a.rcv_off[n_side + tt + 1];
         if (!tma_strip_cta<ENERGY, Q16>(a, maps, tt % a.n_tstrip, tt / a.n_tstrip, it, rcv_b, rcv_e, E, base)) break;
     }
