@@ -45,7 +45,9 @@ enum {
     TW_ERR_MODEL_BOUNDS = -11,  /* interpolation stepped out of the model (grid_parameter.cpp:54-56) */
     TW_ERR_TOO_LARGE = -12,     /* model larger than the no-allocation scratch (TW_NOALLOC_MAX_MODEL_POINTS) */
     TW_ERR_IO = -13,            /* a file could not be opened, read or written, or is malformed */
-    TW_ERR_TIMEOUT = -14        /* a wait inside a step kernel gave up (a staged copy did not arrive) */
+    TW_ERR_TIMEOUT = -14        /* a wait inside a step kernel gave up: a staged copy, or a value from the
+                                   neighbouring tile of an on-chip run, did not arrive (tw_sync and the
+                                   gradients report it; the state is then incomplete until tw_reset) */
 };
 
 /* ---- enums ------------------------------------------------------------------------------ */
@@ -292,6 +294,8 @@ TW_API int tw_slab_run(tw_solver *const *slabs, int n, int steps);
  *   g_rho/vp/vs   dJ/d(padded node model of tw_set_material_model), its layout ((Mx_prmt+2) x
  *                 (My_prmt+2)); TW_ERR_STATE when the material came from tw_set_material_grid;
  *   g_state[5]    dJ/d(initial fields NN, MN, NM, MM0, MM1) at reference sizes.
+ * A wait that gave up on the way is TW_ERR_TIMEOUT, and no output is written; values that are not
+ * finite stay in the gradient and are reported by the next tw_sync.
  * Afterwards the handle holds the state and records of tw_step(nt). Device memory for the call:
  * (nt/ckpt_every + ckpt_every + 2) states plus 15 field-sized arrays. */
 TW_API int tw_adjoint_gradient(tw_solver *s, int nt, const double *obs, int ckpt_every, double *misfit,

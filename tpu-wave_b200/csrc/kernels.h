@@ -231,6 +231,7 @@ constexpr int RES_W = 58;             // most columns of a tile (column My inclu
 constexpr int RES_P = 68;             // values of a shared row (FP32 rows of 5 fields 1360 bytes apart: 13 or
                                       // 14 vectors a row, two or three rows a warp, few bank conflicts)
 constexpr int RES_MIN = 8;            // least rows / columns of a tile: halos and closures meet one neighbour
+constexpr int RES_POLLS = 1 << 20;    // polls of an exchange word before a CTA gives up (about a second)
 template <class C>
 struct ResArgs {
     const C *in[5];           // state before the run
@@ -247,6 +248,7 @@ struct ResArgs {
     int ntx, nty;             // tiles along x and y
     int rows_s;               // rows of a tile's shared memory
     int n;                    // steps of this run
+    int polls;                // polls of an exchange word before a CTA gives up (0: at once)
     unsigned tag0;            // steps the handle has run this way before: tags of the exchange words
     unsigned long long *xbuf; // exchange words: [2][NN, MM0, MM1 (acoustic: MM0)][(Mx + 1) x xcols], FP64 two
                               // words a value

@@ -141,7 +141,6 @@ __device__ __forceinline__ u64 xld(const u64 *p)
     asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
     return v;
 }
-constexpr int X_POLLS = 1 << 20;   // polls before a CTA gives up (about a second)
 // one exchanged value: loaded, and whether it is the step's
 template <class C> struct XV;
 template <> struct XV<float> {
@@ -700,7 +699,7 @@ __device__ __forceinline__ void resident_run(const ResArgs<C> &a, int blk, int n
                 if (!ok || xs[b] < 0) break;
                 XV<C> v[B][3];
                 ok = false;
-                for (int n = 0; n < X_POLLS && !ok; n++) {
+                for (int n = 0; n < a.polls && !ok; n++) {
 #pragma unroll
                     for (int m = 0; m < B; m++) {
                         if (xs[b + m] >= 0) v[m][0].load(xb + xg[b + m]);

@@ -130,6 +130,7 @@ struct tw_solver {
     // a run of a handle with one buffer ends where it began: a tile is stored after its neighbours have
     // sent words of their first step, so after they have loaded it (runs of two steps or more)
     bool res_in_place = false;
+    int res_polls = RES_POLLS;
     unsigned res_tag = 0;             // steps run this way since the exchange words were cleared
     unsigned long long *xbuf = nullptr;
     size_t xbuf_bytes = 0;
@@ -630,6 +631,7 @@ ResArgs<C> resident_args(const tw_solver *s, const ResPlan &p, int n, const int 
     a.nty = p.nty;
     a.rows_s = p.rows_s;
     a.n = n;
+    a.polls = s->res_polls;
     a.tag0 = s->res_tag;
     a.xbuf = s->xbuf;
     a.xcols = (int)(s->d.My + 2) & ~1;   // (even: pairs of words are written whole)
@@ -1119,7 +1121,7 @@ const char *tw_strerror(int status)
     case TW_ERR_MODEL_BOUNDS: return "material interpolation outside the model";
     case TW_ERR_TOO_LARGE: return "model larger than the no-allocation scratch (TW_NOALLOC_MAX_MODEL_POINTS)";
     case TW_ERR_IO: return "file missing, unreadable, unwritable or malformed";
-    case TW_ERR_TIMEOUT: return "a wait inside a step kernel gave up (a staged copy did not arrive)";
+    case TW_ERR_TIMEOUT: return "a wait inside a step kernel gave up";
     }
     return "unknown status";
 }
@@ -1423,7 +1425,8 @@ int create_impl(tw_solver **out, const tw_grid_desc *desc, const SlabSpec &sl)
     }
     // on-chip runs: FP32 / FP64 storage and coefficients, the reference's boundaries, a handle of its
     // own (not a slab), a grid that fits on the SMs. TW_TMA / TW_RESIDENT=0 select the other
-    // kernels for comparisons, TW_RES_NTX / TW_RES_NTY a tiling.
+    // kernels for comparisons, TW_RES_NTX / TW_RES_NTY a tiling, TW_RES_POLLS how often a CTA polls for its
+    // neighbours' words (0: every exchange times out).
     // (acoustic: energy off)
     if ((s->fused || (!s->elastic && !d.energy)) && !s->slab && !s->bnd && !d.coef_fp16 && (d.precision == TW_FP64 || d.precision == TW_FP32) &&
         !std::getenv("TW_TMA") && env_int("TW_RESIDENT", 1) != 0) {
@@ -1454,6 +1457,7 @@ int create_impl(tw_solver **out, const tw_grid_desc *desc, const SlabSpec &sl)
                 cudaMemsetAsync(s->d_done, 0, sizeof(int), s->st);
             }
             s->res_in_place = !s->f2[F_MM0];
+            s->res_polls = std::max(0, env_int("TW_RES_POLLS", RES_POLLS));
             s->res_plan = p;
         }
     }
@@ -2526,11 +2530,16 @@ int adjoint_t(tw_solver *s, int nt, const double *obs, int K, int slots, double 
         }
         s->steps_done += nt;
     }
-    if (misfit) *misfit = J;
     // leave the handle as tw_step(nt) would: the final state, the step counter at nt
     if ((rc = copy_state(s, cur().data(), fin.data())) != TW_OK) return rc;
     TW_CUDA(cudaMemcpyAsync(s->d_step, &nt, sizeof(int), cudaMemcpyHostToDevice, s->st));
+    // a step that gave up waiting has left states unwritten: no gradient (values that are not finite show in
+    // it, and the next tw_sync reports them)
+    int flags = 0;
+    TW_CUDA(cudaMemcpyAsync(&flags, s->d_flags, sizeof(int), cudaMemcpyDeviceToHost, s->st));
     TW_CUDA(cudaStreamSynchronize(s->st));
+    if (flags & FLAG_TIMEOUT) return s->sticky = TW_ERR_TIMEOUT;
+    if (misfit) *misfit = J;
 
     // gradients with respect to the material on each grid: mu, rho (through 1/rho), lambda, 2mu
     for (int k = 0; k < 5; k++) {
