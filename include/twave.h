@@ -134,8 +134,9 @@ TW_API void tw_destroy(tw_solver *s);
 /* Device memory of destroyed handles. A handle takes its buffers from a per-device memory pool
  * (stream-ordered) and tw_destroy returns them to it; the pool keeps them, so that creating the
  * next handle of a similar size maps no new memory (the reference allocates and frees per run,
- * grid.cuh:216-375 and cuda_container_run_time.cuh:268-275). This call gives the memory the
- * pool keeps on `device` back to the driver. No counterpart in the reference. */
+ * grid.cuh:216-375 and cuda_container_run_time.cuh:268-275). The gradients keep up to 4 GiB of their
+ * checkpoints' memory from call to call in a pool of their own. This call gives the memory
+ * both pools keep on `device` back to the driver. No counterpart in the reference. */
 TW_API int tw_release_cached_memory(int device);
 
 /* Material from the reference's padded node model: Class_Grid::retrieve_forward_parameter,
@@ -297,7 +298,8 @@ TW_API int tw_slab_run(tw_solver *const *slabs, int n, int steps);
  * A wait that gave up on the way is TW_ERR_TIMEOUT, and no output is written; values that are not
  * finite stay in the gradient and are reported by the next tw_sync.
  * Afterwards the handle holds the state and records of tw_step(nt). Device memory for the call:
- * (nt/ckpt_every + ckpt_every + 2) states plus 15 field-sized arrays. */
+ * (nt/ckpt_every, rounded up, + ckpt_every + 2) states plus 15 field-sized arrays; up to 4 GiB of it stay
+ * with the library for the next gradient (tw_release_cached_memory). */
 TW_API int tw_adjoint_gradient(tw_solver *s, int nt, const double *obs, int ckpt_every, double *misfit,
                                double *const *g_grid, double *g_rho, double *g_vp, double *g_vs,
                                double *const *g_state);

@@ -29,3 +29,25 @@ def test_a_gradient_whose_exchanges_give_up_is_an_error(tw, monkeypatch):
     s = solver(tw, case, precision="f32")
     assert np.isfinite(s.adjoint_gradient(12, obs, ckpt_every=5)["misfit"])
     s.close()
+
+
+def test_a_gradient_keeps_a_bounded_amount_of_memory(tw):
+    """A gradient whose checkpoints take 5 GB leaves at most 4 GiB with the library, all of it on request."""
+    import torch
+    M, nt = 2048, 60
+    s = tw.Solver(M, M, 1, 500, 1e-4, precision="f32", max_steps=nt, energy=False)
+    model = [np.full((M + 2, M + 2), v) for v in (2.0, 3.0, 1.7)]
+    s.set_material_model(*model)
+    s.set_source(tw.MM, M // 2, M // 2)
+    s.add_receivers(tw.NM, [M // 2], [M // 2 + 4])
+    obs = np.zeros((1, 2, nt))
+    s.adjoint_gradient(2, np.zeros((1, 2, 2)), ckpt_every=1, model=False)   # (kernels loaded, host buffers made)
+    s.reset()
+    tw.release_cached_memory()
+    before = torch.cuda.mem_get_info()[0]
+    assert s.adjoint_gradient(nt, obs, ckpt_every=nt, model=False)["misfit"] > 0
+    slack = 256 << 20
+    assert before - torch.cuda.mem_get_info()[0] <= (4 << 30) + slack
+    tw.release_cached_memory()
+    assert before - torch.cuda.mem_get_info()[0] <= slack
+    s.close()

@@ -61,20 +61,26 @@ bool location_to_index(char type, long num, long den, int num_dx, int den_dx, lo
     return true;
 }
 
-// One memory pool per device for the handles' buffers. A destroyed handle returns its buffers
+// Memory pools per device. POOL_HANDLES: the handles' buffers. A destroyed handle returns its buffers
 // to the pool, which keeps them (release threshold: everything), so that the next handle of a
 // similar size - the next shot of an inversion, the next call of a caller that creates a handle
-// per simulation - maps no new device memory. tw_release_cached_memory gives it back.
+// per simulation - maps no new device memory. POOL_ARENAS: the memory of one gradient call, mostly
+// checkpoints, of which the pool keeps ARENA_KEEP between calls (the gradients of grids up to
+// 1024^2 with segments of 50 steps take 1.4 GB in FP32, 2.8 GB in FP64) and gives back what is above
+// when the call ends. tw_release_cached_memory gives back what either keeps.
 constexpr int MAX_DEVICES = 64;
+enum { POOL_HANDLES = 0, POOL_ARENAS = 1 };
+constexpr unsigned long long ARENA_KEEP = 4ull << 30;
 std::mutex g_pool_mu;
-cudaMemPool_t g_pool[MAX_DEVICES] = {};
+cudaMemPool_t g_pool[2][MAX_DEVICES] = {};
 
-cudaMemPool_t handle_pool(int device, cudaError_t *err)
+cudaMemPool_t device_pool(int device, int kind, cudaError_t *err)
 {
     *err = cudaSuccess;
     if (device < 0 || device >= MAX_DEVICES) { *err = cudaErrorInvalidDevice; return nullptr; }
     std::lock_guard<std::mutex> lk(g_pool_mu);
-    if (!g_pool[device]) {
+    cudaMemPool_t &pool = g_pool[kind][device];
+    if (!pool) {
         cudaMemPoolProps props{};
         props.allocType = cudaMemAllocationTypePinned;
         props.handleTypes = cudaMemHandleTypeNone;
@@ -82,15 +88,17 @@ cudaMemPool_t handle_pool(int device, cudaError_t *err)
         props.location.id = device;
         cudaMemPool_t p = nullptr;
         if ((*err = cudaMemPoolCreate(&p, &props)) != cudaSuccess) return nullptr;
-        unsigned long long keep = ~0ull;   // cuuint64_t
+        unsigned long long keep = kind == POOL_ARENAS ? ARENA_KEEP : ~0ull;   // cuuint64_t
         if ((*err = cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess) {
             cudaMemPoolDestroy(p);
             return nullptr;
         }
-        g_pool[device] = p;
+        pool = p;
     }
-    return g_pool[device];
+    return pool;
 }
+
+cudaMemPool_t handle_pool(int device, cudaError_t *err) { return device_pool(device, POOL_HANDLES, err); }
 
 // let device `peer` read and write the handle buffers of device `owner` (peer stores of the
 // linked slab step, peer copies of the slab exchange)
@@ -1489,15 +1497,16 @@ void tw_destroy(tw_solver *s)
 int tw_release_cached_memory(int device)
 {
     if (device < 0 || device >= MAX_DEVICES) return TW_ERR_INVALID;
-    cudaMemPool_t p;
+    cudaMemPool_t pools[2];
     {
         std::lock_guard<std::mutex> lk(g_pool_mu);
-        p = g_pool[device];
+        for (int k = 0; k < 2; k++) pools[k] = g_pool[k][device];
     }
-    if (!p) return TW_OK;
+    if (!pools[0] && !pools[1]) return TW_OK;
     TW_CUDA(cudaSetDevice(device));
     TW_CUDA(cudaDeviceSynchronize());   // frees still queued on a stream complete first
-    TW_CUDA(cudaMemPoolTrimTo(p, 0));
+    for (cudaMemPool_t p : pools)
+        if (p) TW_CUDA(cudaMemPoolTrimTo(p, 0));
     return TW_OK;
 }
 
@@ -2197,8 +2206,8 @@ struct DevBuf {
     DevBuf(cudaStream_t s, int d) : st(s), device(d) {}
     ~DevBuf()
     {
-        if (base) cudaFreeAsync(base, st);   // (back to the pool: the next gradient maps no memory)
-        cudaStreamSynchronize(st);
+        if (base) cudaFreeAsync(base, st);   // (back to the pool: the next gradient of this size maps no memory)
+        cudaStreamSynchronize(st);           // (and here the pool gives back what it does not keep)
     }
     int get(void **out, size_t bytes)
     {
@@ -2216,7 +2225,7 @@ struct DevBuf {
     int commit()   // allocate and zero the arena, then hand out pieces in the same order
     {
         cudaError_t e = cudaSuccess;
-        const cudaMemPool_t pool = handle_pool(device, &e);
+        const cudaMemPool_t pool = device_pool(device, POOL_ARENAS, &e);
         if (e == cudaSuccess) e = cudaMallocFromPoolAsync((void **)&base, size, pool, st);
         if (e != cudaSuccess) base = nullptr;
         if (e != cudaSuccess) return e == cudaErrorMemoryAllocation ? TW_ERR_NOMEM : cuda_fail(e, "tw_adjoint_gradient");
