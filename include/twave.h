@@ -298,7 +298,7 @@ TW_API int tw_slab_run(tw_solver *const *slabs, int n, int steps);
  * A wait that gave up on the way is TW_ERR_TIMEOUT, and no output is written; values that are not
  * finite stay in the gradient and are reported by the next tw_sync.
  * Afterwards the handle holds the state and records of tw_step(nt). Device memory for the call:
- * (nt/ckpt_every, rounded up, + ckpt_every + 2) states plus 15 field-sized arrays; up to 4 GiB of it stay
+ * (nt/ckpt_every, rounded up, + ckpt_every + 1) states plus 15 field-sized arrays; up to 4 GiB of it stay
  * with the library for the next gradient (tw_release_cached_memory). */
 TW_API int tw_adjoint_gradient(tw_solver *s, int nt, const double *obs, int ckpt_every, double *misfit,
                                double *const *g_grid, double *g_rho, double *g_vp, double *g_vs,

@@ -2393,8 +2393,8 @@ long revolve_check(const std::vector<RvAction> &acts, int nt, int slots)
     return (fin && next_adj == -1) ? fwd : -1;
 }
 
-// the gradient call. K > 0: checkpoints every K steps, each segment recomputed into a buffer of
-// K + 1 states; K == 0: binomial checkpointing in `slots` state slots
+// the gradient call. K > 0: checkpoints every K steps, each segment recomputed from its checkpoint into a
+// buffer of K states; K == 0: binomial checkpointing in `slots` state slots
 template <class C>
 int adjoint_t(tw_solver *s, int nt, const double *obs, int K, int slots, double *misfit, double *const *g_grid,
               double *g_rho, double *g_vp, double *g_vs, double *const *g_state)
@@ -2408,7 +2408,7 @@ int adjoint_t(tw_solver *s, int nt, const double *obs, int K, int slots, double 
     int rc;
     // periodic: checkpoints every K steps and the states of one segment; revolve: the slots, two
     // states of the plan and two scratch states for multi-step advances; both: the final state
-    std::vector<std::array<void *, 5>> ck(periodic ? n_ck : slots + 2), seg(periodic ? K + 1 : 2);
+    std::vector<std::array<void *, 5>> ck(periodic ? n_ck : slots + 2), seg(periodic ? K : 2);   // (seg[k]: the state k + 1 steps after the checkpoint)
     std::array<void *, 5> fin{};
     AdjArgs<C> a{};
     double *d_res = nullptr, *gq[5] = {}, *nd = nullptr;
@@ -2500,13 +2500,13 @@ int adjoint_t(tw_solver *s, int nt, const double *obs, int K, int slots, double 
             const int k0 = c * K, k1 = std::min(nt, k0 + K);
             TW_CUDA(cudaMemcpyAsync(s->d_step, &k0, sizeof(int), cudaMemcpyHostToDevice, s->st));
             if (s->res_plan.ntx > 0) {   // on chip, every state written out (1024^2 FP32: 38 -> 21 us a step)
-                const long stride = K > 1 ? (long)((char *)seg[2][0] - (char *)seg[1][0]) / (long)sizeof(C) : 0;
-                if ((rc = run_resident<C>(s, k1 - k0, s->st, ck[c].data(), seg[1].data(), seg[k1 - k0].data(), stride)) != TW_OK) return rc;
+                const long stride = K > 1 ? (long)((char *)seg[1][0] - (char *)seg[0][0]) / (long)sizeof(C) : 0;
+                if ((rc = run_resident<C>(s, k1 - k0, s->st, ck[c].data(), seg[0].data(), seg[k1 - k0 - 1].data(), stride)) != TW_OK) return rc;
             } else {
-                for (int k = k0; k < k1; k++)   // step k: segment state k - k0 -> k - k0 + 1 (recomputed: no energy)
-                    enqueue_fused_io<C, C>(s, k == k0 ? ck[c].data() : seg[k - k0].data(), seg[k - k0 + 1].data(), none, none, s->st, false);
+                for (int k = k0; k < k1; k++)   // (recomputed: no energy)
+                    enqueue_fused_io<C, C>(s, k == k0 ? ck[c].data() : seg[k - k0 - 1].data(), seg[k - k0].data(), none, none, s->st, false);
             }
-            for (int n = k1 - 1; n >= k0; n--) adjoint_step(n, n == k0 ? ck[c].data() : seg[n - k0].data(), seg[n + 1 - k0].data());
+            for (int n = k1 - 1; n >= k0; n--) adjoint_step(n, n == k0 ? ck[c].data() : seg[n - k0 - 1].data(), seg[n - k0].data());
             TW_CUDA(cudaGetLastError());
         }
     } else {
