@@ -331,10 +331,10 @@ TW_API int tw_data_misfit(tw_solver *s, const double *obs, double *total, double
  * small shots no longer pay a launch per half-step each; G steps are replayed from a CUDA graph.
  * Each shot equals the same handle stepped alone with tw_step, bit for bit.
  * Requirements: acoustic handles on one device with the same precision (FP64/FP32),
- * compensation ('0', '3R', '6R') and x boundary, energy off, material set. The batch copies each
- * shot's set-up (source, receivers, buffers) at tw_batch_create: re-create it after changing a
- * shot's source or receivers. Shots stay usable on their own (readback, tw_step); tw_batch_step
- * orders itself after the shots' queued work and their later work after the batch. */
+ * compensation ('0', '3R', '6R') and x boundary, energy off, material set. A source or receivers
+ * that a shot gets later are those of the next tw_batch_step. Shots stay usable on their own
+ * (readback, tw_step); tw_batch_step orders itself after the shots' queued work and their later
+ * work after the batch. */
 typedef struct tw_batch tw_batch;
 TW_API int tw_batch_create(tw_batch **out, tw_solver *const *shots, int n);
 TW_API void tw_batch_destroy(tw_batch *b);

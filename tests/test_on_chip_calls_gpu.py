@@ -51,3 +51,63 @@ def test_a_gradient_keeps_a_bounded_amount_of_memory(tw):
     tw.release_cached_memory()
     assert before - torch.cuda.mem_get_info()[0] <= slack
     s.close()
+
+
+def acoustic(tw, Mx, My, bc, k=0, max_steps=64, precision="f32", cpst="00"):
+    """A shot with random medium and fields, a source and a few receivers."""
+    s = tw.Solver(Mx, My, 1, max(Mx, My), 1e-4, physics=tw.ACOUSTIC, bc_x=tw.PERIODIC if bc == "periodic" else tw.SAT_FREE,
+                  precision=precision, cpst=cpst, max_steps=max_steps, energy=False)
+    rng = np.random.default_rng(k)
+    for g in (tw.NM, tw.MN, tw.MM):
+        s.set_material_grid(g, 0, rng.uniform(1, 2, s.shape(g)))
+        s.write_field(g, 0, rng.standard_normal(s.shape(g)))
+    s.set_source(tw.MM, Mx // 2, My // 2)
+    s.add_receivers(tw.MM, [0, Mx // 2, Mx - 1], [My - 1, My // 2, 0])
+    s.add_receivers(tw.NM, [Mx - 1], [1])
+    return s
+
+
+def result(tw, s):
+    return [s.read_field(g) for g in (tw.MN, tw.NM, tw.MM)] + [s.read_receivers()]
+
+
+def same(a, b):
+    return all(np.array_equal(p, q) for x, y in zip(a, b) for p, q in zip(x, y))
+
+
+@pytest.mark.parametrize("resident", [True, False])
+@pytest.mark.parametrize("bc", ["periodic", "free"])
+def test_a_batch_takes_up_receivers_and_sources_set_later(tw, bc, resident, monkeypatch):
+    """Receivers added between two batch steps (more than the shot's trace buffer held, which moves) and a
+    source set anew give what the shots stepped alone give."""
+    monkeypatch.setenv("TW_RESIDENT", "1" if resident else "0")
+    sizes = [(60, 75), (130, 41)]
+
+    def run(batched):
+        shots = [acoustic(tw, Mx, My, bc, k) for k, (Mx, My) in enumerate(sizes)]
+        b = tw.Batch(shots) if batched else None
+
+        def step(n):
+            if b:
+                b.step(n)
+            for s in shots if not b else []:
+                s.step(n)
+
+        step(10)
+        shots[0].add_receivers(tw.MM, np.arange(40), np.arange(40))
+        shots[1].add_receivers(tw.MN, [3], [4])
+        step(17)
+        shots[1].set_source(tw.MN, 7, 9)
+        shots[0].clear_source()
+        step(18)
+        step(1)
+        for h in [b] if b else shots:
+            h.sync()
+        out = [result(tw, s) for s in shots]
+        for h in ([b] if b else []) + shots:
+            h.close()
+        return out
+
+    got, want = run(True), run(False)
+    assert np.abs(want[0][3][4:, 0, 10:]).max() > 0 and not want[0][3][4:, 0, :10].any()
+    assert same(got, want)

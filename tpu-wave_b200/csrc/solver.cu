@@ -203,6 +203,7 @@ struct tw_solver {
     double *d_traces = nullptr, *d_energy = nullptr;
     int rcv_cap = 0;
     std::vector<int> rcv_tab;         // n x 4 (slot0, slot1, row, col)
+    int setup_gen = 0;                // counts changes of the source and the receivers (a batch copies them)
     int src_grid = -1;
     long src_ix = 0, src_iy = 0;
     int steps_done = 0;
@@ -774,6 +775,7 @@ int finalize_material(tw_solver *s)
 
 int rebuild_source_table(tw_solver *s)
 {
+    s->setup_gen++;
     std::vector<double> inc(s->d.max_steps, 0.0);
     if (s->src_grid >= 0) {
         const double dt = s->d.dt, dx = (double)s->d.num_dx / (double)s->d.den_dx;
@@ -795,6 +797,7 @@ int rebuild_source_table(tw_solver *s)
 
 int upload_receivers(tw_solver *s)
 {
+    s->setup_gen++;
     const int n = (int)(s->rcv_tab.size() / 4);
     if (n > s->rcv_cap) {
         s->release(s->d_rcv);
@@ -2669,6 +2672,8 @@ struct tw_batch {
     std::vector<int> rcv_off_at, rcv_at;   // where each shot's lists begin in d_rcv_res
     void *d_res = nullptr;            // arguments by position
     int *d_first = nullptr, *d_rcv_res = nullptr;   // CTA offsets (n + 1 per group), receiver lists
+    size_t rcv_res_cap = 0;
+    std::vector<int> gens;            // each shot's setup_gen the layouts were made for
     cudaStream_t st = nullptr;
     cudaEvent_t done = nullptr;
     void *d_shots = nullptr, *d_gather = nullptr;
@@ -2795,6 +2800,34 @@ int batch_layout(tw_batch *b, const BatchShape &shape)
     return b->precision == TW_FP64 ? batch_layout_t<double, double>(b, shape) : batch_layout_t<float, float>(b, shape);
 }
 
+// the receiver lists of the shots on chip
+int batch_resident_receivers(tw_batch *b)
+{
+    std::vector<int> lists;
+    b->rcv_off_at.clear();
+    b->rcv_at.clear();
+    for (size_t i = 0; i < b->order.size(); i++) {
+        std::vector<int> off, list;
+        resident_receivers(b->shots[b->order[i]], b->plans[i], off, list);
+        b->rcv_off_at.push_back((int)lists.size());
+        lists.insert(lists.end(), off.begin(), off.end());
+        while (lists.size() % 4) lists.push_back(0);
+        b->rcv_at.push_back((int)lists.size());
+        lists.insert(lists.end(), list.begin(), list.end());
+    }
+    lists.push_back(0);
+    if (lists.size() > b->rcv_res_cap) {
+        cudaFree(b->d_rcv_res);
+        b->d_rcv_res = nullptr;
+        b->rcv_res_cap = 0;
+        TW_CUDA(cudaMalloc((void **)&b->d_rcv_res, sizeof(int) * lists.size()));
+        b->rcv_res_cap = lists.size();
+    }
+    TW_CUDA(cudaMemcpyAsync(b->d_rcv_res, lists.data(), sizeof(int) * lists.size(), cudaMemcpyHostToDevice, b->st));
+    TW_CUDA(cudaStreamSynchronize(b->st));
+    return TW_OK;
+}
+
 // plans, groups and receiver lists of a batch whose shots all fit on the chip (resident stays false
 // where one does not: the fused or per-point kernels then step every shot)
 template <class C>
@@ -2829,7 +2862,7 @@ int batch_resident_layout_t(tw_batch *b)
         groups[g].push_back(k);
         used[g] += ctas(k);
     }
-    std::vector<int> first, lists;
+    std::vector<int> first;
     for (size_t g = 0; g < groups.size(); g++) {
         tw_batch::Group G{(int)b->order.size(), (int)groups[g].size(), 0, 0, plans[groups[g][0]].cs};
         for (int k : groups[g]) {
@@ -2848,27 +2881,19 @@ int batch_resident_layout_t(tw_batch *b)
             G.smem = std::max(G.smem, plans[k].smem);
             b->order.push_back(k);
             b->plans.push_back(plans[k]);
-            std::vector<int> off, list;
-            resident_receivers(s, plans[k], off, list);
-            b->rcv_off_at.push_back((int)lists.size());
-            lists.insert(lists.end(), off.begin(), off.end());
-            while (lists.size() % 4) lists.push_back(0);
-            b->rcv_at.push_back((int)lists.size());
-            lists.insert(lists.end(), list.begin(), list.end());
         }
         first.push_back(G.ctas);
         b->groups.push_back(G);
     }
-    lists.push_back(0);
     for (const auto &g : b->groups)
         TW_CUDA(b->periodic ? (prepare_resident_shots<C, RES_AC_PER>(b->cpst, g.cs, smem_max))
                             : (prepare_resident_shots<C, RES_AC_FREE>(b->cpst, g.cs, smem_max)));
     TW_CUDA(cudaMalloc(&b->d_res, sizeof(ResArgs<C>) * n));
     TW_CUDA(cudaMalloc((void **)&b->d_first, sizeof(int) * first.size()));
-    TW_CUDA(cudaMalloc((void **)&b->d_rcv_res, sizeof(int) * lists.size()));
     TW_CUDA(cudaMemcpyAsync(b->d_first, first.data(), sizeof(int) * first.size(), cudaMemcpyHostToDevice, b->st));
-    TW_CUDA(cudaMemcpyAsync(b->d_rcv_res, lists.data(), sizeof(int) * lists.size(), cudaMemcpyHostToDevice, b->st));
     TW_CUDA(cudaStreamSynchronize(b->st));
+    const int rc = batch_resident_receivers(b);
+    if (rc != TW_OK) return rc;
     for (tw_solver *s : b->shots) TW_CUDA(cudaStreamSynchronize(s->st));
     b->resident = true;
     return TW_OK;
@@ -2902,6 +2927,18 @@ int run_batch_resident_t(tw_batch *b, int n)
 int run_batch_resident(tw_batch *b, int n)
 {
     return b->precision == TW_FP64 ? run_batch_resident_t<double>(b, n) : run_batch_resident_t<float>(b, n);
+}
+
+// the shots' sources and receivers as they are now (the fused kernels' arguments are made anew on every call)
+int batch_refresh(tw_batch *b)
+{
+    std::vector<int> now;
+    for (const tw_solver *s : b->shots) now.push_back(s->setup_gen);
+    if (now == b->gens) return TW_OK;
+    int rc = b->fused ? TW_OK : batch_layout(b, b->shape);
+    if (rc == TW_OK && b->resident) rc = batch_resident_receivers(b);
+    if (rc == TW_OK) b->gens = now;
+    return rc;
 }
 
 template <class S, class C>
@@ -2974,6 +3011,7 @@ int tw_batch_create(tw_batch **out, tw_solver *const *shots, int n)
     int rc = b->fused ? batch_fused_layout(b, TW_AC_CTAS_PER_SM) : batch_layout(b, BatchShape{32, 8, 1, 0});
     if (rc == TW_OK) rc = b->precision == TW_FP64 ? batch_resident_layout_t<double>(b) : batch_resident_layout_t<float>(b);
     if (rc != TW_OK) return fail(rc);
+    for (const tw_solver *s : b->shots) b->gens.push_back(s->setup_gen);
     *out = b;
     return TW_OK;
 }
@@ -3025,6 +3063,8 @@ int tw_batch_tune(tw_batch *b, int steps, double *best_ms)
         if (steps + 3 > s->d.max_steps) steps = s->d.max_steps - 3;
     }
     if (steps < 1) return TW_ERR_RECORD_FULL;
+    int rc = batch_refresh(b);
+    if (rc != TW_OK) return rc;
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
     std::vector<BatchShape> cand;
@@ -3040,7 +3080,6 @@ int tw_batch_tune(tw_batch *b, int steps, double *best_ms)
     TW_CUDA(cudaEventCreate(&e1));
     double best = 1e300;
     BatchShape pick = b->shape;
-    int rc = TW_OK;
     if (b->resident && steps >= 2) {   // nothing to choose: the shots' tilings are their plans'
         for (int q = 0; q < 2 && rc == TW_OK; q++) {
             for (tw_solver *s : b->shots) cudaMemsetAsync(s->d_step, 0, sizeof(int), b->st);
@@ -3093,6 +3132,10 @@ int tw_batch_step(tw_batch *b, int n)
     if (n == 0) return TW_OK;
     TW_CUDA(cudaSetDevice(b->device));
     for (tw_solver *s : b->shots) TW_CUDA(cudaStreamSynchronize(s->st));   // queued single-shot work first
+    {
+        const int rc = batch_refresh(b);
+        if (rc != TW_OK) return rc;
+    }
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     TW_CUDA(cudaStreamIsCapturing(b->st, &cap));
     if (b->resident && n >= 2 && cap == cudaStreamCaptureStatusNone) {
