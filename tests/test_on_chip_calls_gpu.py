@@ -111,3 +111,27 @@ def test_a_batch_takes_up_receivers_and_sources_set_later(tw, bc, resident, monk
     got, want = run(True), run(False)
     assert np.abs(want[0][3][4:, 0, 10:]).max() > 0 and not want[0][3][4:, 0, :10].any()
     assert same(got, want)
+
+
+@pytest.mark.parametrize("physics,Mx,My", [("elastic", 890, 884), ("elastic", 886, 884), ("periodic", 128, 61), ("free", 77, 40)])
+def test_single_steps_and_runs_in_turn(tw, physics, Mx, My, monkeypatch):
+    """Calls of one step go by other kernels than longer ones (elastic: from 3 x 2^18 cells on)."""
+    def run(resident):
+        monkeypatch.setenv("TW_RESIDENT", "1" if resident else "0")
+        if physics == "elastic":
+            s = tw.Solver(Mx, My, 1, My, 1e-4, precision="f32", max_steps=16, energy=False)
+            rng = np.random.default_rng(1)
+            s.set_material_model(*[rng.uniform(a, b, (Mx + 2, My + 2)) for a, b in ((1.8, 2.7), (3., 4.5), (1., 2.))])
+            s.write_field(tw.MM, 0, rng.standard_normal((Mx, My)))
+            s.set_source(tw.MM, Mx // 2, 0)
+            s.add_receivers(tw.NM, [0, Mx // 2, Mx], [My - 1, 3, 0])
+        else:
+            s = acoustic(tw, Mx, My, physics, max_steps=16)
+        for n in (1, 1, 3, 1, 2, 1, 1, 4):
+            s.step(n)
+        s.sync()
+        out = result(tw, s)
+        s.close()
+        return out
+
+    assert same([run(True)], [run(False)])

@@ -138,6 +138,7 @@ struct tw_solver {
     // a run of a handle with one buffer ends where it began: a tile is stored after its neighbours have
     // sent words of their first step, so after they have loaded it (runs of two steps or more)
     bool res_in_place = false;
+    int res_min = 2;                  // least steps of a call that run there
     int res_polls = RES_POLLS;
     unsigned res_tag = 0;             // steps run this way since the exchange words were cleared
     unsigned long long *xbuf = nullptr;
@@ -1468,6 +1469,13 @@ int create_impl(tw_solver **out, const tw_grid_desc *desc, const SlabSpec &sl)
                 cudaMemsetAsync(s->d_done, 0, sizeof(int), s->st);
             }
             s->res_in_place = !s->f2[F_MM0];
+            // a run loads and stores its tiles around its steps, which one step does not always pay for. Calls of
+            // one step queued one after another, us a call on chip / by the step kernels: elastic FP32 509 x 317 15 /
+            // 26, 750^2 27 / 30, 800^2 30 / 30, 850^2 32 / 29, 1030^2 43 / 32; with the energy 800^2 32 / 35, 900^2
+            // 38 / 38, 1000^2 45 / 39; FP64 740^2 30 / 38 and '6C' 560^2 20 / 34, the largest that fit; acoustic
+            // periodic 128^2 11 / 7, 512^2 13 / 9, 1000^2 27 / 18. Of two steps: elastic 1030^2 60 / 63, acoustic 128^2
+            // 12 / 12, 1000^2 31 / 35
+            s->res_min = s->elastic && Mx * My < (d.energy ? 7L : 6L) << 17 ? 1 : 2;
             s->res_polls = std::max(0, env_int("TW_RES_POLLS", RES_POLLS));
             s->res_plan = p;
         }
@@ -1705,7 +1713,7 @@ int tw_step(tw_solver *s, int n)
     if (s->steps_done + (long)n > s->d.max_steps) return TW_ERR_RECORD_FULL;
     if (n == 0) return TW_OK;
     TW_CUDA(cudaSetDevice(s->d.device));
-    if (s->res_plan.ntx > 0 && (!s->res_in_place || n >= 2)) {
+    if (s->res_plan.ntx > 0 && n >= s->res_min) {
         // (a captured run would be replayed with the tags of its first run)
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         TW_CUDA(cudaStreamIsCapturing(s->st, &cap));
@@ -1717,13 +1725,14 @@ int tw_step(tw_solver *s, int n)
     }
     // a graph of G steps captured once and replayed; leftover steps are launched directly. The
     // graph is captured on the first call of any length when the records hold G steps, so that
-    // a short first call (a warm-up) leaves the next long call only replays and direct launches.
+    // a short first call (a warm-up) leaves the next long call only replays and direct launches
+    // (not by single steps of a handle whose long calls run on chip).
     const int G = 16;
     // the one-launch steps alternate buffers, and their graph starts from the first one; the
     // two-launch kernels update the current buffer in place, and their graph is bound to it
     // (a batch step may have moved the state of a double-buffered shot to the other buffer)
     const int gpar = (s->fused || s->afused) ? 0 : s->parity;
-    if ((!s->gexec || s->graph_steps != G || s->graph_parity != gpar) && s->d.max_steps >= G) {
+    if ((!s->gexec || s->graph_steps != G || s->graph_parity != gpar) && s->d.max_steps >= G && (s->res_plan.ntx == 0 || n >= G)) {
         s->drop_graph();
         cudaGraph_t graph;
         TW_CUDA(cudaStreamBeginCapture(s->st, cudaStreamCaptureModeThreadLocal));
