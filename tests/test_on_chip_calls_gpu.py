@@ -135,3 +135,24 @@ def test_single_steps_and_runs_in_turn(tw, physics, Mx, My, monkeypatch):
         return out
 
     assert same([run(True)], [run(False)])
+
+
+@pytest.mark.parametrize("bc", ["periodic", "free"])
+@pytest.mark.parametrize("prec,cpst", [("f32", "00"), ("f64", "00"), ("f32", "6R")])
+@pytest.mark.parametrize("sizes", [[(61, 70)], [(200, 330)] * 2, [(64, 64), (300, 41), (9, 900)], [(256, 250)] * 5 + [(40, 40)],
+                                   [(512, 500)] * 4 + [(100, 90)]])
+def test_batches_of_few_shots(tw, sizes, prec, cpst, bc, monkeypatch):
+    """Few shots share all the SMs: tilings of more tiles than the least, groups of one shot and of several."""
+    def run(resident):
+        monkeypatch.setenv("TW_RESIDENT", "1" if resident else "0")
+        shots = [acoustic(tw, Mx, My, bc, k, precision=prec, cpst=cpst) for k, (Mx, My) in enumerate(sizes)]
+        b = tw.Batch(shots)
+        for n in (9, 2, 12):
+            b.step(n)
+        b.sync()
+        out = [result(tw, s) for s in shots]
+        for h in [b] + shots:
+            h.close()
+        return out
+
+    assert same(run(True), run(False))

@@ -2,6 +2,9 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <array>
+#include <vector>
+
 #include "stepper.cuh"
 
 namespace tw {
@@ -275,9 +278,15 @@ struct ResPlan {
     bool cs = true;           // coefficients in shared memory
     size_t smem = 0;
 };
-// the tiling of a grid over n_sm SMs with smem_max bytes each: the shortest step, or (shared: the
-// SMs run other shots at the same time) the least SM time a step
-ResPlan resident_plan(long Mx, long My, int esize, int fields, bool comp, int n_sm, size_t smem_max, bool shared = false);
+// the tiling of a grid over n_sm SMs with smem_max bytes each: the shortest step
+ResPlan resident_plan(long Mx, long My, int esize, int fields, bool comp, int n_sm, size_t smem_max);
+// several shots (Mx, My): groups of shots that share the SMs, and each shot's tiling, for the shortest sum of
+// the groups' steps (no groups: a grid does not fit)
+struct ResShots {
+    std::vector<std::vector<int>> groups;
+    std::vector<ResPlan> plans;
+};
+ResShots resident_shots_plan(const std::vector<std::array<long, 2>> &grids, int esize, int fields, bool comp, int n_sm, size_t smem_max);
 // tile index of a point (host side receiver lists)
 int resident_tile(const ResPlan &p, long Mx, long My, int row, int col);
 template <class C, int PHYS>

@@ -2847,30 +2847,17 @@ int batch_resident_layout_t(tw_batch *b)
     TW_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, b->device));
     TW_CUDA(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, b->device));
     smem_max = std::max(0, smem_max - RES_STATIC);
-    std::vector<ResPlan> plans(n);
+    std::vector<std::array<long, 2>> grids(n);
     for (int k = 0; k < n; k++) {
         const tw_solver *s = b->shots[k];
         if (s->res_plan.ntx <= 0) return TW_OK;
-        plans[k] = resident_plan(s->d.Mx, s->d.My, s->esz, 3, b->cpst != TW_CPST_00, n_sm, (size_t)smem_max, true);
-        if (plans[k].ntx <= 0) return TW_OK;
+        grids[k] = {s->d.Mx, s->d.My};
     }
-    // largest first, each into the first group with room
-    std::vector<int> by(n);
-    for (int k = 0; k < n; k++) by[k] = k;
+    const ResShots layout = resident_shots_plan(grids, sizeof(C), 3, b->cpst != TW_CPST_00, n_sm, (size_t)smem_max);
+    const auto &groups = layout.groups;
+    const auto &plans = layout.plans;
+    if (groups.empty()) return TW_OK;
     auto ctas = [&](int k) { return plans[k].ntx * plans[k].nty; };
-    std::stable_sort(by.begin(), by.end(), [&](int x, int y) { return ctas(x) > ctas(y); });
-    std::vector<std::vector<int>> groups;
-    std::vector<int> used;
-    for (int k : by) {
-        size_t g = 0;
-        while (g < groups.size() && (used[g] + ctas(k) > n_sm || plans[groups[g][0]].cs != plans[k].cs)) g++;
-        if (g == groups.size()) {
-            groups.emplace_back();
-            used.push_back(0);
-        }
-        groups[g].push_back(k);
-        used[g] += ctas(k);
-    }
     std::vector<int> first;
     for (size_t g = 0; g < groups.size(); g++) {
         tw_batch::Group G{(int)b->order.size(), (int)groups[g].size(), 0, 0, plans[groups[g][0]].cs};
