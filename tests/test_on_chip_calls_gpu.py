@@ -156,3 +156,45 @@ def test_batches_of_few_shots(tw, sizes, prec, cpst, bc, monkeypatch):
         return out
 
     assert same(run(True), run(False))
+
+
+@pytest.mark.parametrize("bc", ["periodic", "free"])
+def test_batch_calls_of_every_length(tw, bc, monkeypatch):
+    """Calls too short for a batch of several groups go by the batch kernels, longer ones on chip, in turn."""
+    def run(resident):
+        monkeypatch.setenv("TW_RESIDENT", "1" if resident else "0")
+        shots = [acoustic(tw, 520, 500 + k, bc, k) for k in range(7)]
+        b = tw.Batch(shots)
+        for n in (1, 7, 2, 3, 6, 4, 1, 5):
+            b.step(n)
+        b.sync()
+        out = [result(tw, s) for s in shots]
+        for h in [b] + shots:
+            h.close()
+        return out
+
+    assert same(run(True), run(False))
+
+
+def _gives_up(tw, h):
+    try:
+        h.sync()
+    except tw.TwError as e:
+        assert e.name == "TW_ERR_TIMEOUT"
+        return True
+    return False
+
+
+def test_which_batch_calls_run_on_chip(tw, monkeypatch):
+    """With no polls a call of two steps or more that runs on chip times out, and any other does not (one step
+    exchanges nothing)."""
+    monkeypatch.setenv("TW_RES_POLLS", "0")
+    for bc, k, least in (("periodic", 3, 2), ("periodic", 8, 4), ("free", 8, 3), ("periodic", 12, 6), ("free", 12, 4)):
+        shots = [acoustic(tw, 512, 512, bc, max_steps=16) for _ in range(k)]
+        b = tw.Batch(shots)
+        b.step(least - 1)
+        assert not _gives_up(tw, b), (bc, k)
+        b.step(least)
+        assert _gives_up(tw, b), (bc, k)
+        for h in [b] + shots:
+            h.close()

@@ -2674,6 +2674,7 @@ struct tw_batch {
     // for all the steps of a call: per shot (in group order) its plan and receiver lists, per group its
     // shots and shared memory
     bool resident = false;
+    int res_min = 2;                  // least steps of a call that run there
     struct Group { int k0, n, ctas; size_t smem; bool cs; };
     std::vector<Group> groups;
     std::vector<int> order;           // shots by group
@@ -2891,6 +2892,14 @@ int batch_resident_layout_t(tw_batch *b)
     const int rc = batch_resident_receivers(b);
     if (rc != TW_OK) return rc;
     for (tw_solver *s : b->shots) TW_CUDA(cudaStreamSynchronize(s->st));
+    // a call loads and stores every group's tiles, one group after another, where the batch kernels pay by the
+    // step. FP32 shots, us a step of calls of 2 / 4 / 6 / 8 steps, on chip against the batch kernels: periodic, 2
+    // groups (24 x 256^2) 232 / 122 / 84 / 66 against 235 / 136 / 103 / 87, (2 x 1000^2) 70 / 40 / 30 / 25 against 54 / 42
+    // / 38 / 37; 4 groups (12 x 512^2) 226 / 126 / 91 / 74 against 159 / 108 / 90 / 81; 8 groups (24 x 512^2) 459 /
+    // 251 / 181 / 147 against 300 / 201 / 167 / 151; free surface, whose batch kernels are the slower ones, 4 groups
+    // (12 x 512^2) 207 / 120 against 170 / 123, 8 groups 451 / 250 against 379 / 286. FP64 and '6R' cross at the same calls
+    const int ng = (int)b->groups.size();
+    b->res_min = b->periodic ? std::min(2 * ng, 6) : std::min(ng + 1, 4);
     b->resident = true;
     return TW_OK;
 }
@@ -3134,7 +3143,7 @@ int tw_batch_step(tw_batch *b, int n)
     }
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     TW_CUDA(cudaStreamIsCapturing(b->st, &cap));
-    if (b->resident && n >= 2 && cap == cudaStreamCaptureStatusNone) {
+    if (b->resident && n >= b->res_min && cap == cudaStreamCaptureStatusNone) {
         const int rc = run_batch_resident(b, n);
         if (rc != TW_OK) return rc;
         TW_CUDA(cudaEventRecord(b->done, b->st));
