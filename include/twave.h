@@ -326,9 +326,12 @@ TW_API int tw_data_misfit(tw_solver *s, const double *obs, double *total, double
 
 /* ---- batched shots ---------------------------------------------------------------------
  * No counterpart in the reference, which runs one shot per process. A batch advances many
- * acoustic handles (the shots: independent grids of any sizes) together: each half-step is ONE
+ * acoustic handles (the shots: independent grids of any sizes) together. Where every shot fits on the
+ * chip, a call of enough steps (two, or a few more when the shots take turns) is one launch for each
+ * group of shots that share the SMs. Otherwise the batch kernels: each half-step is ONE
  * launch over the tiles of all shots and one more launch records every shot's receivers, so
- * small shots no longer pay a launch per half-step each; G steps are replayed from a CUDA graph.
+ * small shots no longer pay a launch per half-step each (periodic shots: one launch a step); G steps
+ * are replayed from a CUDA graph.
  * Each shot equals the same handle stepped alone with tw_step, bit for bit.
  * Requirements: acoustic handles on one device with the same precision (FP64/FP32),
  * compensation ('0', '3R', '6R') and x boundary, energy off, material set. A source or receivers
@@ -338,13 +341,16 @@ TW_API int tw_data_misfit(tw_solver *s, const double *obs, double *total, double
 typedef struct tw_batch tw_batch;
 TW_API int tw_batch_create(tw_batch **out, tw_solver *const *shots, int n);
 TW_API void tw_batch_destroy(tw_batch *b);
-/* Launch shape: blocks of tx x ty threads (tx*ty <= 256, a multiple of 32), rows_per_thread rows
- * per thread, `ctas` persistent CTAs walking the tile list (0: one CTA per tile). */
+/* Launch shape of the batch kernels: blocks of tx x ty threads (tx*ty <= 256, a multiple of 32),
+ * rows_per_thread rows per thread, `ctas` persistent CTAs walking the tile list (0: one CTA per
+ * tile); periodic shots: `ctas` CTAs of work for each SM. Every call then takes this shape, and none
+ * runs on chip, until tw_batch_tune. tw_batch_get_shape returns the shape the batch kernels have. */
 TW_API int tw_batch_set_shape(tw_batch *b, int tx, int ty, int rows_per_thread, int ctas);
 TW_API int tw_batch_get_shape(tw_batch *b, int *shape4);
 /* Autotuner: times `steps` batched steps for each candidate shape (tx in {32, 64, 128, 256},
- * 1/2/4 rows per thread, one CTA per tile or 4/8/16 persistent CTAs per SM), keeps the fastest
- * and returns its ms per step. It steps the shots, so it RESETS every shot afterwards
+ * 1/2/4 rows per thread, one CTA per tile or 4/8/16 persistent CTAs per SM; periodic shots: 2 to 64
+ * CTAs of work per SM), keeps the fastest for the calls that go by the batch kernels, and returns the
+ * ms per step of a call of `steps` steps, which may be one on chip. It steps the shots, so it RESETS every shot afterwards
  * (tw_reset: fields, records and step counters zeroed); call it before setting initial fields. */
 TW_API int tw_batch_tune(tw_batch *b, int steps, double *best_ms);
 /* Advance every shot n steps (asynchronous); each shot's record must hold n more steps. */

@@ -198,3 +198,24 @@ def test_which_batch_calls_run_on_chip(tw, monkeypatch):
         assert _gives_up(tw, b), (bc, k)
         for h in [b] + shots:
             h.close()
+
+
+@pytest.mark.parametrize("bc,shape", [("periodic", (0, 0, 0, 8)), ("free", (64, 4, 2, 0))])
+def test_a_launch_shape_that_was_asked_for_is_used(tw, bc, shape, monkeypatch):
+    """After tw_batch_set_shape no call runs on chip (where it would time out here), until tw_batch_tune; the shape
+    found by tune is the batch kernels'."""
+    want = acoustic(tw, 200, 210, bc, max_steps=40)
+    want.run(30)
+    monkeypatch.setenv("TW_RES_POLLS", "0")
+    s = acoustic(tw, 200, 210, bc, max_steps=40)
+    b = tw.Batch([s])
+    b.set_shape(*shape)
+    b.step(30)
+    assert not _gives_up(tw, b)
+    assert same([result(tw, s)], [result(tw, want)])
+    assert b.tune(4) > 0
+    assert b.shape()[2] in ((2, 4, 8, 15, 24, 32, 48, 64) if bc == "periodic" else (1, 2, 4))
+    b.step(30)
+    assert _gives_up(tw, b)
+    for h in (b, s, want):
+        h.close()

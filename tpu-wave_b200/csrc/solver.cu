@@ -2675,6 +2675,7 @@ struct tw_batch {
     // shots and shared memory
     bool resident = false;
     int res_min = 2;                  // least steps of a call that run there
+    bool shape_set = false;           // a launch shape asked for by tw_batch_set_shape: every call takes it
     struct Group { int k0, n, ctas; size_t smem; bool cs; };
     std::vector<Group> groups;
     std::vector<int> order;           // shots by group
@@ -3034,12 +3035,11 @@ int tw_batch_set_shape(tw_batch *b, int tx, int ty, int rows_per_thread, int cta
     if (!b) return TW_ERR_INVALID;
     const BatchShape sh{tx, ty, rows_per_thread, ctas};
     TW_CUDA(cudaSetDevice(b->device));
-    if (b->fused) {   // fused batches: `ctas` is the CTAs-per-SM target of the segmentation
-        if (ctas < 1) return TW_ERR_INVALID;
-        return batch_fused_layout(b, ctas);
-    }
-    if (!shape_ok(sh)) return TW_ERR_INVALID;
-    return batch_layout(b, sh);
+    if (b->fused ? ctas < 1 : !shape_ok(sh)) return TW_ERR_INVALID;
+    // fused batches: `ctas` is the CTAs-per-SM target of the segmentation
+    const int rc = b->fused ? batch_fused_layout(b, ctas) : batch_layout(b, sh);
+    if (rc == TW_OK) b->shape_set = true;
+    return rc;
 }
 
 int tw_batch_get_shape(tw_batch *b, int *shape4)
@@ -3085,27 +3085,6 @@ int tw_batch_tune(tw_batch *b, int steps, double *best_ms)
     TW_CUDA(cudaEventCreate(&e1));
     double best = 1e300;
     BatchShape pick = b->shape;
-    if (b->resident && steps >= 2) {   // nothing to choose: the shots' tilings are their plans'
-        for (int q = 0; q < 2 && rc == TW_OK; q++) {
-            for (tw_solver *s : b->shots) cudaMemsetAsync(s->d_step, 0, sizeof(int), b->st);
-            cudaEventRecord(e0, b->st);
-            rc = run_batch_resident(b, steps);
-            cudaEventRecord(e1, b->st);
-            const cudaError_t e = cudaEventSynchronize(e1);
-            if (rc == TW_OK && e != cudaSuccess) rc = cuda_fail(e, "tw_batch_tune");
-            float ms = 0.f;
-            if (rc == TW_OK) cudaEventElapsedTime(&ms, e0, e1);
-            best = ms / steps;
-        }
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
-        for (tw_solver *s : b->shots) {
-            const int r2 = tw_reset(s);
-            if (rc == TW_OK) rc = r2;
-        }
-        if (rc == TW_OK && best_ms) *best_ms = best;
-        return rc;
-    }
     for (const BatchShape &c : cand) {
         if ((rc = b->fused ? batch_fused_layout(b, c.ctas) : batch_layout(b, c)) != TW_OK) break;
         for (tw_solver *s : b->shots) cudaMemsetAsync(s->d_step, 0, sizeof(int), b->st);
@@ -3119,11 +3098,25 @@ int tw_batch_tune(tw_batch *b, int steps, double *best_ms)
         cudaEventElapsedTime(&ms, e0, e1);
         if (ms / steps < best) { best = ms / steps; pick = c; }
     }
+    // (on chip there is nothing to choose: the shots' tilings are their plans')
+    for (int q = 0; q < 2 && rc == TW_OK && b->resident && steps >= b->res_min; q++) {
+        for (tw_solver *s : b->shots) cudaMemsetAsync(s->d_step, 0, sizeof(int), b->st);
+        cudaEventRecord(e0, b->st);
+        rc = run_batch_resident(b, steps);
+        cudaEventRecord(e1, b->st);
+        const cudaError_t e = cudaEventSynchronize(e1);
+        if (rc == TW_OK && e != cudaSuccess) rc = cuda_fail(e, "tw_batch_tune");
+        if (rc != TW_OK) break;
+        float ms = 0.f;
+        cudaEventElapsedTime(&ms, e0, e1);
+        best = std::min(best, (double)ms / steps);
+    }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (rc != TW_OK) return rc;
     for (tw_solver *s : b->shots)
         if ((rc = tw_reset(s)) != TW_OK) return rc;
+    b->shape_set = false;
     if ((rc = b->fused ? batch_fused_layout(b, pick.ctas) : batch_layout(b, pick)) != TW_OK) return rc;
     if (best_ms) *best_ms = best;
     return TW_OK;
@@ -3143,7 +3136,7 @@ int tw_batch_step(tw_batch *b, int n)
     }
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     TW_CUDA(cudaStreamIsCapturing(b->st, &cap));
-    if (b->resident && n >= b->res_min && cap == cudaStreamCaptureStatusNone) {
+    if (b->resident && !b->shape_set && n >= b->res_min && cap == cudaStreamCaptureStatusNone) {
         const int rc = run_batch_resident(b, n);
         if (rc != TW_OK) return rc;
         TW_CUDA(cudaEventRecord(b->done, b->st));
