@@ -219,3 +219,39 @@ def test_a_launch_shape_that_was_asked_for_is_used(tw, bc, shape, monkeypatch):
     assert _gives_up(tw, b)
     for h in (b, s, want):
         h.close()
+
+
+def test_a_handle_without_room_for_the_exchange_words_steps_by_its_other_kernels(tw, monkeypatch):
+    """With the GPU's memory all but taken, a handle that would fit without its on-chip buffers (53 MB here) is
+    made and steps as one that never had them."""
+    import torch
+    M = 740
+
+    def run():
+        s = tw.Solver(M, M, 1, M, 1e-4, precision="f64", max_steps=8, energy=False)
+        s.set_material_model(*[np.full((M + 2, M + 2), v) for v in (2.0, 3.0, 1.7)])
+        s.set_source(tw.MM, 300, 300)
+        s.run(5)
+        out = s.read_field(tw.MM)
+        s.close()
+        return out
+
+    run()   # (kernels loaded)
+    monkeypatch.setenv("TW_RESIDENT", "0")
+    run()
+    tw.release_cached_memory()
+    torch.cuda.empty_cache()
+    before = torch.cuda.mem_get_info()[0]
+    want = run()
+    need = before - torch.cuda.mem_get_info()[0]   # (the pool keeps it)
+    tw.release_cached_memory()
+    assert need > 100 << 20
+    monkeypatch.delenv("TW_RESIDENT")
+    held = torch.empty(torch.cuda.mem_get_info()[0] - need - (24 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        got = run()
+    finally:
+        del held
+        torch.cuda.empty_cache()
+        tw.release_cached_memory()
+    assert np.abs(got).max() > 0 and np.array_equal(got, want)

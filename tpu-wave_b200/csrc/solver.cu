@@ -614,6 +614,28 @@ int resident_coefx(tw_solver *s)
     return TW_OK;
 }
 
+// exchange words for any tiling of the handle's grid
+int resident_xbuf(tw_solver *s)
+{
+    s->xbuf_bytes = (size_t)(s->elastic ? 6 : 2) * (s->d.Mx + 1) * ((s->d.My + 2) & ~1L) * 2 * s->esz;
+    if (s->alloc((void **)&s->xbuf, s->xbuf_bytes) != TW_OK) return TW_ERR_NOMEM;
+    TW_CUDA(cudaMemsetAsync(s->xbuf, 0, s->xbuf_bytes, s->st));
+    return TW_OK;
+}
+
+// the buffers of a handle's runs with plan p; false, and none kept, if there is no room
+bool resident_buffers(tw_solver *s, const ResPlan &p)
+{
+    if ((p.ntx * p.nty == 1 || resident_xbuf(s) == TW_OK) && (p.cs || resident_coefx(s) == TW_OK) &&
+        s->alloc((void **)&s->d_rcv_off_r, sizeof(int) * (p.ntx * p.nty + 1)) == TW_OK)
+        return true;
+    cudaGetLastError();
+    s->release(s->xbuf);
+    for (void *&c : s->coefx) { s->release(c); c = nullptr; }
+    s->xbuf = nullptr;
+    return false;
+}
+
 // the arguments of n steps on chip from the current buffers, with plan p and its receiver lists
 template <class C>
 ResArgs<C> resident_args(const tw_solver *s, const ResPlan &p, int n, const int *rcv_off, const int *rcv)
@@ -1457,17 +1479,13 @@ int create_impl(tw_solver **out, const tw_grid_desc *desc, const SlabSpec &sl)
             };
             e = d.precision == TW_FP64 ? prepare(0.0) : prepare(0.0f);
             if (e != cudaSuccess) return fail(cuda_fail(e, "cudaFuncSetAttribute"));
-            if (p.ntx * p.nty > 1) {
-                s->xbuf_bytes = (size_t)(s->elastic ? 6 : 2) * (Mx + 1) * ((My + 2) & ~1L) * 2 * s->esz;
-                if ((rc_ = s->alloc((void **)&s->xbuf, s->xbuf_bytes)) != TW_OK) return fail(rc_);
-                cudaMemsetAsync(s->xbuf, 0, s->xbuf_bytes, s->st);
-            }
-            if (!p.cs && (rc_ = resident_coefx(s)) != TW_OK) return fail(rc_);
-            if ((rc_ = s->alloc((void **)&s->d_rcv_off_r, sizeof(int) * (p.ntx * p.nty + 1))) != TW_OK) return fail(rc_);
             if (!s->d_done) {
                 if ((rc_ = s->alloc((void **)&s->d_done, sizeof(int))) != TW_OK) return fail(rc_);
                 cudaMemsetAsync(s->d_done, 0, sizeof(int), s->st);
             }
+        }
+        // (no room for what the run needs beside the handle's own buffers: the other step kernels)
+        if (p.ntx > 0 && resident_buffers(s, p)) {
             s->res_in_place = !s->f2[F_MM0];
             // a run loads and stores its tiles around its steps, which one step does not always pay for. Calls of
             // one step queued one after another, us a call on chip / by the step kernels: elastic FP32 509 x 317 15 /
@@ -2865,14 +2883,14 @@ int batch_resident_layout_t(tw_batch *b)
         tw_batch::Group G{(int)b->order.size(), (int)groups[g].size(), 0, 0, plans[groups[g][0]].cs};
         for (int k : groups[g]) {
             tw_solver *s = b->shots[k];
-            if (!s->xbuf) {   // (a shot of one tile when alone)
-                s->xbuf_bytes = (size_t)2 * (s->d.Mx + 1) * ((s->d.My + 2) & ~1L) * 2 * s->esz;
-                if (s->alloc((void **)&s->xbuf, s->xbuf_bytes) != TW_OK) return TW_ERR_NOMEM;
-                TW_CUDA(cudaMemsetAsync(s->xbuf, 0, s->xbuf_bytes, s->st));
-            }
-            if (!plans[k].cs) {
-                const int rc = resident_coefx(s);
-                if (rc != TW_OK) return rc;
+            // (the words of a shot of one tile when alone, the columns of one whose coefficients lie in shared
+            // memory when alone; no room: the batch kernels)
+            if ((!s->xbuf && resident_xbuf(s) != TW_OK) || (!plans[k].cs && resident_coefx(s) != TW_OK)) {
+                cudaGetLastError();
+                b->order.clear();
+                b->plans.clear();
+                b->groups.clear();
+                return TW_OK;
             }
             first.push_back(G.ctas);
             G.ctas += ctas(k);
