@@ -13,7 +13,7 @@ int tma_strips(long My)
     return My >= need ? (int)((My - need) / TMA_CORE) + 1 : 0;
 }
 
-template <bool ENERGY, bool Q16 = false>
+template <bool Q16>
 static size_t tma_smem()
 {
     return (size_t)TmaLayout<Q16>::bytes;
@@ -30,7 +30,7 @@ template <bool ENERGY, bool Q16, bool WITEMS>
 static cudaError_t tma_attr()
 {
     return cudaFuncSetAttribute(k_elastic_tma<ENERGY, Q16, WITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)tma_smem<ENERGY, Q16>());
+                                (int)tma_smem<Q16>());
 }
 
 template <bool ENERGY>
@@ -62,13 +62,13 @@ static void launch_strips(FusedArgs<float, float> &a, const TmaMaps &maps, int n
         int dev = 0;
         cudaGetDevice(&dev);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_elastic_tma<ENERGY, Q16, WITEMS>, FS_THREADS_MAX,
-                                                      tma_smem<ENERGY, Q16>());
+                                                      tma_smem<Q16>());
         cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
     }
     const int n_items = (WITEMS ? a.n_zone * a.n_bstrip + a.n_octa : 0) + a.n_tcta;
     const int n_strips = std::min(n_items, std::max(1, resident) * n_sm);
     a.n_all_ctas = n_side + n_strips;
-    if (go) k_elastic_tma<ENERGY, Q16, WITEMS><<<n_strips, FS_THREADS_MAX, tma_smem<ENERGY, Q16>(), st>>>(a, maps);
+    if (go) k_elastic_tma<ENERGY, Q16, WITEMS><<<n_strips, FS_THREADS_MAX, tma_smem<Q16>(), st>>>(a, maps);
 }
 
 template <bool WITEMS>
