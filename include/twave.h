@@ -115,11 +115,14 @@ typedef struct {
     long row_off;                  /* a slab: global row of its local row 0 (0 otherwise) */
     long own_rows[2];              /* a slab: the global rows [own_rows[0], own_rows[1]) it owns */
     long Mx_glob;                  /* cells along x of the whole grid */
-    int step_kind;                 /* how a step taken by itself runs: 0 the per-point kernels (three or more
-                                      launches), 1 the one-launch fused step, 2 the TMA-staged step (two
-                                      launches side by side), 3 the fused periodic acoustic step. tw_step on
-                                      a grid that fits on the chip (elastic FP32 / FP64, up to about a million
-                                      cells) runs all its steps in one launch whatever this says. */
+    int step_kind;                 /* the kernels that step the handle one launch (or a few) a step: 0 the
+                                      per-point kernels (three or more launches), 1 the one-launch fused
+                                      step, 2 the TMA-staged step (one launch, or two side by side), 3 the fused
+                                      periodic acoustic step. Whatever this says, tw_step on a grid that fits
+                                      on the chip (FP32 / FP64, elastic, or acoustic with the energy off, up to
+                                      about a million cells) runs the steps of a call in one launch: calls of
+                                      two steps or more, and of one where that is the shorter call (elastic
+                                      below 3 x 2^18 cells, 7 x 2^17 with the energy). */
     int launches_per_step;         /* kernels one step launches */
 } tw_info;
 
@@ -179,11 +182,13 @@ TW_API int tw_reset(tw_solver *s);
 /* Advance n steps: forward_simulation_periodic_y (forward_simulation.cpp:21-182) / the device
  * loop (nvcc_device_FDM_2D.cu:449-730). Asynchronous on the handle's stream. */
 TW_API int tw_step(tw_solver *s, int n);
-/* Wait for queued work; returns the first sticky error (TW_ERR_NONFINITE, TW_ERR_CUDA). */
+/* Wait for queued work; returns the first sticky error (TW_ERR_TIMEOUT, TW_ERR_NONFINITE, TW_ERR_CUDA). */
 TW_API int tw_sync(tw_solver *s);
 
 /* Field readback in the reference layout (copy_field_pitched dev_to_hst, grid.cuh:463-469):
- * rows x cols of the grid, row stride ld >= cols, converted to double. field: 0, or 1 for syy on MM. */
+ * rows x cols of the grid, row stride ld >= cols, converted to double. field: 0, or 1 for syy on MM. The first
+ * read gives the handle a staging buffer on the device (at most 64 MB, without which, when there is no
+ * room for it, the host converts). */
 TW_API int tw_read_field(tw_solver *s, int grid, int field, double *host, long ld);
 /* Set a field from the host (reference layout). */
 TW_API int tw_write_field(tw_solver *s, int grid, int field, const double *host, long ld);

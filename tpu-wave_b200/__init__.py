@@ -462,7 +462,8 @@ class Solver:
 
 
 class Batch:
-    """Many acoustic Solver handles stepped together (one launch per half-step for all shots).
+    """Many acoustic Solver handles stepped together (on chip where all fit, else one launch per
+    half-step for all shots).
     The shots keep their own set-up and readback; see tw_batch_create."""
 
     def __init__(self, shots):
@@ -491,7 +492,7 @@ class Batch:
         return tuple(out)
 
     def tune(self, steps: int = 8) -> float:
-        """Pick the fastest launch shape; resets every shot afterwards."""
+        """Pick the batch kernels' fastest launch shape; resets every shot afterwards."""
         ms = C.c_double()
         _ok(lib().tw_batch_tune(self.h, steps, C.byref(ms)), "tw_batch_tune")
         return ms.value

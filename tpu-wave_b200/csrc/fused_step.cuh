@@ -289,9 +289,10 @@ __device__ void interior_warp(const FusedArgs<S, C> &a, int y0, int seg, int it,
     // column My on the one there is 0. That one value a row is staged with the others and takes its
     // tap's place by a select. (Read from global memory where it was used, up to eight loads and two
     // round trips a row, it made these strips' items of the TMA step 33.6 us long at 2048^2, the longest
-    // 62.9, the whole step; us a step, before -> here: 2048^2 63.6 -> 58.9, with the energy 82.8 -> 76.9,
-    // 1200 x 1500 40.0 -> 36.5; here FP64 1024^2 45.0 -> 39.6, FP16 pairs 1500 x 1023 59.0 -> 47.7, 3R 3000 x 2000
-    // 145.0 -> 137.7, '6C' 1000 x 1200 49.8 -> 45.2.)
+    // 62.9, the whole step; us a step, before -> here: 2048^2 62.2 -> 59.8, with the energy 82.4 -> 78.6,
+    // 1200 x 1500 40.5 -> 38.1 (16-bit codes 4095 x 4097 187.7 -> 189.8); here FP64 1024^2 45.1 -> 39.9, FP16 pairs
+    // 1500 x 1023 59.4 -> 47.7 (the packed arithmetic included), 3R 3000 x 2000 150.9 -> 139.4, '6C' 1000 x 1200
+    // 46.9 -> 42.0.)
     const bool z_na = EDGE && c0 == -2;                        // columns -2 and -1: the column after -1
     const bool z_va = EDGE && c0 == My, z_vb = EDGE && c1 == My;   // columns My and My + 1: column My itself
     const bool z_pb = EDGE && c0 == My + 1;
